@@ -1055,14 +1055,17 @@ fgss_status fgss_autotune(fgss_ctx* ctx, const fgss_sets_view* sets, const fgss_
         const std::string key = tune_key(sets->n_sets, sets->n_tokens, o.threshold);
         TuneEntry win;
         win.ms = 1e30f;
-        // every fused-kernel shape, then every query on the global accumulator
-        for (int i = 0; i <= kNumFusedShapes; i++) {
+        // every shape of the keyed kernel, every query on the global accumulator, the claim kernels
+        for (int i = 0; i < kNumFusedShapes + 2; i++) {
             TuneEntry te = filter_entry(FGSS_FILTER_GLOBAL);
             if (i < kNumFusedShapes) {
                 te.threads = kFusedShapes[i][0];
                 te.hash_log2 = kFusedShapes[i][1];
                 te.regs_rt = kFusedShapes[i][2];
                 te.heavy_min_probe = 0;
+                te.keyed = 1;
+            } else if (i > kNumFusedShapes) {
+                te = TuneEntry();
             }
             te.ctas_per_sm = 0;
             c.tune_force = &te;
@@ -1081,8 +1084,8 @@ fgss_status fgss_autotune(fgss_ctx* ctx, const fgss_sets_view* sets, const fgss_
             }
             c.tune_force = nullptr;
             if (c.verbose)
-                fprintf(stderr, "[fgss] autotune %s: threads %d hash_log2 %d regs_rt %d global %d -> %.3f ms\n",
-                        key.c_str(), te.threads, te.hash_log2, te.regs_rt, te.heavy_min_probe, bestms);
+                fprintf(stderr, "[fgss] autotune %s: threads %d hash_log2 %d regs_rt %d global %d keyed %d -> %.3f ms\n",
+                        key.c_str(), te.threads, te.hash_log2, te.regs_rt, te.heavy_min_probe, te.keyed, bestms);
             if (bestms < win.ms) {
                 win = te;
                 win.ms = bestms;

@@ -131,6 +131,38 @@ void fused_launch(Ctx& c, const TuneEntry& te, const JoinArgs* d_args, const Fus
 
 namespace {
 
+// k_claim's shape: 256 consumer threads with 8 entries each and 8192 claim
+// slots, 3 CTAs per SM (56 KB of shared memory each, which leaves the L1 about
+// 60 KB).  Measured on 1,000,000 heavy-tailed records at t = 0.7 / 100,000
+// titles at t = 0.5: 93.5 / 4.36 ms; 6 entries 98.5 / 4.29; 4 entries and 4
+// CTAs 105 / 4.74; 512 threads and 2 CTAs 103 / 4.90.
+using Claim = ClaimShape<256, 8, 13>;
+constexpr int kClaimCtas = 3;
+
+template <bool SIDED>
+void claim_launch_as(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const uint4* items, uint32_t n_items,
+                     uint32_t* counter) {
+    FGSS_CK(cudaFuncSetAttribute(k_claim<Claim, kClaimCtas, SIDED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)Claim::bytes));
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)kClaimCtas * c.num_sms, n_items);
+    k_claim<Claim, kClaimCtas, SIDED><<<grid, Claim::NT, Claim::bytes, c.stream>>>(d_args, d_fargs, items, n_items,
+                                                                                   counter);
+    FGSS_LAUNCH_CK();
+}
+
+void claim_launch(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const uint4* items, uint32_t n_items,
+                  uint32_t* counter, bool sided) {
+    if (sided) claim_launch_as<true>(c, d_args, d_fargs, items, n_items, counter);
+    else claim_launch_as<false>(c, d_args, d_fargs, items, n_items, counter);
+}
+
+void tiny_launch(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const TileMap& m, bool sided) {
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)m.ntiles * (m.tile / 32), (uint64_t)c.num_sms * 16);
+    if (sided) k_tiny<true><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, m);
+    else k_tiny<false><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, m);
+    FGSS_LAUNCH_CK();
+}
+
 constexpr uint32_t kRecTile = 256;  // records per tile of the per-record stages (thread per record in the MLP)
 
 // Uploads the tile map of joins [off[j], off[j+1]) in tiles of `tile` to the
@@ -176,7 +208,7 @@ unsigned tile_grid(Ctx& c, const TileMap& m, unsigned per_sm = 16) {
 
 template <typename K>
 void index_sort(Ctx& c, Batch& B, uint64_t E_cap, int tbits, int jbits, const uint64_t* d_E, const uint64_t* d_loff,
-                uint32_t* list, uint2* ent) {
+                uint32_t* list, const uint64_t* d_toff, uint32_t* tab, uint2* ent) {
     const std::string& p = c.bpfx;
     K* key = c.devT<K>(p + "b.ix.key", E_cap + 1);
     uint64_t* val = c.devT<uint64_t>(p + "b.ix.val", E_cap + 1);
@@ -185,27 +217,27 @@ void index_sort(Ctx& c, Batch& B, uint64_t E_cap, int tbits, int jbits, const ui
     FGSS_LAUNCH_CK();
     radix_sort<K, uint64_t>(c, key, val, E_cap, d_E, 0, tbits + jbits, (p + "b.ixsort").c_str());
     k_index_lists_mj<K><<<grid_for(E_cap, 256, c.num_sms * 32), 256, 0, c.stream>>>(
-        B.d_args, key, val, d_E, (uint32_t)tbits, d_loff, list, ent);
+        B.d_args, key, val, d_E, (uint32_t)tbits, d_loff, list, d_toff, tab, ent);
     FGSS_LAUNCH_CK();
 }
 
 // The batch's pre-pass, first part (index built): windows of every probe
-// token (exact per-query work), the learned model's estimates (model) and the
-// work-item cost of every query (window entries + 4 x predicted candidates +
-// size) with its exclusive prefix in cpre (total at cpre[R]).  d_sums:
-// [0, nj) cost totals, [nj, 2nj) predicted results, [2nj, 3nj) predicted
-// candidates, [3nj] chunk-boundary words for slot tables of cap_entries.
+// token (exact per-query work), the class of every query (classes; else all
+// QC_KEYED), the learned model's estimates (model) and the work-item costs
+// (k_cost_mj).  d_sums: k_cost_mj's 2 nj + 4 sums, then the joins' predicted
+// results (nj) and candidates (nj).
 struct Prepass {
     uint2* win = nullptr;
     uint32_t* wpre = nullptr;
     uint32_t* wtot = nullptr;
     uint4* meta = nullptr;
-    uint64_t* cost = nullptr;
-    uint64_t* cpre = nullptr;
+    uint32_t* pred = nullptr;       // null without the model
+    uint64_t* cost[2] = {};         // class QC_KEYED, QC_CLAIM
     uint64_t* d_sums = nullptr;
+    size_t n_sums = 0;
 };
 
-Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bool model) {
+Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bool model, bool classes) {
     const size_t nj = B.js.size();
     const std::string& p = c.bpfx;
     const uint64_t R = B.R;
@@ -216,33 +248,60 @@ Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bo
     pp.meta = c.devT<uint4>(p + "b.meta", R + 1);
     float* feat = c.devT<float>(p + "b.feat", (R + 1) * kFeatures);
     uint32_t* pred = c.devT<uint32_t>(p + "b.pred", R + 1);
-    pp.cost = c.devT<uint64_t>(p + "b.cost", R + 1);
-    pp.cpre = c.devT<uint64_t>(p + "b.cpre", R + 1);
-    pp.d_sums = c.devT<uint64_t>(p + "b.sums", 3 * nj + 2);
-    FGSS_CK(cudaMemsetAsync(pp.d_sums, 0, (3 * nj + 2) * 8, c.stream));
+    pp.cost[0] = c.devT<uint64_t>(p + "b.cost0", R + 1);
+    pp.cost[1] = c.devT<uint64_t>(p + "b.cost1", R + 1);
+    pp.n_sums = 4 * nj + 4;
+    pp.d_sums = c.devT<uint64_t>(p + "b.sums", pp.n_sums);
+    FGSS_CK(cudaMemsetAsync(pp.d_sums, 0, pp.n_sums * 8, c.stream));
     if (R == 0) return pp;
     const unsigned g = tile_grid(c, B.rec);
-    k_windows_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta);
+    k_windows_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, classes);
     FGSS_LAUNCH_CK();
     if (model) {
+        pp.pred = pred;
         k_features_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, feat);
         FGSS_LAUNCH_CK();
-        model_predict_tiles(c, feat, B.rec, pred, pp.d_sums + nj, pp.d_sums + 2 * nj);
+        model_predict_tiles(c, feat, B.rec, pred, pp.d_sums + 2 * nj + 4, pp.d_sums + 3 * nj + 4);
     }
-    k_cost_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, pp.wtot, model ? pred : nullptr, cap_entries, pp.cost,
-                                       (unsigned long long*)(pp.d_sums + 3 * nj));
-    FGSS_LAUNCH_CK();
-    exclusive_scan<uint64_t>(c, pp.cost, pp.cpre, R, nullptr, pp.cpre + R, (p + "b.scan.c").c_str());
-    k_join_cost_totals<<<grid_for(nj, 128), 128, 0, c.stream>>>(B.rec.roff, (uint32_t)nj, pp.cpre, pp.d_sums);
+    k_cost_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, pp.meta, pp.pred, cap_entries, pp.cost[0], pp.cost[1],
+                                       (unsigned long long*)pp.d_sums);
     FGSS_LAUNCH_CK();
     return pp;
+}
+
+// Work items of one class, K[j] of join j, longest first (on the device).
+uint4* batch_items(Ctx& c, Batch& B, const Prepass& pp, int cls, const std::vector<uint32_t>& K, uint64_t nitems) {
+    const size_t nj = B.js.size();
+    const std::string p = c.bpfx + "b.i" + std::to_string(cls) + ".";
+    uint64_t* cpre = c.devT<uint64_t>(p + "cpre", B.R + 1);
+    exclusive_scan<uint64_t>(c, pp.cost[cls], cpre, B.R, nullptr, cpre + B.R, (p + "scan").c_str());
+    uint32_t* hk = c.pinnedT<uint32_t>(p + "hkoff", nj + 1);
+    hk[0] = 0;
+    for (size_t i = 0; i < nj; i++) hk[i + 1] = hk[i] + K[i];
+    uint32_t* d_koff = c.devT<uint32_t>(p + "koff", nj + 1);
+    FGSS_CK(cudaMemcpyAsync(d_koff, hk, (nj + 1) * 4, cudaMemcpyHostToDevice, c.stream));
+    uint4* items = c.devT<uint4>(p + "items", nitems + 1);
+    uint32_t* ikey = c.devT<uint32_t>(p + "key", nitems + 1);
+    uint32_t* ival = c.devT<uint32_t>(p + "val", nitems + 1);
+    k_items_mj<<<grid_for(nitems, 128), 128, 0, c.stream>>>(B.rec.roff, d_koff, (uint32_t)nj, (uint32_t)nitems, cpre,
+                                                             pp.d_sums + cls * nj, items, ikey, ival);
+    FGSS_LAUNCH_CK();
+    if (nitems > 1) {
+        // longest-processing-time order: sort items by descending cost
+        uint4* sorted = c.devT<uint4>(p + "items2", nitems + 1);
+        radix_sort<uint32_t, uint32_t>(c, ikey, ival, nitems, nullptr, 0, 16, (p + "sort").c_str());
+        k_permute_items<<<grid_for(nitems, 128), 128, 0, c.stream>>>(items, ival, nitems, sorted);
+        FGSS_LAUNCH_CK();
+        items = sorted;
+    }
+    return items;
 }
 
 // Second part: every record's token bitmap and the chunk splits of the
 // queries whose windows exceed cap_entries, into a boundary buffer of
 // cbuf_cap words (a query that finds it full is bisected by the fused kernel
 // instead); returns the fused kernel's per-join arguments on the device.
-FusedArgs* batch_filters(Ctx& c, Batch& B, const Prepass& pp, uint32_t cap_entries, uint64_t cbuf_cap) {
+FusedArgs* batch_filters(Ctx& c, Batch& B, const Prepass& pp, uint32_t cap_entries, uint64_t cbuf_cap, bool chunks) {
     const size_t nj = B.js.size();
     const std::string& p = c.bpfx;
     const uint64_t R = B.R;
@@ -276,6 +335,7 @@ FusedArgs* batch_filters(Ctx& c, Batch& B, const Prepass& pp, uint32_t cap_entri
     const unsigned g = tile_grid(c, B.rec);
     k_bitmaps_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, B.rec);
     FGSS_LAUNCH_CK();
+    if (!chunks) return d_fargs;  // no query for k_fused
     k_chunks_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, B.rec, pp.wtot, cap_entries, cbuf, cbuf_cap, cused);
     FGSS_LAUNCH_CK();
     return d_fargs;
@@ -391,22 +451,38 @@ void batch_index(Ctx& c, Batch& B, uint64_t E_cap) {
     const int tbits = bits_for((uint64_t)B.terms_max + 1);
     const int jbits = bits_for(nj);
     // join j's list offsets: n_terms + 1 entries from loff[j], positions in
-    // the batch's entry arrays
-    uint64_t* hl = c.pinnedT<uint64_t>(p + "b.hloff", nj + 1);
-    hl[0] = 0;
-    for (size_t j = 0; j < nj; j++) hl[j + 1] = hl[j] + B.js[j]->in.n_terms + 1;
-    const uint64_t L = hl[nj];
-    uint64_t* d_loff = c.devT<uint64_t>(p + "b.loff", nj + 1);
-    FGSS_CK(cudaMemcpyAsync(d_loff, hl, (nj + 1) * 8, cudaMemcpyHostToDevice, c.stream));
+    // the batch's entry arrays; its block table, n_terms nb + 1 entries from
+    // toff[j].  A join of at most kBlockIds records has one block and its list
+    // offsets are the table; one whose table would hold more words than a
+    // quarter of its tokens (k-mers: millions of terms with short lists) has none.
+    uint64_t* hl = c.pinnedT<uint64_t>(p + "b.hloff", 2 * nj + 2);
+    uint64_t* ht = hl + nj + 1;
+    hl[0] = ht[0] = 0;
+    for (size_t j = 0; j < nj; j++) {
+        const fgss_sets_view& in = B.js[j]->in;
+        JoinArgs& a = B.js[j]->args;
+        hl[j + 1] = hl[j] + in.n_terms + 1;
+        const uint64_t nb = (in.n_sets + kBlockIds - 1) / kBlockIds;
+        a.nb = nb <= 1 ? (uint32_t)nb : nb * in.n_terms <= in.n_tokens / 4 + 65536 ? (uint32_t)nb : 0u;
+        ht[j + 1] = ht[j] + (a.nb > 1 ? nb * in.n_terms + 1 : 0);
+    }
+    const uint64_t L = hl[nj], TB = ht[nj];
+    uint64_t* d_loff = c.devT<uint64_t>(p + "b.loff", 2 * nj + 2);
+    const uint64_t* d_toff = d_loff + nj + 1;
+    FGSS_CK(cudaMemcpyAsync(d_loff, hl, (2 * nj + 2) * 8, cudaMemcpyHostToDevice, c.stream));
     uint32_t* list = c.devT<uint32_t>(p + "b.list", L + 1);
+    uint32_t* tab = c.devT<uint32_t>(p + "b.tab", TB + 1);
     uint2* ent = c.devT<uint2>(p + "b.ent", E_cap + 1);
     for (size_t j = 0; j < nj; j++) {
         JoinArgs& a = B.js[j]->args;
         a.list_off = list + hl[j];
+        a.tab = a.nb > 1 ? tab + ht[j] : a.list_off;
         a.ent = ent;
     }
+    upload_args(c, B, p + "b.ha1");
     // a join without entries keeps these zero offsets (empty lists)
     FGSS_CK(cudaMemsetAsync(list, 0, L * 4, c.stream));
+    if (TB) FGSS_CK(cudaMemsetAsync(tab, 0, TB * 4, c.stream));
     FGSS_CK(cudaMemsetAsync(B.d_e, 0, nj * 16, c.stream));
     if (B.R) {
         uint64_t* d_E = c.devT<uint64_t>(p + "b.dE", 2);
@@ -414,17 +490,18 @@ void batch_index(Ctx& c, Batch& B, uint64_t E_cap) {
         FGSS_LAUNCH_CK();
         k_join_entries<<<grid_for(nj, 128), 128, 0, c.stream>>>(B.rec.roff, (uint32_t)nj, B.ioff, B.d_e);
         FGSS_LAUNCH_CK();
-        if (tbits + jbits <= 32) index_sort<uint32_t>(c, B, E_cap, tbits, jbits, d_E, d_loff, list, ent);
-        else index_sort<uint64_t>(c, B, E_cap, tbits, jbits, d_E, d_loff, list, ent);
+        if (tbits + jbits <= 32) index_sort<uint32_t>(c, B, E_cap, tbits, jbits, d_E, d_loff, list, d_toff, tab, ent);
+        else index_sort<uint64_t>(c, B, E_cap, tbits, jbits, d_E, d_loff, list, d_toff, tab, ent);
     }
-    upload_args(c, B, p + "b.ha1");
 }
 
 void batch_query_costs(Ctx& c, Batch& B, bool use_model, uint64_t* out) {
     if (B.R == 0) return;
     const TuneEntry te = batch_shape(c, B);
-    const Prepass pp = batch_prepass(c, B, (1u << te.hash_log2) / 4 * 3, B.P, use_model && c.model);
-    FGSS_CK(cudaMemcpyAsync(out, pp.cost, B.R * 8, cudaMemcpyDeviceToHost, c.stream));
+    const Prepass pp = batch_prepass(c, B, (1u << te.hash_log2) / 4 * 3, B.P, use_model && c.model, false);
+    k_query_costs_mj<<<tile_grid(c, B.rec), 256, 0, c.stream>>>(B.d_args, B.rec, pp.wtot, pp.pred, pp.cost[0]);
+    FGSS_LAUNCH_CK();
+    FGSS_CK(cudaMemcpyAsync(out, pp.cost[0], B.R * 8, cudaMemcpyDeviceToHost, c.stream));
     c.sync();
 }
 
@@ -445,64 +522,61 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     const uint64_t P_cap = plan ? plan->P_cap : B.P;
     if (P_cap < B.P) fail(FGSS_ERR_CUDA, "window buffers below the batch's probe-token count");
     const bool model = use_model && c.model;
-    const Prepass pp = batch_prepass(c, B, cap_entries, P_cap, model);
+    // the caller's own choice of a strategy, a tuned keyed shape and the global accumulator take every query
+    bool classes = te.heavy_min_probe == 0 && !te.keyed;
+    for (size_t i = 0; i < nj; i++) classes &= joins[i]->filter == FGSS_FILTER_AUTO;
+    const Prepass pp = batch_prepass(c, B, cap_entries, P_cap, model, classes);
 
-    // work items: ~256 per resident CTA over the whole batch (a few queries per
-    // item at 100k records), split by cost share and handed out longest first,
-    // so the dynamic queue ends with short items
-    std::vector<uint32_t> K(nj, 0);
-    uint64_t nitems = 0;
-    uint64_t* hsum = c.pinnedT<uint64_t>(p + "b.hsum", 3 * nj + 2);
+    // work items per class of k_fused and k_claim: ~256 per resident CTA over
+    // the whole batch (a few queries per item at 100k records), split by cost
+    // share and handed out longest first, so the dynamic queue ends with short
+    // items.  A class without queries gets none, or under a plan (whose graph
+    // may be replayed on other data) a few.
+    std::vector<uint32_t> K[2] = {std::vector<uint32_t>(nj, 0), std::vector<uint32_t>(nj, 0)};
+    uint64_t nitems[2] = {0, 0};
+    bool tiny = classes && B.R != 0;
+    uint64_t* hsum = c.pinnedT<uint64_t>(p + "b.hsum", pp.n_sums);
     if (capture) {
-        K = plan->K;
-        nitems = plan->nitems;
+        for (int k = 0; k < 2; k++) {
+            K[k] = plan->K[k];
+            nitems[k] = plan->nitems[k];
+        }
     } else {
-        FGSS_CK(cudaMemcpyAsync(hsum, pp.d_sums, (3 * nj + 2) * 8, cudaMemcpyDeviceToHost, c.stream));
+        FGSS_CK(cudaMemcpyAsync(hsum, pp.d_sums, pp.n_sums * 8, cudaMemcpyDeviceToHost, c.stream));
         c.sync();
         for (size_t i = 0; i < nj; i++) {
             if (!model || joins[i]->res_cap_hint) continue;
-            joins[i]->pred_results = hsum[nj + i];
-            joins[i]->pred_candidates = hsum[2 * nj + i];
+            joins[i]->pred_results = hsum[2 * nj + 4 + i];
+            joins[i]->pred_candidates = hsum[3 * nj + 4 + i];
         }
-        uint64_t grand = 0;
-        for (size_t i = 0; i < nj; i++) grand += hsum[i];
-        const uint64_t want = (uint64_t)256 * fused_resident_ctas(c, te);
-        for (size_t i = 0; i < nj; i++) {
-            const uint64_t n = joins[i]->in.n_sets;
-            if (n == 0) continue;
-            uint64_t k = grand ? (want * hsum[i] + grand - 1) / grand : 1;
-            k = std::max<uint64_t>(1, std::min<uint64_t>(k, n));
-            K[i] = (uint32_t)k;
-            nitems += k;
+        const uint64_t* count = hsum + 2 * nj;  // queries per class
+        for (int k = 0; k < 2; k++) {
+            if (k == QC_CLAIM && !classes) continue;
+            if (count[k] == 0 && !plan) continue;
+            uint64_t grand = 0;
+            for (size_t i = 0; i < nj; i++) grand += hsum[k * nj + i];
+            const uint64_t ctas = k == QC_CLAIM ? (uint64_t)kClaimCtas * c.num_sms : fused_resident_ctas(c, te);
+            const uint64_t want = (count[k] ? 256 : 4) * ctas;
+            for (size_t i = 0; i < nj; i++) {
+                const uint64_t n = joins[i]->in.n_sets;
+                if (n == 0) continue;
+                uint64_t v = grand ? (want * hsum[k * nj + i] + grand - 1) / grand : 1;
+                v = std::max<uint64_t>(1, std::min<uint64_t>(v, n));
+                K[k][i] = (uint32_t)v;
+                nitems[k] += v;
+            }
         }
+        if (!plan) tiny &= count[QC_TINY] != 0;
     }
-    if (nitems >= 0xffffffffull) fail(FGSS_ERR_UNSUPPORTED, "too many work items");
+    if (nitems[0] >= 0xffffffffull || nitems[1] >= 0xffffffffull) fail(FGSS_ERR_UNSUPPORTED, "too many work items");
     // chunk boundaries: exactly the words the splits take (the plan's size in
     // a capture; a replay on other data that needs more bisects instead)
-    const uint64_t cbuf_cap = capture ? plan->cbuf_cap : std::min<uint64_t>(hsum[3 * nj], 0xfffffff0ull);
+    const uint64_t cbuf_cap = capture ? plan->cbuf_cap : std::min<uint64_t>(hsum[2 * nj + 3], 0xfffffff0ull);
     if (plan && !capture) plan->cbuf_cap = cbuf_cap;
-    FusedArgs* d_fargs = batch_filters(c, B, pp, cap_entries, cbuf_cap);
-    uint32_t* hk = c.pinnedT<uint32_t>(p + "b.hkoff", nj + 1);
-    hk[0] = 0;
-    for (size_t i = 0; i < nj; i++) hk[i + 1] = hk[i] + K[i];
-    uint32_t* d_koff = c.devT<uint32_t>(p + "b.koff", nj + 1);
-    FGSS_CK(cudaMemcpyAsync(d_koff, hk, (nj + 1) * 4, cudaMemcpyHostToDevice, c.stream));
-    uint4* items = c.devT<uint4>(p + "b.items", nitems + 1);
-    if (nitems) {
-        uint32_t* ikey = c.devT<uint32_t>(p + "b.ikey", nitems + 1);
-        uint32_t* ival = c.devT<uint32_t>(p + "b.ival", nitems + 1);
-        k_items_mj<<<grid_for(nitems, 128), 128, 0, c.stream>>>(B.rec.roff, d_koff, (uint32_t)nj, (uint32_t)nitems,
-                                                                 pp.cpre, pp.d_sums, items, ikey, ival);
-        FGSS_LAUNCH_CK();
-        if (nitems > 1) {
-            // longest-processing-time order: sort items by descending cost
-            uint4* sorted = c.devT<uint4>(p + "b.items2", nitems + 1);
-            radix_sort<uint32_t, uint32_t>(c, ikey, ival, nitems, nullptr, 0, 16, (p + "b.isort").c_str());
-            k_permute_items<<<grid_for(nitems, 128), 128, 0, c.stream>>>(items, ival, nitems, sorted);
-            FGSS_LAUNCH_CK();
-            items = sorted;
-        }
-    }
+    FusedArgs* d_fargs = batch_filters(c, B, pp, cap_entries, cbuf_cap, nitems[QC_KEYED] != 0);
+    const uint4* items[2] = {nullptr, nullptr};
+    for (int k = 0; k < 2; k++)
+        if (nitems[k]) items[k] = batch_items(c, B, pp, k, K[k], nitems[k]);
 
     bool sided = false;
     for (size_t i = 0; i < nj; i++) sided |= joins[i]->args.side != nullptr;
@@ -527,7 +601,7 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
                 uint64_t v;
                 if (J.res_cap_hint) v = J.res_cap_hint;
                 else if (J.res_cap_user) v = J.res_cap_user;
-                else if (model) v = std::max<uint64_t>((uint64_t)((double)hsum[nj + i] * 1.5) + 4096, last);
+                else if (model) v = std::max<uint64_t>((uint64_t)((double)hsum[2 * nj + 4 + i] * 1.5) + 4096, last);
                 else v = std::max<uint64_t>(J.in.n_sets + 4096, last);
                 cap[i] = std::min<uint64_t>(v, 0xfffffff0ull);
             }
@@ -547,7 +621,11 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
         upload_args(c, B, p + "b.ha2");
         FGSS_CK(cudaMemsetAsync(counter, 0, (4 + nj) * 4, c.stream));
         FGSS_CK(cudaEventRecordWithFlags(c.ev[4], c.stream, rec_flags));
-        if (nitems) fused_launch(c, te, B.d_args, d_fargs, items, (uint32_t)nitems, counter, sided);
+        if (nitems[QC_CLAIM])
+            claim_launch(c, B.d_args, d_fargs, items[QC_CLAIM], (uint32_t)nitems[QC_CLAIM], counter + 1, sided);
+        if (nitems[QC_KEYED])
+            fused_launch(c, te, B.d_args, d_fargs, items[QC_KEYED], (uint32_t)nitems[QC_KEYED], counter, sided);
+        if (tiny) tiny_launch(c, B.d_args, d_fargs, B.rec, sided);
         FGSS_CK(cudaEventRecordWithFlags(c.ev[5], c.stream, rec_flags));
         c.probe_timed = true;
         // queries deferred to the global-memory accumulator: one persistent
@@ -595,8 +673,8 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     }
     if (plan && !capture) {
         plan->te = te;
-        plan->K = K;
-        plan->nitems = nitems;
+        for (int k = 0; k < 2; k++) plan->K[k] = K[k];
+        for (int k = 0; k < 2; k++) plan->nitems[k] = nitems[k];
         plan->heavy_slots = slots;
         plan->res_cap = cap;
     }

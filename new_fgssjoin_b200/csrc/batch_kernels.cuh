@@ -4,7 +4,7 @@
 // per-join stages' own (join_kernels.cuh, fused_kernels.cuh).
 #pragma once
 
-#include "fused_kernels.cuh"
+#include "claim_kernels.cuh"
 #include "tiles.cuh"
 
 namespace fgss {
@@ -52,26 +52,64 @@ __global__ void k_index_entries_mj(const JoinArgs* __restrict__ joins, TileMap m
     }
 }
 
-// After the stable sort by (join, term): the entry columns and every join's
-// list offsets, as positions in the batch's entry arrays (a join without
-// entries keeps the zero offsets its buffer was cleared to).
+// Warp-collective: every lane writes v to p[from .. to); long runs by the whole warp.
+__device__ __forceinline__ void warp_fill_runs(uint32_t* p, uint64_t from, uint64_t to, uint32_t v) {
+    const bool lng = to > from && to - from > 8;
+    if (!lng)
+        for (uint64_t x = from; x < to; x++) p[x] = v;
+    for (uint32_t m = __ballot_sync(kFull, lng); m; m &= m - 1) {
+        const uint32_t l = __ffs(m) - 1;
+        uint32_t* pp = reinterpret_cast<uint32_t*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(p), l));
+        const uint64_t f = __shfl_sync(kFull, from, l), t = __shfl_sync(kFull, to, l);
+        const uint32_t vv = __shfl_sync(kFull, v, l);
+        for (uint64_t x = f + lane_id(); x < t; x += 32) pp[x] = vv;
+    }
+}
+
+// After the stable sort by (join, term): the entry columns, every join's list
+// offsets, as positions in the batch's entry arrays (a join without entries
+// keeps the zero offsets its buffer was cleared to), and the block tables of
+// the joins that have one of more than one block (toff[j]: join j's in
+// tab_all; with one block the list offsets are the table).
 template <typename K>
 __global__ void k_index_lists_mj(const JoinArgs* __restrict__ joins, const K* __restrict__ key,
                                         const uint64_t* __restrict__ val, const uint64_t* __restrict__ d_e,
                                         uint32_t tbits, const uint64_t* __restrict__ loff,
-                                        uint32_t* __restrict__ list_all, uint2* __restrict__ ent) {
+                                        uint32_t* __restrict__ list_all, const uint64_t* __restrict__ toff,
+                                        uint32_t* __restrict__ tab_all, uint2* __restrict__ ent) {
     const uint64_t E = *d_e;
     const uint64_t tmask = (1ull << tbits) - 1;
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < E; k += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t v = val[k], kk = (uint64_t)key[k];
-        ent[k] = make_uint2((uint32_t)(v >> 32), (uint32_t)v);
-        const uint32_t j = (uint32_t)(kk >> tbits), w = (uint32_t)(kk & tmask);
-        uint32_t* lo = list_all + loff[j];
-        if (k == 0 || (uint32_t)((uint64_t)key[k - 1] >> tbits) != j)
-            for (uint32_t x = 0; x <= w; x++) lo[x] = (uint32_t)k;  // terms before the join's first
-        uint32_t nxt = joins[j].n_terms;
-        if (k + 1 < E && (uint32_t)((uint64_t)key[k + 1] >> tbits) == j) nxt = (uint32_t)((uint64_t)key[k + 1] & tmask);
-        for (uint32_t x = w + 1; x <= nxt; x++) lo[x] = (uint32_t)(k + 1);
+    for (uint64_t k0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; k0 < E;
+         k0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t k = k0 + lane_id();
+        const bool in = k < E;
+        uint32_t *lo = list_all, *tb = tab_all;
+        uint64_t w = 0, nxt = 0, c = 0, cn = 0;  // this entry's term and the next one's; their rows in the block table
+        bool first = false, table = false;
+        if (in) {
+            const uint64_t v = val[k], kk = (uint64_t)key[k];
+            const uint32_t s = (uint32_t)(v >> 32);
+            ent[k] = make_uint2(s, (uint32_t)v);
+            const uint64_t j = kk >> tbits;
+            const uint64_t kn = k + 1 < E ? (uint64_t)key[k + 1] : ~0ull;
+            const bool more = k + 1 < E && kn >> tbits == j;
+            first = k == 0 || (uint64_t)key[k - 1] >> tbits != j;
+            w = kk & tmask;
+            nxt = more ? kn & tmask : joins[j].n_terms;
+            lo += loff[j];
+            const uint64_t nb = joins[j].nb;
+            if (nb > 1) {
+                table = true;
+                tb += toff[j];
+                c = w * nb + s / kBlockIds;
+                cn = nxt * nb + (more ? (uint32_t)(val[k + 1] >> 32) / kBlockIds : 0u);
+            }
+        }
+        // offsets up to the join's first entry, then from this entry's to the next one's
+        warp_fill_runs(lo, 0, first ? w + 1 : 0, (uint32_t)k);
+        warp_fill_runs(lo, w + 1, in ? nxt + 1 : 0, (uint32_t)k + 1);
+        warp_fill_runs(tb, 0, first && table ? c + 1 : 0, (uint32_t)k);
+        warp_fill_runs(tb, c + 1, table ? cn + 1 : 0, (uint32_t)k + 1);
     }
 }
 
@@ -85,13 +123,13 @@ static __global__ void k_join_entries(const uint64_t* __restrict__ roff, uint32_
 // Warp per record: the windows of every probe token (windows_query) of every join.
 static __global__ void k_windows_mj(const JoinArgs* __restrict__ joins, TileMap m, const uint32_t* __restrict__ poff,
                                     uint2* __restrict__ win, uint32_t* __restrict__ wpre, uint32_t* __restrict__ wtot,
-                                    uint4* __restrict__ meta) {
+                                    uint4* __restrict__ meta, bool classes) {
     const uint32_t wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (uint32_t b = blockIdx.x; b < m.ntiles; b += gridDim.x) {
         const TileRange t = tile_range(m, b);
         const uint64_t g0 = __ldg(m.roff + t.j);
         for (uint32_t q = t.r0 + wid; q < t.r1; q += nw)
-            windows_query(joins[t.j], q, poff + g0, win, wpre, wtot + g0, meta + g0);
+            windows_query(joins[t.j], q, poff + g0, win, wpre, wtot + g0, meta + g0, classes);
     }
 }
 
@@ -118,8 +156,9 @@ static __global__ void k_chunks_mj(const JoinArgs* __restrict__ joins, const Fus
         const FusedArgs& fa = fargs[t.j];
         const uint64_t g0 = __ldg(m.roff + t.j);
         for (uint32_t q = t.r0 + wid; q < t.r1; q += nw)
-            chunks_query(joins[t.j], q, fa.poff, fa.win, wtot + g0, cap, const_cast<uint2*>(fa.qchunk), cbuf,
-                         cbuf_cap, cbuf_used);
+            if ((fa.meta[q].z >> 16) == QC_KEYED)
+                chunks_query(joins[t.j], q, fa.poff, fa.win, wtot + g0, cap, const_cast<uint2*>(fa.qchunk), cbuf,
+                             cbuf_cap, cbuf_used);
     }
 }
 
@@ -170,39 +209,75 @@ static __global__ void k_features_mj(const JoinArgs* __restrict__ joins, TileMap
     }
 }
 
-// Work-item cost of every query: exact window entries + 4 x the learned
-// estimate of its candidates (when given) + its size; 0 outside the join's
-// query range.  Also sums into *need the chunk-boundary words the queries'
-// splits for slot tables of `cap` entries take (chunks_query).
-static __global__ void k_cost_mj(const JoinArgs* __restrict__ joins, TileMap m, const uint32_t* __restrict__ wtot,
-                                 const uint32_t* __restrict__ pred, uint32_t cap, uint64_t* __restrict__ cost,
-                                 unsigned long long* __restrict__ need) {
-    unsigned long long words = 0;
+// Work estimate of one query: exact window entries + 4 x the learned estimate
+// of its candidates (when given) + its size; 0 outside the join's query range.
+__device__ __forceinline__ unsigned long long query_cost(const JoinArgs& a, uint32_t q, uint32_t L,
+                                                         const uint32_t* __restrict__ pred) {
+    if (q < a.q_lo || q >= a.q_hi) return 0;
+    unsigned long long v = (unsigned long long)L + a.len[q];
+    if (pred) v += 4ull * *pred;
+    return v;
+}
+
+// Estimates of every query (fgss_query_costs).
+static __global__ void k_query_costs_mj(const JoinArgs* __restrict__ joins, TileMap m, const uint32_t* __restrict__ wtot,
+                                        const uint32_t* __restrict__ pred, uint64_t* __restrict__ cost) {
+    for (uint32_t b = blockIdx.x; b < m.ntiles; b += gridDim.x) {
+        const TileRange tr = tile_range(m, b);
+        const uint64_t g0 = __ldg(m.roff + tr.j);
+        for (uint32_t q = tr.r0 + threadIdx.x; q < tr.r1; q += blockDim.x)
+            cost[g0 + q] = query_cost(joins[tr.j], q, wtot[g0 + q], pred ? pred + g0 + q : nullptr);
+    }
+}
+
+// Costs the work items of k_fused (class 0) and k_claim (class 1) are cut by:
+// a query's estimate in its own class and 1 elsewhere (the kernel steps over
+// it), so a class without work still cuts into items of equal counts.  sums,
+// per class c: [c nj, (c + 1) nj) the joins' totals; then at 2 nj the queries
+// of classes 0, 1 and 2, and at 2 nj + 3 the chunk-boundary words the splits of
+// the class-0 queries for slot tables of `cap` entries take (chunks_query).
+// Launched with one thread per record of a tile.
+static __global__ void __launch_bounds__(256) k_cost_mj(const JoinArgs* __restrict__ joins, TileMap m,
+                                                        const uint4* __restrict__ meta,
+                                                        const uint32_t* __restrict__ pred, uint32_t cap,
+                                                        uint64_t* __restrict__ cost0, uint64_t* __restrict__ cost1,
+                                                        unsigned long long* __restrict__ sums) {
+    __shared__ unsigned long long s_sum[6][8];
     for (uint32_t b = blockIdx.x; b < m.ntiles; b += gridDim.x) {
         const TileRange tr = tile_range(m, b);
         const JoinArgs& a = joins[tr.j];
         const uint64_t g0 = __ldg(m.roff + tr.j);
-        for (uint32_t q = tr.r0 + threadIdx.x; q < tr.r1; q += blockDim.x) {
-            unsigned long long v = 0;
-            const uint32_t L = wtot[g0 + q];
-            if (q >= a.q_lo && q < a.q_hi) {
-                v = (unsigned long long)L + a.len[q];
-                if (pred) v += 4ull * pred[g0 + q];
+        const uint32_t q = tr.r0 + threadIdx.x;
+        unsigned long long v[6] = {0, 0, 0, 0, 0, 0};
+        if (q < tr.r1) {
+            const uint4 mt = meta[g0 + q];
+            const uint32_t cls = mt.z >> 16;
+            const unsigned long long c = query_cost(a, q, mt.w, pred ? pred + g0 + q : nullptr);
+            v[0] = cls == QC_KEYED && c > 1 ? c : 1;
+            v[1] = cls == QC_CLAIM && c > 1 ? c : 1;
+            cost0[g0 + q] = v[0];
+            cost1[g0 + q] = v[1];
+            if (cls != QC_NONE) v[2 + cls] = 1;
+            if (cls == QC_KEYED) {
+                uint32_t qp, span;
+                const uint32_t n = chunk_count(a, q, mt.w, cap, qp, span);
+                v[5] = (unsigned long long)(n - 1) * qp;
             }
-            cost[g0 + q] = v;
-            uint32_t qp, span;
-            words += (unsigned long long)(chunk_count(a, q, L, cap, qp, span) - 1) * qp;
         }
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+            v[i] = warp_sum(v[i]);
+            if (lane_id() == 0) s_sum[i][threadIdx.x >> 5] = v[i];
+        }
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            unsigned long long t = 0;
+            for (uint32_t w = 0; w < 8; w++) t += s_sum[threadIdx.x][w];
+            const uint32_t at = threadIdx.x < 2 ? threadIdx.x * m.nj + tr.j : 2 * m.nj + threadIdx.x - 2;
+            if (t) atomicAdd(sums + at, t);
+        }
+        __syncthreads();
     }
-    words = warp_sum(words);
-    if (lane_id() == 0 && words) atomicAdd(need, words);
-}
-
-// Cost total of every join from the batch's exclusive cost prefix.
-static __global__ void k_join_cost_totals(const uint64_t* __restrict__ roff, uint32_t nj,
-                                          const uint64_t* __restrict__ cpre, uint64_t* __restrict__ tot) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nj; j += gridDim.x * blockDim.x)
-        tot[j] = cpre[roff[j + 1]] - cpre[roff[j]];
 }
 
 // The join of batch-wide item k: the last j with koff[j] <= k.

@@ -28,6 +28,7 @@ struct TuneEntry {
     int ctas_per_sm = 0;   // persistent grid = ctas_per_sm x SMs (0 = as many as fit)
     int heavy_min_probe = 0;  // queries with a probe prefix this long take the global accumulator (0: only
                               // those beyond the fused kernel's shared-memory caps)
+    int keyed = 0;         // 1: the keyed slot table (k_fused) for every query, 0: k_claim and k_tiny where they apply
     float ms = 0.f;        // best time seen
 };
 

@@ -73,12 +73,33 @@ struct FusedLayout {
     static_assert(off_bm % 16 == 0, "the membership words are cleared with 16-byte stores");
 };
 
+// The class of a query: the kernel that filters and verifies it, in
+// meta[q].z above the 16 bits of the index prefix.
+enum : uint32_t {
+    QC_KEYED = 0,  // k_fused: keyed slot table
+    QC_CLAIM = 1,  // k_claim (claim_kernels.cuh): a CTA per query
+    QC_TINY = 2,   // k_tiny (claim_kernels.cuh): a warp per query
+    QC_NONE = 3    // no window entry: nothing to do
+};
+constexpr uint32_t kClaimPC = 640;   // probe tokens of a k_claim query
+constexpr uint32_t kTinyMax = 128;   // window entries of a k_tiny query
+
+// Class of a query with W window entries and qp probe tokens.  Up to kTinyMax
+// entries fit four registers per lane of one warp; 500,000 reads (22 entries
+// each on average) take 1.1 ms with a warp each, 2.8 ms with the keyed table.
+// kClaimPC windows fit k_claim's shared memory at three CTAs per SM.
+__device__ __forceinline__ uint32_t query_class(uint32_t qp, uint32_t W) {
+    return W == 0 ? QC_NONE : W <= kTinyMax ? QC_TINY : qp <= kClaimPC ? QC_CLAIM : QC_KEYED;
+}
+
 // Windows of one query's probe tokens (warp-collective): win[poff[q] + j] =
 // (lo, hi), wpre[poff[q] + j] = entries in the query's windows before window j,
-// wtot[q] = sum of the window sizes (also meta[q].w).
+// wtot[q] = sum of the window sizes (also meta[q].w).  The block table bounds
+// the searches to the blocks that hold q + 1 and send - 1.  classes: give the
+// query its class (else every query is QC_KEYED).
 __device__ __forceinline__ void windows_query(const JoinArgs& a, uint32_t q, const uint32_t* __restrict__ poff,
                                               uint2* __restrict__ win, uint32_t* __restrict__ wpre,
-                                              uint32_t* __restrict__ wtot, uint4* __restrict__ meta) {
+                                              uint32_t* __restrict__ wtot, uint4* __restrict__ meta, bool classes) {
     const uint32_t lane = lane_id();
     const bool unsorted = (*a.status & ST_UNSORTED) != 0;
     const uint32_t lq = a.len[q];
@@ -93,12 +114,19 @@ __device__ __forceinline__ void windows_query(const JoinArgs& a, uint32_t q, con
         uint32_t lo = 0, hi = 0;
         if (j < qp) {
             const uint32_t w = __ldg(qt + j);
-            const uint32_t b = __ldg(a.list_off + w), e = __ldg(a.list_off + w + 1);
-            lo = e;
-            hi = e;
             if (send > q + 1) {
-                lo = lower_bound_src(a.ent, b, e, q + 1);
-                hi = unsorted ? e : lower_bound_src(a.ent, lo, e, send);
+                if (a.nb) {
+                    const uint32_t* row = a.tab + (uint64_t)w * a.nb;
+                    const uint32_t bq = (q + 1) / kBlockIds, bs = (send - 1) / kBlockIds;
+                    const uint32_t q0 = __ldg(row + bq), q1 = __ldg(row + bq + 1);
+                    const uint32_t s0 = bs == bq ? q0 : __ldg(row + bs), s1 = bs == bq ? q1 : __ldg(row + bs + 1);
+                    lo = lower_bound_src(a.ent, q0, q1, q + 1);
+                    hi = unsorted ? s1 : lower_bound_src(a.ent, max(lo, s0), s1, send);
+                } else {
+                    const uint32_t b = __ldg(a.list_off + w), e = __ldg(a.list_off + w + 1);
+                    lo = lower_bound_src(a.ent, b, e, q + 1);
+                    hi = unsorted ? e : lower_bound_src(a.ent, lo, e, send);
+                }
             }
         }
         const uint32_t incl = warp_incl_scan(hi - lo);
@@ -110,7 +138,8 @@ __device__ __forceinline__ void windows_query(const JoinArgs& a, uint32_t q, con
     }
     if (lane == 0) {
         wtot[q] = tot;
-        meta[q] = make_uint4(a.pos[q], lq, lq <= 65535u ? a.index[lq] : 0u, tot);
+        const uint32_t cls = classes ? query_class(qp, tot) : (uint32_t)QC_KEYED;
+        meta[q] = make_uint4(a.pos[q], lq, (lq <= 65535u ? a.index[lq] : 0u) | (cls << 16), tot);
     }
 }
 
@@ -169,7 +198,7 @@ struct FusedArgs {
     const uint32_t* poff;    // per query: first probe window
     const uint2* win;
     const uint4* smin;       // per length sum S: (cand_min, inter_min, need, 0)
-    const uint4* meta;       // per record: (pos, len, index prefix, window entries)
+    const uint4* meta;       // per record: (pos, len, index prefix | class << 16, window entries)
     const uint32_t* wpre;    // per probe window: entries of the query's earlier windows
     const uint2* qchunk;     // per query: (first boundary in cbuf, number of chunks)
     const uint32_t* cbuf;    // chunk boundaries: per inner boundary, first entry of each probe window
@@ -600,11 +629,12 @@ __device__ void fused_query(const JoinArgs& a, const FusedArgs& fa, uint32_t q, 
                         cand = c + min(A, ls - smx) >= sm.x;
                         ver = c + min(A - 1, ls - smx - 1) >= sm.y;
                     } else {
-                        const uint4 sm4 = fa.meta[s];  // (pos, len, index prefix)
+                        const uint4 sm4 = fa.meta[s];  // (pos, len, index prefix | class << 16)
+                        const uint32_t ips = sm4.z & 0xffffu;
                         const uint32_t* st = a.tok + sm4.x;
                         const uint32_t xq = qsrc[jm];
-                        cand = (c + A >= sm.x) && smax_le(st, (int)ls + (int)c - (int)sm.x, c, sm4.z, xq);
-                        ver = (c + A - 1 >= sm.y) && smax_le(st, (int)ls + (int)c - 1 - (int)sm.y, c, sm4.z, xq);
+                        cand = (c + A >= sm.x) && smax_le(st, (int)ls + (int)c - (int)sm.x, c, ips, xq);
+                        ver = (c + A - 1 >= sm.y) && smax_le(st, (int)ls + (int)c - 1 - (int)sm.y, c, ips, xq);
                     }
                     my_cand += cand;
                     if (ver) {
@@ -742,7 +772,11 @@ __global__ void __launch_bounds__(NT, RT / NT) k_fused(const JoinArgs* __restric
         }
         const JoinArgs& a = joins[w.x];
         const FusedArgs& fa = fargs[w.x];
-        for (uint32_t q = w.y; q < w.z; q++) fused_query<NT, HLOG, SIDED>(a, fa, q, smem, ctr);
+        for (uint32_t q0 = w.y; q0 < w.z; q0 += 32) {  // the item's queries of this kernel's class
+            const uint32_t ql = q0 + lane_id();
+            uint32_t todo = __ballot_sync(kFull, ql < w.z && (fa.meta[ql].z >> 16) == QC_KEYED);
+            for (; todo; todo &= todo - 1) fused_query<NT, HLOG, SIDED>(a, fa, q0 + __ffs(todo) - 1, smem, ctr);
+        }
         const uint32_t big = max(max(ctr.cand, ctr.window), max(ctr.merged, ctr.verified));
         if (__any_sync(kFull, big > (1u << 30))) flush_fused_counters(a, ctr);
         __syncthreads();

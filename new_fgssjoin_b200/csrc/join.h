@@ -144,8 +144,8 @@ struct BatchPlan {
     bool capture = false;             // issue device work only, with these decisions
     TuneEntry te;
     uint64_t E_cap = 0, P_cap = 0;    // index entries, probe windows the buffers hold
-    std::vector<uint32_t> K;          // work items per join
-    uint64_t nitems = 0;
+    std::vector<uint32_t> K[2];       // work items per join (k_fused, k_claim)
+    uint64_t nitems[2] = {0, 0};
     std::vector<uint64_t> res_cap;    // result slots per join
     uint64_t cbuf_cap = 0;            // chunk-boundary words
     uint32_t heavy_slots = 0;

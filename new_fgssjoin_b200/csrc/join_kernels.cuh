@@ -30,6 +30,9 @@ namespace fgss {
 
 constexpr uint32_t kEmpty = 0xffffffffu;
 
+// Source ids per block of a join's block table (JoinArgs.tab).
+constexpr uint32_t kBlockIds = 4096;
+
 // status bits (per join)
 enum : uint32_t {
     ST_UNSORTED = 1u << 0,   // record sizes not non-increasing in memory order
@@ -81,6 +84,10 @@ struct JoinArgs {
     const uint32_t* list_off;  // [n_terms + 1]
     const uint2* ent;          // per entry: (source record, source size << 16 | position of the token
                                // in the source); sources ascending within a list
+    // block table: tab[w nb + b] = first entry of term w with a source in [b kBlockIds, ..) or later
+    // (the next term's row follows, so tab[w nb + b + 1] ends block b); nb = 0: the join has none
+    const uint32_t* tab;
+    uint32_t nb;
     // plain method
     uint32_t* vcnt;            // count pass: per query, candidates that need a merge
     uint32_t* ccnt;            // count pass: per query, candidates (reference definition)
