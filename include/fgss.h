@@ -15,10 +15,11 @@
  *
  * Ownership.  The caller owns its inputs.  The library owns what it returns
  * (fgss_sets, fgss_pairs) until the matching *_free call.  The host columns
- * of a result are one page-locked block where one can be had (the copies
- * from the device run at the link's rate); fgss_pairs_free gives that block
- * back to a process-wide pool, which keeps at most 1 GiB of free blocks for
- * later results and releases the rest.
+ * of a result, and of token sets made on the device, are one page-locked block
+ * where one can be had (the copies from and to the device run at the link's
+ * rate); fgss_pairs_free and fgss_sets_free give that block back to a
+ * process-wide pool, which keeps at most 1 GiB of free blocks for later results
+ * and releases the rest.
  *
  * Threading.  A context is bound to one device and one stream and is not
  * thread-safe; separate contexts are independent.

@@ -182,6 +182,28 @@ def _arr(a, dtype=np.uint32):
     return np.ascontiguousarray(a, dtype=dtype)
 
 
+def _view(ptr, n, owner, ctype=ctypes.c_uint32, dtype=np.uint32):
+    """A numpy array over n elements at ptr that keeps ``owner`` alive."""
+    buf = (ctype * n).from_address(ctypes.cast(ptr, ctypes.c_void_p).value)
+    buf._owner = owner
+    return np.frombuffer(buf, dtype)
+
+
+class _SetsOwner:
+    """Owns one fgss_sets (a copy of the struct) and frees it once."""
+
+    def __init__(self, lib, s):
+        self._lib = lib
+        self._s = _Sets()
+        ctypes.memmove(ctypes.byref(self._s), ctypes.byref(s), ctypes.sizeof(_Sets))
+
+    def __del__(self):
+        try:
+            self._lib.fgss_sets_free(ctypes.byref(self._s))
+        except Exception:  # interpreter shutdown
+            pass
+
+
 class Sets:
     """Token sets in the reference's MEMORY order (src/fgssjoin/data.cu:97-113).
 
@@ -209,10 +231,13 @@ class Sets:
 
     @classmethod
     def _from_c(cls, s):
+        """Sets over the library's columns without copying them (they are released,
+        fgss_sets_free, with the last array over them)."""
         n, T = s.n_sets, s.n_tokens
+        owner = _SetsOwner(load_library(), s)
 
         def take(p, k):
-            return np.ctypeslib.as_array(p, shape=(k,)).copy() if k else np.zeros(0, np.uint32)
+            return _view(p, k, owner) if k else np.zeros(0, np.uint32)
         loc = take(s.loc, T) if s.loc else None
         return cls(take(s.id, n), take(s.pos, n), take(s.len, n), take(s.tokens, T), s.n_terms, loc)
 
@@ -223,10 +248,7 @@ class Sets:
         st = L.fgss_load_bin(os.fsencode(path), ctypes.byref(s))
         if st != 0:
             raise FgssError(st, "cannot load %s: %s" % (path, L.fgss_strerror(st).decode()))
-        try:
-            return cls._from_c(s)
-        finally:
-            L.fgss_sets_free(ctypes.byref(s))
+        return cls._from_c(s)
 
     def _as_c(self):
         s = _Sets()
@@ -342,10 +364,7 @@ class Context:
         s = _Sets()
         st = self._L.fgss_tokenize(self._ctx, text, len(text), ctypes.byref(o), ctypes.byref(s))
         _check(self._L, self._ctx, st)
-        try:
-            return Sets._from_c(s)
-        finally:
-            self._L.fgss_sets_free(ctypes.byref(s))
+        return Sets._from_c(s)
 
     def tokenize_dual(self, text_r, text_s, q=3, mode="qgram", pad=False, pad_char=1, suffix=True, lower=True):
         """Two texts over one vocabulary -> (Sets of R, Sets of S) (fgss_tokenize_dual)."""
@@ -356,11 +375,7 @@ class Context:
         st = self._L.fgss_tokenize_dual(self._ctx, text_r, len(text_r), text_s, len(text_s), ctypes.byref(o),
                                         ctypes.byref(a), ctypes.byref(b))
         _check(self._L, self._ctx, st)
-        try:
-            return Sets._from_c(a), Sets._from_c(b)
-        finally:
-            self._L.fgss_sets_free(ctypes.byref(a))
-            self._L.fgss_sets_free(ctypes.byref(b))
+        return Sets._from_c(a), Sets._from_c(b)
 
     # ----------------------------------------------------------------- join
     @staticmethod
@@ -388,11 +403,7 @@ class Context:
         owner = _PairsOwner(L, p)
 
         def take(ptr, ctype=ctypes.c_uint32, dtype=np.uint32):
-            if not n:
-                return np.zeros(0, dtype)
-            buf = (ctype * n).from_address(ctypes.cast(ptr, ctypes.c_void_p).value)
-            buf._owner = owner  # the arrays keep the columns alive
-            return np.frombuffer(buf, dtype)
+            return _view(ptr, n, owner, ctype, dtype) if n else np.zeros(0, dtype)
         cands = None
         if want_candidates:
             nc = p.n_cand

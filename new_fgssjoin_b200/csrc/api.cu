@@ -17,6 +17,7 @@
 
 #include "join.h"
 #include "model.h"
+#include "pinned.h"
 #include "prims.cuh"
 #include "tokenize.h"
 
@@ -33,6 +34,12 @@ void set_thread_error(const std::string& msg) { g_err = msg; }
 
 namespace {
 
+// After an error: copies from or to the caller's page-locked arrays that the
+// call queued are done before it returns.
+void settle(fgss_ctx* ctx) {
+    if (ctx && ctx->c.stream && cudaStreamSynchronize(ctx->c.stream) != cudaSuccess) (void)cudaGetLastError();
+}
+
 template <typename F>
 fgss_status guard(fgss_ctx* ctx, F&& f) {
     try {
@@ -40,13 +47,16 @@ fgss_status guard(fgss_ctx* ctx, F&& f) {
         if (ctx) ctx->c.last_error.clear();
         return FGSS_OK;
     } catch (const Error& e) {
+        settle(ctx);
         if (ctx) ctx->c.last_error = e.msg;
         g_err = e.msg;
         return e.st;
     } catch (const std::bad_alloc&) {
+        settle(ctx);
         if (ctx) ctx->c.last_error = "host allocation failed";
         return FGSS_ERR_NOMEM;
     } catch (...) {
+        settle(ctx);
         if (ctx) ctx->c.last_error = "unknown error";
         return FGSS_ERR_CUDA;
     }
@@ -70,66 +80,6 @@ void fill_stats(const JoinState& J, fgss_stats* st) {
     st->query_tokens = J.stats_host[SS_QTOK];
     st->predicted_candidates = J.pred_candidates;
     st->predicted_results = J.pred_results;
-}
-
-// Page-locked host blocks for the pairs handed to the caller: the device-to-host
-// copies of the columns run at the link's rate and write no freshly mapped
-// pages.  fgss_pairs_free gives a block back to a process-wide pool that the
-// next call takes it from; the pool keeps at most kPinnedPoolBytes of free
-// blocks and releases the rest.  Where page-locked memory cannot be had the
-// columns are malloc'd as before.
-struct PinnedPool {
-    std::mutex mu;
-    std::multimap<size_t, void*> free_blocks;  // size -> free block
-    std::map<void*, size_t> sizes;             // every block of the pool, handed out or free
-    size_t free_bytes = 0;
-};
-constexpr size_t kPinnedPoolBytes = size_t(1) << 30;
-
-PinnedPool& pinned_pool() {
-    static PinnedPool* pool = new PinnedPool;  // never destroyed: blocks may be given back at exit
-    return *pool;
-}
-
-// A block of at least `bytes` (a free one of at most twice the size, else a new
-// one), or nullptr.
-void* pinned_take(size_t bytes) {
-    PinnedPool& P = pinned_pool();
-    {
-        std::lock_guard<std::mutex> lk(P.mu);
-        auto it = P.free_blocks.lower_bound(bytes);
-        if (it != P.free_blocks.end() && it->first <= 2 * bytes + (size_t(1) << 20)) {
-            void* b = it->second;
-            P.free_bytes -= it->first;
-            P.free_blocks.erase(it);
-            return b;
-        }
-    }
-    void* b = nullptr;
-    if (cudaHostAlloc(&b, bytes, cudaHostAllocPortable) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return nullptr;
-    }
-    std::lock_guard<std::mutex> lk(P.mu);
-    P.sizes[b] = bytes;
-    return b;
-}
-
-// Gives a block of the pool back (true), or returns false for other memory.
-bool pinned_give(void* b) {
-    PinnedPool& P = pinned_pool();
-    std::lock_guard<std::mutex> lk(P.mu);
-    auto it = P.sizes.find(b);
-    if (it == P.sizes.end()) return false;
-    const size_t sz = it->second;
-    if (P.free_bytes + sz <= kPinnedPoolBytes) {
-        P.free_blocks.emplace(sz, b);
-        P.free_bytes += sz;
-    } else {
-        P.sizes.erase(it);
-        if (cudaFreeHost(b) != cudaSuccess) (void)cudaGetLastError();
-    }
-    return true;
 }
 
 // Host columns of R pairs (freed by fgss_pairs_free): one page-locked block of
@@ -699,6 +649,10 @@ fgss_sets_view fgss_sets_view_of(const fgss_sets* s) {
 
 void fgss_sets_free(fgss_sets* s) {
     if (!s) return;
+    if (s->id && pinned_give(s->id)) {  // the columns were one block of the page-locked pool
+        memset(s, 0, sizeof *s);
+        return;
+    }
     free(s->id);
     free(s->pos);
     free(s->len);
@@ -763,14 +717,7 @@ fgss_status fgss_tokenize_dual(fgss_ctx* ctx, const char* text_r, uint64_t n_r, 
                 d.n_sets = cnt[sd];
                 d.n_tokens = tok[sd];
                 d.n_terms = all.n_terms;
-                const size_t nb = (cnt[sd] ? cnt[sd] : 1) * 4, tb = (tok[sd] ? tok[sd] : 1) * 4;
-                d.id = (uint32_t*)malloc(nb);
-                d.pos = (uint32_t*)malloc(nb);
-                d.len = (uint32_t*)malloc(nb);
-                d.tokens = (uint32_t*)malloc(tb);
-                d.loc = all.loc ? (uint32_t*)malloc(tb) : nullptr;
-                if (!d.id || !d.pos || !d.len || !d.tokens || (all.loc && !d.loc))
-                    fail(FGSS_ERR_NOMEM, "host allocation for token sets");
+                alloc_host_sets(&d, cnt[sd], tok[sd], all.loc != nullptr);
             }
             uint64_t at[2] = {0, 0}, ti[2] = {0, 0};
             for (uint64_t i = 0; i < all.n_sets; i++) {

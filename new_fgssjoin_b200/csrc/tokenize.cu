@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "pinned.h"
 #include "prims.cuh"
 #include "tokenize.h"
 
@@ -484,12 +485,7 @@ void tokenize_device(Ctx& c, const char* text, uint64_t n_bytes, const TokParams
     out->n_sets = nrec;
     out->n_tokens = Tn;
     out->n_terms = V;
-    out->id = (uint32_t*)malloc(((uint64_t)nrec + 1) * 4);
-    out->len = (uint32_t*)malloc(((uint64_t)nrec + 1) * 4);
-    out->pos = (uint32_t*)malloc(((uint64_t)nrec + 1) * 4);
-    out->tokens = (uint32_t*)malloc((Tn + 1) * 4);
-    out->loc = (uint32_t*)malloc((Tn + 1) * 4);
-    if (!out->id || !out->len || !out->pos || !out->tokens || !out->loc) fail(FGSS_ERR_NOMEM, "host allocation");
+    alloc_host_sets(out, nrec, Tn, true);
     if (nrec) {
         FGSS_CK(cudaMemcpyAsync(out->id, mid, (uint64_t)nrec * 4, cudaMemcpyDeviceToHost, c.stream));
         FGSS_CK(cudaMemcpyAsync(out->len, mlen, (uint64_t)nrec * 4, cudaMemcpyDeviceToHost, c.stream));

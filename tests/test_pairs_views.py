@@ -63,3 +63,27 @@ def test_empty_result_frees_its_struct():
     del out
     gc.collect()
     assert host._L.freed == [None]
+
+
+def test_token_sets_are_views_freed_once_after_the_last_array(monkeypatch):
+    class Lib:
+        freed = []
+
+        def fgss_sets_free(self, sref):
+            self.freed.append(ctypes.cast(sref._obj.id, ctypes.c_void_p).value)
+
+    monkeypatch.setattr(B, "load_library", lambda: Lib())
+    cols = [np.arange(k, k + 40, dtype=np.uint32) for k in range(5)]
+    s = B._Sets()
+    s.id, s.pos, s.len, s.tokens, s.loc = [c.ctypes.data_as(B._u32p) for c in cols]
+    s.n_sets, s.n_tokens, s.n_terms = 40, 40, 80
+    got = B.Sets._from_c(s)
+    for a, want in zip((got.id, got.pos, got.len, got.tokens, got.loc), cols):
+        assert a.ctypes.data == want.ctypes.data and np.array_equal(a, want)
+    keep = got.tokens[5:9]
+    del got, a
+    gc.collect()
+    assert Lib.freed == [] and keep[0] == cols[3][5]
+    del keep
+    gc.collect()
+    assert Lib.freed == [cols[0].ctypes.data]
