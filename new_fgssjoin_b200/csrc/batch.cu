@@ -604,6 +604,13 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
                 else if (model) v = std::max<uint64_t>((uint64_t)((double)hsum[2 * nj + 4 + i] * 1.5) + 4096, last);
                 else v = std::max<uint64_t>(J.in.n_sets + 4096, last);
                 cap[i] = std::min<uint64_t>(v, 0xfffffff0ull);
+                if (model && !J.res_cap_hint && !J.res_cap_user && cap[i] > (1ull << 26)) {
+                    // a wild estimate must not take the device's memory (about 48 bytes a
+                    // slot): too small a buffer only costs an exact re-run
+                    size_t free_b = 0, total_b = 0;
+                    FGSS_CK(cudaMemGetInfo(&free_b, &total_b));
+                    cap[i] = std::min<uint64_t>(cap[i], std::max<uint64_t>({J.in.n_sets + 4096, last, free_b / 256}));
+                }
             }
             capoff[i + 1] = capoff[i] + cap[i];
         }
