@@ -44,6 +44,10 @@ template <typename F>
 fgss_status guard(fgss_ctx* ctx, F&& f) {
     try {
         f();
+        if (ctx && ctx->c.err_host && *(volatile uint32_t*)ctx->c.err_host) {
+            *ctx->c.err_host = 0;
+            fail(FGSS_ERR_TIMEOUT, "a device wait of a scan or sort gave up");
+        }
         if (ctx) ctx->c.last_error.clear();
         return FGSS_OK;
     } catch (const Error& e) {
@@ -601,6 +605,9 @@ fgss_status fgss_create(fgss_ctx** out, const fgss_options* opt) {
             c.own_stream = true;
         }
         for (auto& e : c.ev) FGSS_CK(cudaEventCreate(&e));
+        FGSS_CK(cudaHostAlloc((void**)&c.err_host, 4, cudaHostAllocMapped));
+        *c.err_host = 0;
+        FGSS_CK(cudaHostGetDevicePointer((void**)&c.err_dev, c.err_host, 0));
         tune_load(c);
         c.graphs = new GraphCache();
     });
@@ -627,6 +634,7 @@ void fgss_destroy(fgss_ctx* ctx) {
         if (kv.second.p) cudaFreeHost(kv.second.p);
     for (auto& e : c.ev)
         if (e) cudaEventDestroy(e);
+    if (c.err_host) cudaFreeHost(c.err_host);
     if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);
     delete c.model;
     delete ctx;

@@ -95,6 +95,11 @@ struct Ctx {
         return static_cast<T*>(pinned(name, count * sizeof(T)));
     }
     void sync() { FGSS_CK(cudaStreamSynchronize(stream)); }
+    // Error word the kernels' bounded waits set (mapped page-locked memory, so
+    // reading it after a wait costs no copy); made with the context.
+    uint32_t* err_host = nullptr;
+    uint32_t* err_dev = nullptr;
+    uint32_t* dev_err() const { return err_dev; }
     // Frees every pooled device buffer whose name starts with `prefix`.
     void release_prefix(const std::string& prefix) {
         for (auto it = bufs.begin(); it != bufs.end();) {
