@@ -98,6 +98,7 @@ fgss_status fgss_model_train(fgss_ctx* ctx, const fgss_sets_view* sets, const fl
         c.last_error.clear();
         return FGSS_OK;
     } catch (const Error& e) {
+        if (cudaStreamSynchronize(ctx->c.stream) != cudaSuccess) (void)cudaGetLastError();  // copies from the caller's arrays
         ctx->c.last_error = e.msg;
         return e.st;
     }
