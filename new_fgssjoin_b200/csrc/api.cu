@@ -339,7 +339,7 @@ bool replay_graph(Ctx& c, GraphEntry& g, const fgss_sets_view* sets, const fgss_
     // validation, fresh counters and the index and probe totals; the graph
     // holds every later stage
     batch_prep(c, B, v, sets, opts);
-    if (B.E > g.plan.E_cap || B.P > g.plan.P_cap) {
+    if (B.E > g.plan.E_cap || B.P > g.plan.P_cap || (g.plan.light && B.keyed_possible)) {
         c.bpfx.clear();
         return false;
     }
@@ -349,9 +349,7 @@ bool replay_graph(Ctx& c, GraphEntry& g, const fgss_sets_view* sets, const fgss_
     c.probe_timed = true;
     c.heavy_timed = g.plan.heavy_slots > 0;
     FGSS_CK(cudaEventRecord(c.ev[2], c.stream));
-    uint32_t* h = c.pinnedT<uint32_t>(g.ns + "h.st", 8 * (size_t)n);
-    FGSS_CK(cudaMemcpyAsync(h, B.status, 32 * (size_t)n, cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
+    const uint32_t* h = batch_read_status(c, B);
     for (int i = 0; i < n; i++) {
         const uint32_t bad = ST_RES_OVERFLOW | ST_HEAVY_OVERFLOW | ST_HASH_FULL;
         if ((h[8 * i] & bad) || h[8 * i + 3] > g.plan.res_cap[i]) {
@@ -426,8 +424,9 @@ void run_joins(Ctx& c, const fgss_sets_view* sets, const fgss_join_opts* opts, i
     std::unique_ptr<Batch> Bp(new Batch());
     try {
         if (!batched) {
-            FGSS_CK(cudaEventRecord(ev[0], c.stream));
+            // the joins one after another, in the same batch-level buffers
             for (int i = 0; i < n; i++) {
+                FGSS_CK(cudaEventRecord(ev[0], c.stream));
                 fgss_sets_view v = sets[i];
                 if (!v.on_device) {
                     // the same host arrays as an earlier join of the batch: copied to the device once
@@ -441,18 +440,21 @@ void run_joins(Ctx& c, const fgss_sets_view* sets, const fgss_join_opts* opts, i
                         }
                     }
                 }
-                join_setup(c, *js[i], v, opts[i], i, false);
+                Batch B;
+                batch_prep(c, B, {jv[i]}, &v, opts + i);
+                batch_index(c, B, B.E);
+                FGSS_CK(cudaEventRecord(ev[1], c.stream));
+                plain_filter_verify(c, B, opts[i].want_candidates != 0);
+                FGSS_CK(cudaEventRecord(ev[2], c.stream));
+                const uint64_t n_res = js[i]->n_res;
+                batch_finish_status(c, B);
+                js[i]->n_res = n_res;
+                add_times(c, times);
             }
-            c.sync();  // one wait for the whole batch's input validation
-            for (int i = 0; i < n; i++) join_check_input(c, *js[i]);
-            for (int i = 0; i < n; i++) join_index(c, *js[i]);
+            FGSS_CK(cudaEventRecord(ev[0], c.stream));
             FGSS_CK(cudaEventRecord(ev[1], c.stream));
-            for (int i = 0; i < n; i++) join_plain_filter_verify(c, *js[i], opts[i].want_candidates != 0);
             FGSS_CK(cudaEventRecord(ev[2], c.stream));
-            for (int i = 0; i < n; i++) {
-                join_finish_status(c, *js[i]);
-                export_pairs(c, *js[i], opts[i], &outs[i]);
-            }
+            for (int i = 0; i < n; i++) export_pairs(c, *js[i], opts[i], &outs[i]);
             add_times(c, times);
         } else {
             for (const auto& gr : groups) {
@@ -777,12 +779,14 @@ fgss_status fgss_rsjoin(fgss_ctx* ctx, const fgss_sets_view* r, const fgss_sets_
             FGSS_CK(cudaEventRecord(ev[2], c.stream));
             batch_finish_status(c, B);
         } else {
-            join_setup(c, J, u.view, *opts, 0);
-            join_index(c, J);
+            batch_prep(c, B, v, &u.view, opts);
+            batch_index(c, B, B.E);
             FGSS_CK(cudaEventRecord(ev[1], c.stream));
-            join_plain_filter_verify(c, J, false);
+            plain_filter_verify(c, B, false);
             FGSS_CK(cudaEventRecord(ev[2], c.stream));
-            join_finish_status(c, J);
+            const uint64_t n_res = J.n_res;
+            batch_finish_status(c, B);
+            J.n_res = n_res;
         }
         rs_output(c, J, u);
         export_pairs(c, J, *opts, out);

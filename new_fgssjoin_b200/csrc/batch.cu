@@ -139,27 +139,47 @@ namespace {
 using Claim = ClaimShape<256, 8, 13>;
 constexpr int kClaimCtas = 3;
 
-template <bool SIDED>
-void claim_launch_as(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const uint4* items, uint32_t n_items,
+template <int MODE, bool SIDED>
+void claim_launch_as(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const ClaimItems& items,
                      uint32_t* counter) {
-    FGSS_CK(cudaFuncSetAttribute(k_claim<Claim, kClaimCtas, SIDED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    FGSS_CK(cudaFuncSetAttribute(k_claim<Claim, kClaimCtas, MODE, SIDED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)Claim::bytes));
-    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)kClaimCtas * c.num_sms, n_items);
-    k_claim<Claim, kClaimCtas, SIDED><<<grid, Claim::NT, Claim::bytes, c.stream>>>(d_args, d_fargs, items, n_items,
-                                                                                   counter);
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)kClaimCtas * c.num_sms, items.n);
+    k_claim<Claim, kClaimCtas, MODE, SIDED><<<grid, Claim::NT, Claim::bytes, c.stream>>>(d_args, d_fargs, items, counter);
     FGSS_LAUNCH_CK();
 }
 
-void claim_launch(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const uint4* items, uint32_t n_items,
-                  uint32_t* counter, bool sided) {
-    if (sided) claim_launch_as<true>(c, d_args, d_fargs, items, n_items, counter);
-    else claim_launch_as<false>(c, d_args, d_fargs, items, n_items, counter);
+template <int MODE>
+void claim_launch(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const ClaimItems& items, uint32_t* counter,
+                  bool sided) {
+    if (sided) claim_launch_as<MODE, true>(c, d_args, d_fargs, items, counter);
+    else claim_launch_as<MODE, false>(c, d_args, d_fargs, items, counter);
 }
 
+// m in tiles small enough to make at least `want` of them, but not below `low` records.
+TileMap tiles_for(const TileMap& m, uint64_t want, uint32_t low) {
+    uint32_t tile = m.tile;
+    while (tile > low && (uint64_t)m.ntiles * (m.tile / tile) < want) tile >>= 1;
+    return finer_tiles(m, tile);
+}
+
+// Tiles of the warp-per-record stages: small enough to give every SM 8 CTAs of 8 warps
+// as long as a warp still has a record (500 titles: k_windows_mj 40 -> 4.1 us,
+// k_bitmaps_mj 32 -> 3.3, k_index_entries_mj 21 -> 2.9 with tiles of 8 instead of 256).
+TileMap warp_tiles(Ctx& c, const TileMap& m) { return tiles_for(m, (uint64_t)8 * c.num_sms, 8); }
+
+// Items of the records in order: about 128 per CTA.
+ClaimItems items_in_order(Ctx& c, const TileMap& m) {
+    const TileMap t = tiles_for(m, (uint64_t)128 * kClaimCtas * c.num_sms, 1);
+    return {nullptr, t, t.ntiles};
+}
+
+template <int MODE>
 void tiny_launch(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const TileMap& m, bool sided) {
-    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)m.ntiles * (m.tile / 32), (uint64_t)c.num_sms * 16);
-    if (sided) k_tiny<true><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, m);
-    else k_tiny<false><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, m);
+    const TileMap t = tiles_for(finer_tiles(m, 32), (uint64_t)8 * c.num_sms, kTinyWarps);
+    const unsigned grid = std::min<unsigned>(t.ntiles, (unsigned)c.num_sms * 16);
+    if (sided) k_tiny<MODE, true><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, t);
+    else k_tiny<MODE, false><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, t);
     FGSS_LAUNCH_CK();
 }
 
@@ -191,6 +211,7 @@ TileMap upload_tiles(Ctx& c, const std::string& name, const std::vector<uint64_t
     m.nj = (uint32_t)nj;
     m.tile = tile;
     m.ntiles = (uint32_t)t;
+    m.split = 1;
     return m;
 }
 
@@ -212,8 +233,8 @@ void index_sort(Ctx& c, Batch& B, uint64_t E_cap, int tbits, int jbits, const ui
     const std::string& p = c.bpfx;
     K* key = c.devT<K>(p + "b.ix.key", E_cap + 1);
     uint64_t* val = c.devT<uint64_t>(p + "b.ix.val", E_cap + 1);
-    k_index_entries_mj<K><<<tile_grid(c, B.rec), 256, 0, c.stream>>>(B.d_args, B.rec, B.ioff, (uint32_t)tbits, key,
-                                                                      val);
+    const TileMap wt = warp_tiles(c, B.rec);
+    k_index_entries_mj<K><<<tile_grid(c, wt), 256, 0, c.stream>>>(B.d_args, wt, B.ioff, (uint32_t)tbits, key, val);
     FGSS_LAUNCH_CK();
     radix_sort<K, uint64_t>(c, key, val, E_cap, d_E, 0, tbits + jbits, (p + "b.ixsort").c_str());
     k_index_lists_mj<K><<<grid_for(E_cap, 256, c.num_sms * 32), 256, 0, c.stream>>>(
@@ -237,7 +258,8 @@ struct Prepass {
     size_t n_sums = 0;
 };
 
-Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bool model, bool classes) {
+// light: the windows and classes only.
+Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bool model, bool classes, bool light = false) {
     const size_t nj = B.js.size();
     const std::string& p = c.bpfx;
     const uint64_t R = B.R;
@@ -246,6 +268,15 @@ Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bo
     pp.wpre = c.devT<uint32_t>(p + "b.wpre", P_cap + 1);
     pp.wtot = c.devT<uint32_t>(p + "b.wtot", R + 1);
     pp.meta = c.devT<uint4>(p + "b.meta", R + 1);
+    const TileMap wt = warp_tiles(c, B.rec);
+    const unsigned wg = tile_grid(c, wt);
+    if (light) {
+        if (R) {
+            k_windows_mj<<<wg, 256, 0, c.stream>>>(B.d_args, wt, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, classes);
+            FGSS_LAUNCH_CK();
+        }
+        return pp;
+    }
     float* feat = c.devT<float>(p + "b.feat", (R + 1) * kFeatures);
     uint32_t* pred = c.devT<uint32_t>(p + "b.pred", R + 1);
     pp.cost[0] = c.devT<uint64_t>(p + "b.cost0", R + 1);
@@ -254,16 +285,15 @@ Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bo
     pp.d_sums = c.devT<uint64_t>(p + "b.sums", pp.n_sums);
     FGSS_CK(cudaMemsetAsync(pp.d_sums, 0, pp.n_sums * 8, c.stream));
     if (R == 0) return pp;
-    const unsigned g = tile_grid(c, B.rec);
-    k_windows_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, classes);
+    k_windows_mj<<<wg, 256, 0, c.stream>>>(B.d_args, wt, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, classes);
     FGSS_LAUNCH_CK();
     if (model) {
         pp.pred = pred;
-        k_features_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, feat);
+        k_features_mj<<<wg, 256, 0, c.stream>>>(B.d_args, wt, feat);
         FGSS_LAUNCH_CK();
         model_predict_tiles(c, feat, B.rec, pred, pp.d_sums + 2 * nj + 4, pp.d_sums + 3 * nj + 4);
     }
-    k_cost_mj<<<g, 256, 0, c.stream>>>(B.d_args, B.rec, pp.meta, pp.pred, cap_entries, pp.cost[0], pp.cost[1],
+    k_cost_mj<<<tile_grid(c, B.rec), 256, 0, c.stream>>>(B.d_args, B.rec, pp.meta, pp.pred, cap_entries, pp.cost[0], pp.cost[1],
                                        (unsigned long long*)pp.d_sums);
     FGSS_LAUNCH_CK();
     return pp;
@@ -332,11 +362,12 @@ FusedArgs* batch_filters(Ctx& c, Batch& B, const Prepass& pp, uint32_t cap_entri
     unsigned long long* cused = c.devT<unsigned long long>(p + "b.cused", 1);
     FGSS_CK(cudaMemsetAsync(cused, 0, 8, c.stream));
     if (R == 0) return d_fargs;
-    const unsigned g = tile_grid(c, B.rec);
-    k_bitmaps_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, B.rec);
+    const TileMap wt = warp_tiles(c, B.rec);
+    const unsigned g = tile_grid(c, wt);
+    k_bitmaps_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, wt);
     FGSS_LAUNCH_CK();
     if (!chunks) return d_fargs;  // no query for k_fused
-    k_chunks_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, B.rec, pp.wtot, cap_entries, cbuf, cbuf_cap, cused);
+    k_chunks_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, wt, pp.wtot, cap_entries, cbuf, cbuf_cap, cused);
     FGSS_LAUNCH_CK();
     return d_fargs;
 }
@@ -438,8 +469,12 @@ void batch_prep(Ctx& c, Batch& B, const std::vector<JoinState*>& js, const fgss_
     FGSS_CK(cudaMemcpyAsync(h + nj * 8, B.ioff + B.R, 4, cudaMemcpyDeviceToHost, c.stream));
     FGSS_CK(cudaMemcpyAsync(h + nj * 8 + 1, B.poff + B.R, 4, cudaMemcpyDeviceToHost, c.stream));
     c.sync();
-    for (size_t j = 0; j < nj; j++)
+    B.keyed_possible = false;
+    B.status_host = nullptr;
+    for (size_t j = 0; j < nj; j++) {
         if (js[j]->in.n_sets) check_input_status(h[8 * j]);
+        B.keyed_possible |= js[j]->lut.probe_max[std::min<uint32_t>(h[8 * j + 1], kMaxLen)] > kClaimPC;
+    }
     B.E = h[nj * 8];
     B.P = h[nj * 8 + 1];
 }
@@ -525,7 +560,12 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     // the caller's own choice of a strategy, a tuned keyed shape and the global accumulator take every query
     bool classes = te.heavy_min_probe == 0 && !te.keyed;
     for (size_t i = 0; i < nj; i++) classes &= joins[i]->filter == FGSS_FILTER_AUTO;
-    const Prepass pp = batch_prepass(c, B, cap_entries, P_cap, model, classes);
+    // light: no query can be k_fused's and there is no learned estimate to order them by, so
+    // k_claim takes the records in order and the costs, items and their sort, and the wait
+    // for their counts, are left out (1,000 titles: 60 us of 450)
+    const bool light = capture ? plan->light : classes && !model && !B.keyed_possible && B.R != 0;
+    if (plan && !capture) plan->light = light;
+    const Prepass pp = batch_prepass(c, B, cap_entries, P_cap, model, classes, light);
 
     // work items per class of k_fused and k_claim: ~256 per resident CTA over
     // the whole batch (a few queries per item at 100k records), split by cost
@@ -535,8 +575,10 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     std::vector<uint32_t> K[2] = {std::vector<uint32_t>(nj, 0), std::vector<uint32_t>(nj, 0)};
     uint64_t nitems[2] = {0, 0};
     bool tiny = classes && B.R != 0;
-    uint64_t* hsum = c.pinnedT<uint64_t>(p + "b.hsum", pp.n_sums);
-    if (capture) {
+    uint64_t* hsum = c.pinnedT<uint64_t>(p + "b.hsum", std::max<size_t>(pp.n_sums, 1));
+    if (light) {
+        // nothing to read back
+    } else if (capture) {
         for (int k = 0; k < 2; k++) {
             K[k] = plan->K[k];
             nitems[k] = plan->nitems[k];
@@ -571,12 +613,14 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     if (nitems[0] >= 0xffffffffull || nitems[1] >= 0xffffffffull) fail(FGSS_ERR_UNSUPPORTED, "too many work items");
     // chunk boundaries: exactly the words the splits take (the plan's size in
     // a capture; a replay on other data that needs more bisects instead)
-    const uint64_t cbuf_cap = capture ? plan->cbuf_cap : std::min<uint64_t>(hsum[2 * nj + 3], 0xfffffff0ull);
+    const uint64_t cbuf_cap = light ? 0 : capture ? plan->cbuf_cap : std::min<uint64_t>(hsum[2 * nj + 3], 0xfffffff0ull);
     if (plan && !capture) plan->cbuf_cap = cbuf_cap;
     FusedArgs* d_fargs = batch_filters(c, B, pp, cap_entries, cbuf_cap, nitems[QC_KEYED] != 0);
     const uint4* items[2] = {nullptr, nullptr};
     for (int k = 0; k < 2; k++)
         if (nitems[k]) items[k] = batch_items(c, B, pp, k, K[k], nitems[k]);
+    const ClaimItems claims = light ? items_in_order(c, B.rec)
+                                    : ClaimItems{items[QC_CLAIM], B.rec, (uint32_t)nitems[QC_CLAIM]};
 
     bool sided = false;
     for (size_t i = 0; i < nj; i++) sided |= joins[i]->args.side != nullptr;
@@ -628,11 +672,10 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
         upload_args(c, B, p + "b.ha2");
         FGSS_CK(cudaMemsetAsync(counter, 0, (4 + nj) * 4, c.stream));
         FGSS_CK(cudaEventRecordWithFlags(c.ev[4], c.stream, rec_flags));
-        if (nitems[QC_CLAIM])
-            claim_launch(c, B.d_args, d_fargs, items[QC_CLAIM], (uint32_t)nitems[QC_CLAIM], counter + 1, sided);
+        if (claims.n) claim_launch<MODE_FUSED>(c, B.d_args, d_fargs, claims, counter + 1, sided);
         if (nitems[QC_KEYED])
             fused_launch(c, te, B.d_args, d_fargs, items[QC_KEYED], (uint32_t)nitems[QC_KEYED], counter, sided);
-        if (tiny) tiny_launch(c, B.d_args, d_fargs, B.rec, sided);
+        if (tiny) tiny_launch<MODE_FUSED>(c, B.d_args, d_fargs, B.rec, sided);
         FGSS_CK(cudaEventRecordWithFlags(c.ev[5], c.stream, rec_flags));
         c.probe_timed = true;
         // queries deferred to the global-memory accumulator: one persistent
@@ -640,13 +683,13 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
         // plan always, with scratch for a fixed slot count (a launch whose
         // queues are empty returns at once).
         uint32_t max_nh = 0;
-        if (!capture) {
+        if (!capture && !plan && nitems[QC_KEYED]) {  // only k_fused defers queries
             FGSS_CK(cudaMemcpyAsync(hst, B.status, nj * 32, cudaMemcpyDeviceToHost, c.stream));
             c.sync();
             for (size_t i = 0; i < nj; i++) max_nh = std::max(max_nh, hst[8 * i + 2]);
         }
         const uint32_t all_slots = std::min<uint32_t>(std::max<uint32_t>(B.n_max, 1), (uint32_t)c.num_sms);
-        slots = capture ? plan->heavy_slots : plan ? all_slots : std::min<uint32_t>(max_nh, (uint32_t)c.num_sms);
+        slots = light ? 0 : capture ? plan->heavy_slots : plan ? all_slots : std::min<uint32_t>(max_nh, (uint32_t)c.num_sms);
         if (slots) {
             const HeavyScratch hs = heavy_scratch(c, p, B.n_max, slots, capture);
             FGSS_CK(cudaEventRecordWithFlags(c.ev[6], c.stream, rec_flags));
@@ -658,12 +701,11 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
             c.heavy_timed = true;
         }
         if (capture) break;
-        FGSS_CK(cudaMemcpyAsync(hst, B.status, nj * 32, cudaMemcpyDeviceToHost, c.stream));
-        c.sync();
+        const uint32_t* st = batch_read_status(c, B);
         bool over = false;
         for (size_t i = 0; i < nj; i++) {
             JoinState& J = *joins[i];
-            const uint32_t got = hst[8 * i + 3];
+            const uint32_t got = st[8 * i + 3];
             if (got > cap[i]) {
                 // The learned (or remembered) capacity was too small: the kernel
                 // kept counting, so the batch re-runs with the exact size.  A
@@ -696,7 +738,7 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
             rcap[i] = cap[i];
             continue;
         }
-        const uint32_t got = hst[8 * i + 3];
+        const uint32_t got = B.status_host[8 * i + 3];
         J.n_res = got;
         J.res_cap_hint = 0;
         // remember a sufficient capacity for the next call on this slot
@@ -742,7 +784,146 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     FGSS_LAUNCH_CK();
 }
 
-void batch_finish_status(Ctx& c, Batch& B) {
+namespace {
+
+__global__ void k_sum_u32(const uint32_t* __restrict__ in, uint64_t n, unsigned long long* out) {
+    unsigned long long s = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        s += in[i];
+    s = warp_sum(s);
+    if (lane_id() == 0 && s) atomicAdd(out, s);
+}
+
+template <int MODE, int NT, int HLOG>
+void probe_launch(Ctx& c, const JoinArgs* d_args, uint64_t n) {
+    FGSS_CK(cudaFuncSetAttribute(k_probe<MODE, NT, HLOG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ProbeLayout<MODE, HLOG>::bytes));
+    k_probe<MODE, NT, HLOG><<<(unsigned)n, NT, ProbeLayout<MODE, HLOG>::bytes, c.stream>>>(d_args);
+    FGSS_LAUNCH_CK();
+}
+
+}  // namespace
+
+void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
+    JoinState& J = *B.js[0];
+    const uint64_t n = J.in.n_sets;
+    JoinArgs& a = J.args;
+    J.n_res = 0;
+    if (n == 0) return;
+    const std::string& p = c.bpfx;
+    // ---- pre-pass: windows and classes of the queries; k_claim takes the records in order
+    const Prepass pp = batch_prepass(c, B, 1u << 30, B.P, false, true, true);
+    const bool keyed = B.keyed_possible, sided = a.side != nullptr;
+    const ClaimItems claims = items_in_order(c, B.rec);
+    FusedArgs* d_fargs = batch_filters(c, B, pp, 1u << 30, 0, false);
+    const FusedArgs& fa = c.pinnedT<FusedArgs>(p + "b.hf", 1)[0];
+    a.meta = pp.meta;
+    a.vcnt = c.devT<uint32_t>(J.pfx("vcnt"), n + 1);
+    a.ccnt = c.devT<uint32_t>(J.pfx("ccnt"), n + 1);
+    a.wcnt = c.devT<uint32_t>(J.pfx("wcnt"), n + 1);
+    uint32_t* voff = c.devT<uint32_t>(J.pfx("voff"), n + 1);
+    a.voff = voff;
+    uint32_t* hcnt = c.pinnedT<uint32_t>(J.pfx("h.cnt"), 8);
+    // words: candidates, results (64-bit, the scans write the low halves), then per pass
+    // the counters of the work items and of the queue of the global accumulator
+    uint32_t* ctr = c.devT<uint32_t>(J.pfx("words"), 8);
+    uint64_t* d_nc = reinterpret_cast<uint64_t*>(ctr);
+    J.d_nres = d_nc + 1;
+    ctr += 4;
+    FGSS_CK(cudaMemsetAsync(a.vcnt, 0, n * 4, c.stream));
+    FGSS_CK(cudaMemsetAsync(d_nc, 0, 32, c.stream));
+    // ---- count pass
+    upload_args(c, B, p + "b.ha2");
+    claim_launch<MODE_COUNT>(c, B.d_args, d_fargs, claims, ctr, sided);
+    tiny_launch<MODE_COUNT>(c, B.d_args, d_fargs, B.rec, sided);
+    HeavyScratch hs;
+    uint32_t hslots = 0;
+    if (keyed) {
+        // probe prefixes above kClaimPC: the keyed table, or the global accumulator
+        FGSS_CK(cudaMemsetAsync(a.ccnt, 0, n * 4, c.stream));
+        FGSS_CK(cudaMemsetAsync(a.wcnt, 0, n * 4, c.stream));
+        FGSS_CK(cudaMemsetAsync(a.heavy_count, 0, 4, c.stream));
+        probe_launch<MODE_COUNT, 256, 12>(c, B.d_args, n);
+        FGSS_CK(cudaMemcpyAsync(hcnt, a.heavy_count, 4, cudaMemcpyDeviceToHost, c.stream));
+        c.sync();
+        hslots = std::min<uint32_t>(hcnt[0], (uint32_t)c.num_sms);
+        if (hslots) {
+            hs = heavy_scratch(c, "", n, hslots, false);
+            k_probe_heavy<MODE_COUNT, 512><<<hslots, 512, 0, c.stream>>>(B.d_args, 0, 1, hs.zero, hs.zero_words, hs.aux,
+                                                                         hs.aux_words, ctr + 1);
+            FGSS_LAUNCH_CK();
+        }
+        k_sum_u32<<<grid_for(n, 256, c.num_sms * 8), 256, 0, c.stream>>>(a.ccnt, n, &J.stats[SS_CANDIDATES]);
+        FGSS_LAUNCH_CK();
+        k_sum_u32<<<grid_for(n, 256, c.num_sms * 8), 256, 0, c.stream>>>(a.wcnt, n, &J.stats[SS_WINDOW]);
+        FGSS_LAUNCH_CK();
+    }
+    exclusive_scan<uint32_t>(c, a.vcnt, voff, n, nullptr, reinterpret_cast<uint32_t*>(d_nc), J.pfx("scan.v").c_str());
+    FGSS_CK(cudaMemcpyAsync(hcnt, d_nc, 4, cudaMemcpyDeviceToHost, c.stream));
+    c.sync();
+    const uint64_t C = hcnt[0];
+    // ---- fill pass
+    uint4* cand = c.devT<uint4>(J.pfx("cand"), C + 1);
+    a.cand = cand;
+    if (C) {
+        FGSS_CK(cudaMemsetAsync(a.ccnt, 0, n * 4, c.stream));
+        ctr += 2;
+        if (keyed) FGSS_CK(cudaMemsetAsync(a.heavy_count, 0, 4, c.stream));
+        upload_args(c, B, p + "b.ha2");
+        claim_launch<MODE_FILL>(c, B.d_args, d_fargs, claims, ctr, sided);
+        tiny_launch<MODE_FILL>(c, B.d_args, d_fargs, B.rec, sided);
+        if (keyed) probe_launch<MODE_FILL, 256, 12>(c, B.d_args, n);
+        if (hslots) {
+            k_probe_heavy<MODE_FILL, 512><<<hslots, 512, 0, c.stream>>>(B.d_args, 0, 1, hs.zero, hs.zero_words, hs.aux,
+                                                                        hs.aux_words, ctr + 1);
+            FGSS_LAUNCH_CK();
+        }
+    }
+    if (want_cand) {
+        std::vector<uint4> hc(C);
+        if (C) FGSS_CK(cudaMemcpyAsync(hc.data(), cand, C * 16, cudaMemcpyDeviceToHost, c.stream));
+        c.sync();
+        J.cand_host.resize(3 * C);
+        for (uint64_t i = 0; i < C; i++) {
+            J.cand_host[3 * i] = hc[i].x;
+            J.cand_host[3 * i + 1] = hc[i].y;
+            J.cand_host[3 * i + 2] = hc[i].z;
+        }
+    }
+    if (C == 0) return;
+    // ---- verification (thread-per-candidate merge in the reference; see k_verify)
+    uint32_t* ov = c.devT<uint32_t>(J.pfx("ov"), C + 1);
+    uint32_t per = 32;
+    while (per > 1 && C < (uint64_t)per * 64 * c.num_sms) per >>= 1;
+    k_verify<<<grid_for((C + per - 1) / per * 32, 256, c.num_sms * 32), 256, 0, c.stream>>>(a, cand, d_nc, per, ov,
+                                                                                            fa.bmap, fa.bmw);
+    FGSS_LAUNCH_CK();
+    // ---- compaction of the verified pairs: count -> scan -> fill
+    uint32_t* flag = c.devT<uint32_t>(J.pfx("flag"), C + 1);
+    uint32_t* off = c.devT<uint32_t>(J.pfx("off"), C + 1);
+    k_result_flags<<<grid_for(C, 256, c.num_sms * 32), 256, 0, c.stream>>>(a, cand, ov, d_nc, flag);
+    FGSS_LAUNCH_CK();
+    exclusive_scan<uint32_t>(c, flag, off, C, nullptr, reinterpret_cast<uint32_t*>(J.d_nres),
+                             J.pfx("scan.r").c_str());
+    // up to 65,536 candidates the buffers and grids are theirs and the number of results
+    // is read back at the end: a wait here costs more than the launches it would shrink
+    FGSS_CK(cudaMemcpyAsync(hcnt + 2, J.d_nres, 4, cudaMemcpyDeviceToHost, c.stream));
+    const bool wait = C > 65536;
+    if (wait) c.sync();
+    const uint64_t R = wait ? hcnt[2] : C;
+    uint64_t* keys = c.devT<uint64_t>(J.pfx("rkey"), R + 1);
+    uint32_t* vals = c.devT<uint32_t>(J.pfx("rval"), R + 1);
+    if (R) {
+        k_result_fill<<<grid_for(C, 256, c.num_sms * 32), 256, 0, c.stream>>>(cand, ov, flag, off, d_nc,
+                                                                              (uint32_t)bits_for(n), keys, vals);
+        FGSS_LAUNCH_CK();
+    }
+    join_output(c, J, keys, vals, J.d_nres, R);
+    batch_read_status(c, B);
+    J.n_res = hcnt[2];
+}
+
+const uint32_t* batch_read_status(Ctx& c, Batch& B) {
     const size_t nj = B.js.size();
     uint32_t* h = c.pinnedT<uint32_t>(c.bpfx + "b.hfin", nj * 8);
     unsigned long long* hs = c.pinnedT<unsigned long long>(c.bpfx + "b.hfin.stats", nj * SS_N);
@@ -751,6 +932,15 @@ void batch_finish_status(Ctx& c, Batch& B) {
     FGSS_CK(cudaMemcpyAsync(hs, B.stats, nj * SS_N * 8, cudaMemcpyDeviceToHost, c.stream));
     FGSS_CK(cudaMemcpyAsync(he, B.d_e, nj * 16, cudaMemcpyDeviceToHost, c.stream));
     c.sync();
+    B.status_host = h;
+    return h;
+}
+
+void batch_finish_status(Ctx& c, Batch& B) {
+    const size_t nj = B.js.size();
+    const uint32_t* h = B.status_host ? B.status_host : batch_read_status(c, B);
+    const unsigned long long* hs = c.pinnedT<unsigned long long>(c.bpfx + "b.hfin.stats", nj * SS_N);
+    const uint64_t* he = c.pinnedT<uint64_t>(c.bpfx + "b.hfin.E", nj * 2);
     for (size_t j = 0; j < nj; j++) {
         B.js[j]->n_entries = he[2 * j];
         B.js[j]->n_res = h[8 * j + 3];

@@ -22,13 +22,26 @@
 
 namespace fgss {
 
-// The bitmap bound of one source that passed the position test: does it still
-// need a merge?  q4: the query's bitmap (shared or global memory).
-__device__ __forceinline__ bool bitmap_keeps(const uint4* q4, const uint4* __restrict__ b4, uint32_t bmw, uint32_t S,
-                                             uint32_t im) {
-    uint32_t pc = popc_xor(q4[0], __ldg(b4)) + popc_xor(q4[1], __ldg(b4 + 1));
-    if (bmw == 4) pc += popc_xor(q4[2], __ldg(b4 + 2)) + popc_xor(q4[3], __ldg(b4 + 3));
-    return S >= 2 * im + pc;
+// The kernels run in three modes: MODE_FUSED verifies and emits the results (the
+// batched method); MODE_COUNT adds every query's sources that need verification to
+// a.vcnt, MODE_FILL writes them as (query, source, matches, query position of the
+// last) from a.cand[a.voff[query]] (the plain method's two passes; a.ccnt is the
+// fill's cursor, zero at launch).  Candidates and window entries are counted in the
+// first two.
+
+// Lanes' sources of one query into the plain method's counts or records
+// (warp-collective): bit `take` lanes give (s, cj = matches | query position << 16).
+template <int MODE>
+__device__ __forceinline__ void plain_take(const JoinArgs& a, uint32_t q, bool take, uint32_t s, uint32_t cj) {
+    const uint32_t m = __ballot_sync(kFull, take);
+    if (m == 0) return;
+    uint32_t base = 0;
+    if (lane_id() == 0) base = atomicAdd(MODE == MODE_COUNT ? &a.vcnt[q] : &a.ccnt[q], (uint32_t)__popc(m));
+    if (MODE == MODE_COUNT) return;
+    const uint32_t i = __shfl_sync(kFull, base, 0) + __popc(m & lanemask_lt());
+    if (!take) return;
+    if (i < a.vcnt[q]) a.cand[a.voff[q] + i] = make_uint4(q, s, cj & 0xffffu, cj >> 16);
+    else atomicOr(a.status, ST_HASH_FULL);
 }
 
 __device__ __forceinline__ void bar_named(uint32_t id, uint32_t threads) {
@@ -72,6 +85,20 @@ struct ClaimShape {
     static_assert(MC <= 32 * NWC, "a warp's share of the merge list fits its lanes");
 };
 
+// Work items of k_claim: a list of (join, first query, end), or without one the
+// tiles of the map in order -- records come in descending size, so the costly
+// queries still come first.
+struct ClaimItems {
+    const uint4* list;
+    TileMap m;
+    uint32_t n;
+};
+__device__ __forceinline__ uint4 claim_item(const ClaimItems& I, uint32_t it) {
+    if (I.list) return I.list[it];
+    const TileRange t = tile_range(I.m, it);
+    return make_uint4(t.j, t.r0, t.r1, 0);
+}
+
 // What the consumers do next: the entries of a range of the query's id
 // window, laid out in rank form in buffer (step & 1).
 struct ClaimStep {
@@ -85,18 +112,17 @@ enum : uint32_t {
 
 // Producer warp: walks the work items and lays out the steps, one ahead of
 // the consumers.
-template <typename S>
+template <typename S, int MODE>
 __device__ void claim_producer(const JoinArgs* __restrict__ joins, const FusedArgs* __restrict__ fargs,
-                               const uint4* __restrict__ items, uint32_t n_items, uint32_t* counter,
-                               unsigned char* smem, ClaimStep* steps) {
+                               const ClaimItems& items, uint32_t* counter, unsigned char* smem, ClaimStep* steps) {
     const uint32_t lane = lane_id(), lt = lanemask_lt();
     uint32_t k = 0;  // steps published
     uint32_t cur = 0xffffffffu;
     unsigned long long n_win = 0, n_tok = 0;  // window entries and query tokens of join cur
     auto flush_counts = [&] {
-        if (lane == 0 && n_win) {
+        if (lane == 0 && n_win && MODE != MODE_FILL) {
             atomicAdd(&joins[cur].stats[SS_WINDOW], n_win);
-            atomicAdd(&joins[cur].stats[SS_QTOK], n_tok);
+            if (MODE == MODE_FUSED) atomicAdd(&joins[cur].stats[SS_QTOK], n_tok);
         }
         n_win = n_tok = 0;
     };
@@ -109,8 +135,8 @@ __device__ void claim_producer(const JoinArgs* __restrict__ joins, const FusedAr
     uint32_t it = 0;
     if (lane == 0) it = atomicAdd(counter, 1u);
     it = __shfl_sync(kFull, it, 0);
-    while (it < n_items) {
-        const uint4 w = items[it];
+    while (it < items.n) {
+        const uint4 w = claim_item(items, it);
         uint32_t ahead = 0;
         if (lane == 0) ahead = atomicAdd(counter, 1u);
         const JoinArgs& a = joins[w.x];
@@ -284,7 +310,7 @@ __device__ __noinline__ void merge_now(const JoinArgs& a, const FusedArgs& fa, c
 //       the query's end or when it is half full.
 // No slot is compared-and-swapped, probed, listed or cleared: one that is read
 // was written in the same step.
-template <typename S, bool SIDED>
+template <typename S, int MODE, bool SIDED>
 __device__ void claim_consumer(const JoinArgs* __restrict__ joins, const FusedArgs* __restrict__ fargs,
                                unsigned char* smem, const ClaimStep* steps, ClaimQuery* s_query, uint32_t* s_nm,
                                unsigned long long* s_cnt) {
@@ -314,8 +340,8 @@ __device__ void claim_consumer(const JoinArgs* __restrict__ joins, const FusedAr
     auto flush_counts = [&](uint32_t join) {  // warp-collective
         const unsigned long long c = warp_sum((unsigned long long)n_cand), v = warp_sum((unsigned long long)n_ver);
         if (lane == 0) {
-            if (c) atomicAdd(&joins[join].stats[SS_CANDIDATES], c);
-            if (v) atomicAdd(&joins[join].stats[SS_VERIFIED], v);
+            if (c && MODE != MODE_FILL) atomicAdd(&joins[join].stats[SS_CANDIDATES], c);
+            if (v && MODE == MODE_FUSED) atomicAdd(&joins[join].stats[SS_VERIFIED], v);
         }
         n_cand = n_ver = 0;
     };
@@ -391,7 +417,7 @@ __device__ void claim_consumer(const JoinArgs* __restrict__ joins, const FusedAr
             const uint32_t lq = st.lq, pos = st.pos;
             const uint32_t qmode = a.n_terms <= S::BW * 32 ? QM_EXACT : (lq <= kQHashMax ? QM_HASH : QM_BLOOM);
             ClaimQuery& cq = s_query[par];
-            if (tid < 4) cq.bits[tid] = tid < fa.bmw ? __ldg(fa.bmap + (uint64_t)fa.bmw * st.q + tid) : make_uint4(0, 0, 0, 0);
+            if (MODE == MODE_FUSED && tid < 4) cq.bits[tid] = tid < fa.bmw ? __ldg(fa.bmap + (uint64_t)fa.bmw * st.q + tid) : make_uint4(0, 0, 0, 0);
             if (tid == 0) {
                 cq.join = st.join;
                 cq.q = st.q;
@@ -400,7 +426,7 @@ __device__ void claim_consumer(const JoinArgs* __restrict__ joins, const FusedAr
                 cq.qmode = qmode;
             }
             uint32_t* qtok = reinterpret_cast<uint32_t*>(smem + S::off_qtok) + par * S::QC;
-            if (lq <= S::QC)
+            if (MODE == MODE_FUSED && lq <= S::QC)
                 for (uint32_t j = tid; j < lq; j += S::NTC) qtok[j] = __ldg(a.tok + pos + j);
         }
         const uint32_t L = st.L, lq = st.lq, join = st.join;
@@ -451,7 +477,9 @@ __device__ void claim_consumer(const JoinArgs* __restrict__ joins, const FusedAr
         if (flags & CS_FIRST) {
             if (any_query && tid == 0 && s_query[par ^ 1].join != join) flush_merge_counts(s_query[par ^ 1].join);
             any_query = true;
-            for (uint32_t i = tid; i < S::BW / 4; i += S::NTC) reinterpret_cast<uint4*>(bm)[i] = make_uint4(0, 0, 0, 0);
+            if (MODE == MODE_FUSED)
+                for (uint32_t i = tid; i < S::BW / 4; i += S::NTC)
+                    reinterpret_cast<uint4*>(bm)[i] = make_uint4(0, 0, 0, 0);
         }
         uint32_t pend = mine;  // bit u: entry u has no leader yet
         uint32_t mul = 0;      // 0: the low bits of the source
@@ -492,7 +520,7 @@ __device__ void claim_consumer(const JoinArgs* __restrict__ joins, const FusedAr
             bar_named(2, S::NTC);
         }
         const FusedArgs& fa = fargs[join];
-        if (flags & CS_FIRST) {  // the query's membership structure, for the merges from the next step on
+        if (MODE == MODE_FUSED && (flags & CS_FIRST)) {  // the query's membership structure, for the merges from the next step on
             const uint32_t qmode = s_query[par].qmode;
             const uint32_t* qsrc = tokens_of(par);
 #pragma unroll 1
@@ -539,33 +567,36 @@ __device__ void claim_consumer(const JoinArgs* __restrict__ joins, const FusedAr
             const uint32_t f = vl[min(i0 + lane, nv - 1)];
             const uint32_t s = srcs[f];
             const uint2 g = agg[f];  // (y, matches | query position << 16)
-            const bool check = i0 + lane < nv &&
-                bitmap_keeps(s_query[par].bits, fa.bmap + (uint64_t)fa.bmw * s, fa.bmw, lq + (g.x >> 16),
-                             __ldg(&smin[g.x >> 16].y));
-            const uint32_t m = __ballot_sync(kFull, check);
-            if (m == 0) continue;
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(s_nm, (uint32_t)__popc(m));
-            const uint32_t mi = __shfl_sync(kFull, base, 0) + __popc(m & (le >> 1));
-            if (check && mi < S::MC) {
-                ml_s[mi] = s;
-                ml_y[mi] = g.x;
-                ml_c[mi] = g.y;
-            }
+            if constexpr (MODE != MODE_FUSED) {
+                plain_take<MODE>(joins[join], st.q, i0 + lane < nv, s, g.y);
+            } else {
+                const bool check = i0 + lane < nv &&
+                    bitmap_keeps(s_query[par].bits, fa.bmap + (uint64_t)fa.bmw * s, fa.bmw, lq + (g.x >> 16),
+                                 __ldg(&smin[g.x >> 16].y));
+                const uint32_t m = __ballot_sync(kFull, check);
+                if (m == 0) continue;
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(s_nm, (uint32_t)__popc(m));
+                const uint32_t mi = __shfl_sync(kFull, base, 0) + __popc(m & (le >> 1));
+                if (check && mi < S::MC) {
+                    ml_s[mi] = s;
+                    ml_y[mi] = g.x;
+                    ml_c[mi] = g.y;
+                }
 #pragma unroll 1
-            for (uint32_t over = __ballot_sync(kFull, check && mi >= S::MC); over; over &= over - 1) {
-                const uint32_t l = __ffs(over) - 1;
-                merge_now(joins[join], fa, s_query[par], __shfl_sync(kFull, s, l), __shfl_sync(kFull, g.x, l),
-                          __shfl_sync(kFull, g.y, l), tokens_of(par), s_cnt);
+                for (uint32_t over = __ballot_sync(kFull, check && mi >= S::MC); over; over &= over - 1) {
+                    const uint32_t l = __ffs(over) - 1;
+                    merge_now(joins[join], fa, s_query[par], __shfl_sync(kFull, s, l), __shfl_sync(kFull, g.x, l),
+                              __shfl_sync(kFull, g.y, l), tokens_of(par), s_cnt);
+                }
             }
         }
     }
 }
 
-template <typename S, int CTAS, bool SIDED>
+template <typename S, int CTAS, int MODE, bool SIDED>
 __global__ void __launch_bounds__(S::NT, CTAS) k_claim(const JoinArgs* __restrict__ joins,
-                                                       const FusedArgs* __restrict__ fargs,
-                                                       const uint4* __restrict__ items, uint32_t n_items,
+                                                       const FusedArgs* __restrict__ fargs, ClaimItems items,
                                                        uint32_t* counter) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ClaimStep s_step[2];
@@ -577,9 +608,9 @@ __global__ void __launch_bounds__(S::NT, CTAS) k_claim(const JoinArgs* __restric
     if (threadIdx.x == 0) s_nm = 0;
     __syncthreads();
     if (threadIdx.x >= S::NTC)
-        claim_producer<S>(joins, fargs, items, n_items, counter, smem, s_step);
+        claim_producer<S, MODE>(joins, fargs, items, counter, smem, s_step);
     else
-        claim_consumer<S, SIDED>(joins, fargs, smem, s_step, s_query, &s_nm, s_cnt);
+        claim_consumer<S, MODE, SIDED>(joins, fargs, smem, s_step, s_query, &s_nm, s_cnt);
 }
 
 // -------------------------------------------------------------------- k_tiny
@@ -601,7 +632,7 @@ struct TinyShared {
     uint16_t vl[kTinyMax];    // entries whose source needs verification
 };
 
-template <bool SIDED>
+template <int MODE, bool SIDED>
 __global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __restrict__ joins,
                                                           const FusedArgs* __restrict__ fargs, TileMap m) {
     __shared__ TinyShared s_all[kTinyWarps];
@@ -612,10 +643,9 @@ __global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __rest
     static_assert((1 << HB) == 4 * kTinyMax, "slot hash bits");
     FusedCounters ctr = {0, 0, 0, 0, 0, 0, 0};
     uint32_t cur = 0xffffffffu;
-    const uint32_t per = m.tile / 32;
-    for (uint32_t b = blockIdx.x; b < m.ntiles * per; b += gridDim.x) {
-        const TileRange t = tile_range(m, b / per);
-        const uint32_t r0 = t.r0 + (b % per) * 32;
+    for (uint32_t b = blockIdx.x; b < m.ntiles; b += gridDim.x) {  // tiles of at most 32 records
+        const TileRange t = tile_range(m, b);
+        const uint32_t r0 = t.r0;
         if (r0 >= t.r1) continue;
         if (t.j != cur) {
             if (cur != 0xffffffffu) flush_fused_counters(joins[cur], ctr);
@@ -720,44 +750,52 @@ __global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __rest
             __syncwarp();
 #pragma unroll 1
             for (uint32_t i0 = 0; i0 < nv; i0 += 32) {
-                bool check = false;
-                uint32_t s0 = 0, y0 = 0, cj0 = 0, im0 = 0;
-                if (i0 + lane < nv) {
-                    const uint32_t f = sh.vl[i0 + lane];
-                    const uint2 g = sh.agg[f];
-                    s0 = sh.src[f];
-                    y0 = g.x;
-                    cj0 = g.y;
-                    im0 = __ldg(&smin[y0 >> 16].y);
-                    check = bitmap_keeps(fa.bmap + (uint64_t)fa.bmw * q, fa.bmap + (uint64_t)fa.bmw * s0, fa.bmw,
-                                         lq + (y0 >> 16), im0);
-                }
-#pragma unroll 1
-                for (uint32_t mm = __ballot_sync(kFull, check); mm; mm &= mm - 1) {
-                    // merge, 32 source tokens per step, with the early exit of checking.cu:150-157
-                    const uint32_t l = __ffs(mm) - 1;
-                    const uint32_t s = __shfl_sync(kFull, s0, l), y = __shfl_sync(kFull, y0, l);
-                    const uint32_t cj = __shfl_sync(kFull, cj0, l), im = __shfl_sync(kFull, im0, l);
-                    const uint32_t ls = y >> 16, c = cj & 0xffffu, j = cj >> 16, qrest = lq - j - 1, k0 = (y & 0xffffu) + 1;
-                    const uint32_t* st = a.tok + fa.meta[s].x;
-                    uint32_t k = k0, cnt = c;
-#pragma unroll 1
-                    while (k < ls && cnt + min(ls - k, qrest - (cnt - c)) >= im) {
-                        const uint32_t kk = k + lane;
-                        const bool hit = kk < ls && contains_gen(qt, j + 1, lq, __ldg(st + kk));
-                        cnt += __popc(__ballot_sync(kFull, hit));
-                        k = min(k + 32u, ls);
+                if constexpr (MODE != MODE_FUSED) {
+                    const uint32_t f = sh.vl[min(i0 + lane, nv - 1)];
+                    plain_take<MODE>(a, q, i0 + lane < nv, sh.src[f], sh.agg[f].y);
+                } else {
+                    bool check = false;
+                    uint32_t s0 = 0, y0 = 0, cj0 = 0, im0 = 0;
+                    if (i0 + lane < nv) {
+                        const uint32_t f = sh.vl[i0 + lane];
+                        const uint2 g = sh.agg[f];
+                        s0 = sh.src[f];
+                        y0 = g.x;
+                        cj0 = g.y;
+                        im0 = __ldg(&smin[y0 >> 16].y);
+                        check = bitmap_keeps(fa.bmap + (uint64_t)fa.bmw * q, fa.bmap + (uint64_t)fa.bmw * s0, fa.bmw,
+                                             lq + (y0 >> 16), im0);
                     }
-                    if (lane == 0) {
-                        ctr.merged += k - k0;
-                        tally_overlap(a, ctr, q, s, cnt, im, __ldg(&smin[ls].z));
+#pragma unroll 1
+                    for (uint32_t mm = __ballot_sync(kFull, check); mm; mm &= mm - 1) {
+                        // merge, 32 source tokens per step, with the early exit of checking.cu:150-157
+                        const uint32_t l = __ffs(mm) - 1;
+                        const uint32_t s = __shfl_sync(kFull, s0, l), y = __shfl_sync(kFull, y0, l);
+                        const uint32_t cj = __shfl_sync(kFull, cj0, l), im = __shfl_sync(kFull, im0, l);
+                        const uint32_t ls = y >> 16, c = cj & 0xffffu, j = cj >> 16, qrest = lq - j - 1, k0 = (y & 0xffffu) + 1;
+                        const uint32_t* st = a.tok + fa.meta[s].x;
+                        uint32_t k = k0, cnt = c;
+#pragma unroll 1
+                        while (k < ls && cnt + min(ls - k, qrest - (cnt - c)) >= im) {
+                            const uint32_t kk = k + lane;
+                            const bool hit = kk < ls && contains_gen(qt, j + 1, lq, __ldg(st + kk));
+                            cnt += __popc(__ballot_sync(kFull, hit));
+                            k = min(k + 32u, ls);
+                        }
+                        if (lane == 0) {
+                            ctr.merged += k - k0;
+                            tally_overlap(a, ctr, q, s, cnt, im, __ldg(&smin[ls].z));
+                        }
                     }
                 }
             }
-            if (lane == 0) {
-                ctr.verified += nv;
+            if (MODE == MODE_FILL) ctr.cand = 0;
+            if (lane == 0 && MODE != MODE_FILL) {
                 ctr.window += W;
-                ctr.qtok += lq;
+                if (MODE == MODE_FUSED) {
+                    ctr.verified += nv;
+                    ctr.qtok += lq;
+                }
             }
             __syncwarp();
         }

@@ -44,6 +44,7 @@ struct Ctx {
     std::map<std::string, DevBuf> bufs;
     std::map<std::string, DevBuf> host_bufs;  // pinned
     std::map<std::string, TuneEntry> tune;
+    std::map<std::string, std::vector<uint16_t>> probe_max;  // per bound table: largest probe prefix up to a size
     const TuneEntry* tune_force = nullptr;  // set by the autotuner while it times a shape
     // Buffer-name namespace of the batch-level buffers: "" normally, a graph's
     // own "g<id>." while a graph-eligible batch is recorded or captured, so no

@@ -21,6 +21,7 @@ struct DevBounds {
     uint32_t* inter_min;
     uint32_t* need;
     uint4* smin;  // per length sum: (cand_min, inter_min, need, 0)
+    const uint16_t* probe_max = nullptr;  // host: the largest probe prefix of any size up to n
 };
 DevBounds device_bounds(Ctx& c, float t, int mode);
 
@@ -39,14 +40,12 @@ struct JoinState {
     int filter = 0;            // FGSS_FILTER_* (batched method)
     DevBounds lut{};
     JoinArgs args{};
-    JoinArgs* d_args = nullptr;
     uint32_t* status = nullptr;
     unsigned long long* stats = nullptr;
     uint64_t* d_e = nullptr;   // index entries (u64 copy of the scan total)
     uint32_t* icnt = nullptr;
     uint32_t* pcnt = nullptr;
     uint32_t* maxlen = nullptr;
-    int term_bits = 1;
     // outputs (device)
     uint64_t* d_nres = nullptr;
     uint32_t *oq = nullptr, *os = nullptr, *oidq = nullptr, *oids = nullptr, *oo = nullptr;
@@ -61,7 +60,6 @@ struct JoinState {
     std::vector<uint32_t> cand_host;  // (q, s, partial) triples when requested
     uint64_t pred_results = 0;        // the learned model's estimates (batched method, 0 without it)
     uint64_t pred_candidates = 0;
-    uint64_t* d_cost = nullptr;       // batched pre-pass: per-query work estimates
     const uint8_t* side = nullptr;    // R-S join: side byte of every record (JoinArgs.side)
     std::string ns;                   // buffer-name namespace ("" or a captured graph's own "g<id>.")
     std::string pfx(const char* name) const { return ns + "j" + std::to_string(slot) + "." + name; }
@@ -82,23 +80,13 @@ RsInput rs_union(Ctx& c, const fgss_sets_view& r, const fgss_sets_view& s);
 // After join_output: pairs as (index in R, index in S), sorted by that.
 void rs_output(Ctx& c, JoinState& J, const RsInput& u);
 
-// Queues the input validation and the per-record counts of one join.  With
-// check=false the caller synchronizes the stream once for a whole batch and
-// then calls join_check_input for every join before any kernel reads tokens.
-void join_setup(Ctx& c, JoinState& J, const fgss_sets_view& v, const fgss_join_opts& o, int slot, bool check = true);
-// The part of join_setup both methods share: options, the input's copy to the
-// device (host input), the bound tables and the JoinArgs fields that need no
-// per-join buffer.
+// Host side of a join's setup: options, the input's copy to the device (host
+// input), the bound tables and the JoinArgs fields that need no per-join buffer.
 void join_setup_host(Ctx& c, JoinState& J, const fgss_sets_view& v, const fgss_join_opts& o, int slot);
-void join_check_input(Ctx& c, JoinState& J);
 void check_input_status(uint32_t st);  // throws on the input-validation bits
 // Host copies of a join's status word and counters; throws on bad input or a
 // filter-table overflow.
 void apply_status(JoinState& J, uint32_t st, const unsigned long long* stats);
-void join_index(Ctx& c, JoinState& J);
-void join_plain_filter_verify(Ctx& c, JoinState& J, bool want_cand);
-void join_features(Ctx& c, JoinState& J, float* d_feat);
-void join_finish_status(Ctx& c, JoinState& J);  // D2H of status + stats, throws on bad input
 void join_output(Ctx& c, JoinState& J, uint64_t* keys, uint32_t* vals, const uint64_t* d_n, uint64_t n_cap);
 
 // Scratch of the global-memory accumulator kernel (k_probe_heavy) for `slots`
@@ -121,6 +109,8 @@ struct Batch {
     uint64_t R = 0;                    // records of the batch
     uint64_t E = 0, P = 0;             // index entries, probe windows (read back by batch_prep)
     uint32_t n_max = 0;                // records of the largest join
+    bool keyed_possible = false;       // a record's probe prefix may exceed kClaimPC (read back by batch_prep)
+    const uint32_t* status_host = nullptr;  // status words, once read back after the filter (batch_read_status)
     uint32_t terms_max = 0;
     TileMap rec{};                     // tiles of 256 records (device arrays)
     JoinArgs* d_args = nullptr;        // nj
@@ -144,6 +134,7 @@ struct BatchPlan {
     bool capture = false;             // issue device work only, with these decisions
     TuneEntry te;
     uint64_t E_cap = 0, P_cap = 0;    // index entries, probe windows the buffers hold
+    bool light = false;               // every query is the claim kernels', whose items are the records in order
     std::vector<uint32_t> K[2];       // work items per join (k_fused, k_claim)
     uint64_t nitems[2] = {0, 0};
     std::vector<uint64_t> res_cap;    // result slots per join
@@ -160,7 +151,14 @@ void batch_prep(Ctx& c, Batch& B, const std::vector<JoinState*>& js, const fgss_
 // term), one list pass.  E_cap: entries the buffers hold (>= B.E).
 void batch_index(Ctx& c, Batch& B, uint64_t E_cap);
 void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan = nullptr);
-// Status words and counters of every join to the host (one copy, one wait).
+// The plain method on a one-join batch (its index built): exact count pass ->
+// scan -> fill pass -> one verification launch -> result compaction, with a
+// wait between the stages.  The results are in the JoinState's own buffers.
+void plain_filter_verify(Ctx& c, Batch& B, bool want_cand);
+// Status words (8 per join), counters and entry counts of every join to the host
+// (one wait); batch_finish_status hands them to the JoinStates, reading them
+// first where that has not been done since the filter.
+const uint32_t* batch_read_status(Ctx& c, Batch& B);
 void batch_finish_status(Ctx& c, Batch& B);
 // Per-query work estimates of a one-join batch (its index built), copied to
 // host `out` (n values).

@@ -89,8 +89,10 @@ struct JoinArgs {
     const uint32_t* tab;
     uint32_t nb;
     // plain method
+    const uint4* meta;         // (pos, len, index prefix | class << 16, window entries) per record
     uint32_t* vcnt;            // count pass: per query, candidates that need a merge
-    uint32_t* ccnt;            // count pass: per query, candidates (reference definition)
+    uint32_t* ccnt;            // count pass: per query of k_probe, candidates (reference definition);
+                               // fill pass: records written so far (claim kernels)
     uint32_t* wcnt;            // count pass: per query, window entries read
     const uint32_t* voff;      // fill pass: exclusive scan of vcnt
     uint4* cand;               // fill pass: (q, s, matches, last_q << 16 | last_s)
@@ -246,16 +248,6 @@ __device__ __forceinline__ void prep_skip_test(const JoinArgs& a) {
     if (l0 <= 65535u && ln > a.maxsz[l0]) atomicOr(a.status, ST_SKIP_ALL);
 }
 
-static __global__ void k_prep(JoinArgs a, uint32_t* __restrict__ icnt, uint32_t* __restrict__ pcnt, uint32_t* maxlen,
-                              int check_tokens) {
-    uint32_t local_max = 0, bad = 0;
-    unsigned long long probe = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x)
-        prep_record(a, i, icnt + i, pcnt + i, local_max, bad, probe, check_tokens);
-    prep_flush(a, maxlen, local_max, bad, probe);
-    if (blockIdx.x == 0 && threadIdx.x == 0) prep_skip_test(a);
-}
-
 // send[L] for every query length L: the number of records of size >= lmin[L]
 // (records have non-increasing sizes).
 __device__ __forceinline__ uint32_t send_of(const uint32_t* __restrict__ len, uint32_t n, uint32_t target) {
@@ -266,12 +258,6 @@ __device__ __forceinline__ uint32_t send_of(const uint32_t* __restrict__ len, ui
         else hi = mid;
     }
     return lo;
-}
-
-static __global__ void k_send(const uint32_t* __restrict__ len, uint32_t n, const uint32_t* __restrict__ lmin,
-                              uint32_t* __restrict__ send, uint32_t nl) {
-    for (uint32_t L = blockIdx.x * blockDim.x + threadIdx.x; L < nl; L += gridDim.x * blockDim.x)
-        send[L] = send_of(len, n, lmin[L]);
 }
 
 // -------------------------------------------------------------- index stage
@@ -291,36 +277,6 @@ __device__ __forceinline__ void index_entries_record(const JoinArgs& a, uint32_t
     }
 }
 
-static __global__ void k_index_entries(JoinArgs a, const uint32_t* __restrict__ ioff, uint32_t* __restrict__ key,
-                                       uint64_t* __restrict__ val) {
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.n; i += warps)
-        index_entries_record<uint32_t>(a, i, ioff[i], 0u, key, val);
-}
-
-// After the stable sort by term: list offsets (no atomics: the thread at each
-// term boundary fills the offsets of the terms it spans) and the 8-byte entries.
-static __global__ void k_index_lists(const uint32_t* __restrict__ key, const uint64_t* __restrict__ val,
-                              const uint64_t* __restrict__ d_e, uint32_t n_terms, uint32_t* __restrict__ list_off,
-                              uint2* __restrict__ ent) {
-    const uint32_t E = (uint32_t)*d_e;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (E == 0) {
-        for (uint32_t w = tid; w <= n_terms; w += stride) list_off[w] = 0;
-        return;
-    }
-    for (uint32_t k = tid; k < E; k += stride) {
-        uint64_t v = val[k];
-        ent[k] = make_uint2((uint32_t)(v >> 32), (uint32_t)v);
-        uint32_t w = key[k];
-        if (k == 0)
-            for (uint32_t x = 0; x <= w; x++) list_off[x] = 0;
-        uint32_t nxt = (k + 1 < E) ? key[k + 1] : n_terms;
-        for (uint32_t x = w + 1; x <= nxt; x++) list_off[x] = k + 1;
-    }
-}
-
 }  // namespace fgss
 
 namespace fgss {
@@ -331,14 +287,13 @@ enum { MODE_COUNT = 0, MODE_FILL = 1, MODE_FUSED = 2 };
 
 constexpr uint32_t kPCap = 1024;     // probe tokens whose windows fit in shared memory
 constexpr uint32_t kQCap = 2048;     // query tokens staged in shared memory
-constexpr uint32_t kBmWords = 2048;  // query term bitmap: 65536 bits
 constexpr unsigned long long kEmptySlot = 0xffffffff00000000ull;
 
 // Shared-memory layout of the light-query kernel.
 //   slots u64[H]   (source << 32 | matches << 16 | last query position)
 //   wlo/whi u32[kPCap]   full id window of each probe token's list
 //   clo u32[kPCap], wpre u32[kPCap + 4]   the current chunk: first entry, exclusive scan of sizes
-//   qtok u32[kQCap]   query tokens;  bitmap u32[kBmWords] (fused only)
+//   qtok u32[kQCap]   query tokens
 template <int MODE, int HLOG>
 struct ProbeLayout {
     static constexpr uint32_t H = 1u << HLOG;
@@ -348,8 +303,7 @@ struct ProbeLayout {
     static constexpr size_t off_clo = off_whi + 4ull * kPCap;
     static constexpr size_t off_wpre = off_clo + 4ull * kPCap;
     static constexpr size_t off_qtok = off_wpre + 4ull * (kPCap + 4);
-    static constexpr size_t off_bm = off_qtok + 4ull * kQCap;
-    static constexpr size_t bytes = off_bm + (MODE == MODE_FUSED ? 4ull * kBmWords : 0);
+    static constexpr size_t bytes = off_qtok + 4ull * kQCap;
 };
 
 struct CtaCounters {
@@ -364,18 +318,6 @@ __device__ __forceinline__ void flush_counters(const JoinArgs& a, const CtaCount
     if (c.verified) atomicAdd(&a.stats[SS_VERIFIED], c.verified);
     if (c.heavy) atomicAdd(&a.stats[SS_HEAVY], c.heavy);
     if (c.merged) atomicAdd(&a.stats[SS_MERGED], c.merged);
-}
-
-// All lanes of a warp: sum the per-thread counters, one lane adds them.
-__device__ __forceinline__ void flush_counters_warp(const JoinArgs& a, CtaCounters c) {
-    c.cand = warp_sum(c.cand);
-    c.inter = warp_sum(c.inter);
-    c.res = warp_sum(c.res);
-    c.window = warp_sum(c.window);
-    c.verified = warp_sum(c.verified);
-    c.heavy = warp_sum(c.heavy);
-    c.merged = warp_sum(c.merged);
-    if (lane_id() == 0) flush_counters(a, c);
 }
 
 // Emits one verified pair (called by one lane).
@@ -460,53 +402,11 @@ __device__ __forceinline__ SlotVerdict slot_verdict(const JoinArgs& a, uint32_t 
     return v;
 }
 
-// Thread-serial merge of a source's tokens from position p0 against the
-// query's term bitmap, counting only tokens above xq (the query token of the
-// last prefix match: everything at or below it was counted by the filter).
-// Stops as soon as c + matches + what can still match < im.
-__device__ __forceinline__ uint32_t thread_merge(const uint32_t* __restrict__ st, uint32_t p0, uint32_t ls,
-                                                 uint32_t xq, uint32_t c, uint32_t qrest, uint32_t im,
-                                                 const uint32_t* bm, bool exact, const uint32_t* qtok, uint32_t qa,
-                                                 uint32_t lq, uint32_t* nread) {
-    uint32_t cnt = c;
-    uint32_t k = p0;
-    auto visit = [&](uint32_t x) {
-        if (x <= xq) return;
-        const uint32_t b = exact ? x : ((x * 0x9E3779B1u) >> 16);
-        bool hit = (bm[b >> 5] >> (b & 31)) & 1u;
-        if (hit && !exact) hit = contains_gen(qtok, qa, lq, x);
-        cnt += hit;
-    };
-    auto alive = [&](uint32_t kk) { return cnt + min(ls - kk, qrest - (cnt - c)) >= im; };
-    bool go = true;
-    while (k < ls && (reinterpret_cast<uintptr_t>(st + k) & 15u)) {
-        if (!alive(k)) { go = false; break; }
-        visit(__ldg(st + k));
-        k++;
-    }
-    while (go && k + 4 <= ls) {
-        if (!alive(k)) { go = false; break; }
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(st + k));
-        visit(v.x);
-        visit(v.y);
-        visit(v.z);
-        visit(v.w);
-        k += 4;
-    }
-    while (go && k < ls) {
-        if (!alive(k)) break;
-        visit(__ldg(st + k));
-        k++;
-    }
-    *nread = k - p0;
-    return cnt;
-}
-
 // Light query on one CTA: shared-memory slot table; the id window is split
 // into chunks of at most `cap` entries (depth-first bisection).  Queries
 // beyond the shared-memory caps go to the heavy queue.
 template <int MODE, int NT, int HLOG>
-__device__ void probe_query_smem(const JoinArgs& a, uint32_t q, unsigned char* smem, CtaCounters& ctr) {
+__device__ void probe_query_smem(const JoinArgs& a, uint32_t q, unsigned char* smem) {
     using Lay = ProbeLayout<MODE, HLOG>;
     unsigned long long* slots = reinterpret_cast<unsigned long long*>(smem);
     uint32_t* wlo = reinterpret_cast<uint32_t*>(smem + Lay::off_wlo);
@@ -514,7 +414,6 @@ __device__ void probe_query_smem(const JoinArgs& a, uint32_t q, unsigned char* s
     uint32_t* clo = reinterpret_cast<uint32_t*>(smem + Lay::off_clo);
     uint32_t* wpre = reinterpret_cast<uint32_t*>(smem + Lay::off_wpre);
     uint32_t* qtok = reinterpret_cast<uint32_t*>(smem + Lay::off_qtok);
-    uint32_t* bm = reinterpret_cast<uint32_t*>(smem + Lay::off_bm);
     __shared__ uint32_t s_L, s_vc, s_cand, s_sp, s_win;
     __shared__ uint32_t s_sa[48], s_sb[48];
     __shared__ uint32_t wsum[33];
@@ -532,18 +431,12 @@ __device__ void probe_query_smem(const JoinArgs& a, uint32_t q, unsigned char* s
         return;
     }
     const bool unsorted = (st_bits & ST_UNSORTED) != 0;
-    const bool exact_bm = a.n_terms <= kBmWords * 32;
     const uint32_t* qt = a.tok + a.pos[q];
     const uint32_t send = unsorted ? a.n : a.send[lq];
     if (send <= q + 1) return;
     // 1. stage the query (and its term bitmap); full windows [q+1, send)
     for (uint32_t j = tid; j < lq; j += NT) {
-        uint32_t x = __ldg(qt + j);
-        qtok[j] = x;
-        if (MODE == MODE_FUSED) {
-            uint32_t b = exact_bm ? x : ((x * 0x9E3779B1u) >> 16);
-            atomicOr(&bm[b >> 5], 1u << (b & 31));
-        }
+        qtok[j] = __ldg(qt + j);
     }
     __syncthreads();
     for (uint32_t j = tid; j < qp; j += NT) {
@@ -646,22 +539,6 @@ __device__ void probe_query_smem(const JoinArgs& a, uint32_t q, unsigned char* s
                     uint32_t i = atomicAdd(&s_vc, 1u);
                     if (i < a.vcnt[q]) a.cand[a.voff[q] + i] = make_uint4(q, s, c, jm);
                     else atomicOr(a.status, ST_HASH_FULL);
-                } else if (MODE == MODE_FUSED) {
-                    // 5. merge right here, one thread per candidate, against the query bitmap
-                    const uint32_t ls = a.len[s], S = lq + ls;
-                    const uint32_t im = a.inter_min[S];
-                    uint32_t nread = 0;
-                    const uint32_t o = thread_merge(a.tok + a.pos[s], c, ls, qtok[jm], c, lq - jm - 1, im, bm,
-                                                    exact_bm, qtok, jm + 1, lq, &nread);
-                    ctr.verified++;
-                    ctr.merged += nread;
-                    if (o >= im && o > 0) {
-                        ctr.inter++;
-                        if (o >= a.need[S]) {
-                            ctr.res++;
-                            emit_result(a, q, s, o);
-                        }
-                    }
                 }
             }
         }
@@ -681,61 +558,21 @@ __device__ void probe_query_smem(const JoinArgs& a, uint32_t q, unsigned char* s
             a.vcnt[q] = s_vc;
             a.ccnt[q] = s_cand;
             a.wcnt[q] = s_win;
-        } else if (MODE == MODE_FUSED) {
-            ctr.cand += s_cand;
-            ctr.window += s_win;
         }
     }
-    if (MODE == MODE_FUSED) {
-        for (uint32_t j = tid; j < lq; j += NT) {
-            uint32_t x = qtok[j];
-            uint32_t b = exact_bm ? x : ((x * 0x9E3779B1u) >> 16);
-            bm[b >> 5] = 0u;
-        }
-    }
-    __syncthreads();
 }
 
-// Light-query kernel.  items == nullptr: one CTA per query of joins[0]
-// (plain method).  Otherwise persistent: CTAs pull (join, q_begin, q_end)
-// items from a queue.
+// The plain method's keyed kernel (queries of QC_KEYED): one CTA per query of joins[0].
 template <int MODE, int NT, int HLOG>
-__global__ void __launch_bounds__(NT) k_probe(const JoinArgs* __restrict__ joins, const uint4* __restrict__ items,
-                                              uint32_t n_items, uint32_t* item_counter) {
+__global__ void __launch_bounds__(NT) k_probe(const JoinArgs* __restrict__ joins) {
     extern __shared__ __align__(16) unsigned char smem[];
     using Lay = ProbeLayout<MODE, HLOG>;
+    const JoinArgs& a = joins[0];
+    if (a.meta[blockIdx.x].z >> 16) return;  // a query of the claim kernels
     unsigned long long* slots = reinterpret_cast<unsigned long long*>(smem);
     for (uint32_t h = threadIdx.x; h < Lay::H; h += NT) slots[h] = kEmptySlot;
-    if (MODE == MODE_FUSED) {
-        uint32_t* bm = reinterpret_cast<uint32_t*>(smem + Lay::off_bm);
-        for (uint32_t i = threadIdx.x; i < kBmWords; i += NT) bm[i] = 0u;
-    }
     __syncthreads();
-    CtaCounters ctr = {0, 0, 0, 0, 0, 0, 0};
-    if (items == nullptr) {
-        const JoinArgs& a = joins[0];
-        probe_query_smem<MODE, NT, HLOG>(a, blockIdx.x, smem, ctr);
-        if (MODE == MODE_FUSED) flush_counters_warp(a, ctr);
-        return;
-    }
-    __shared__ uint32_t s_item;
-    uint32_t cur_join = 0xffffffffu;
-    for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(item_counter, 1u);
-        __syncthreads();
-        const uint32_t it = s_item;
-        __syncthreads();
-        if (it >= n_items) break;
-        const uint4 w = items[it];
-        if (w.x != cur_join) {
-            if (cur_join != 0xffffffffu) flush_counters_warp(joins[cur_join], ctr);
-            ctr = {0, 0, 0, 0, 0, 0, 0};
-            cur_join = w.x;
-        }
-        const JoinArgs& a = joins[w.x];
-        for (uint32_t q = w.y; q < w.z; q++) probe_query_smem<MODE, NT, HLOG>(a, q, smem, ctr);
-    }
-    if (cur_join != 0xffffffffu) flush_counters_warp(joins[cur_join], ctr);
+    probe_query_smem<MODE, NT, HLOG>(a, blockIdx.x, smem);
 }
 
 // ------------------------------------------------------------ heavy queries
@@ -934,13 +771,6 @@ __device__ __forceinline__ void bitmap_record(const JoinArgs& a, uint32_t r, uin
     __syncwarp();
 }
 
-static __global__ void k_bitmaps(JoinArgs a, uint4* __restrict__ bmap, uint32_t bmw) {
-    __shared__ uint32_t sw[8][16];  // launched with 256 threads: a bitmap per warp
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < a.n; r += warps)
-        bitmap_record(a, r, bmap, bmw, sw[threadIdx.x >> 5]);
-}
-
 // Bitmap width of a join in uint4 words: 4 (512 bits) when its records average
 // more than 96 tokens (a 256-bit bitmap of a long record is too full to bound
 // much), else 2 (256 bits).
@@ -952,45 +782,68 @@ __device__ __forceinline__ uint32_t popc_xor(uint4 a, uint4 b) {
     return __popc(a.x ^ b.x) + __popc(a.y ^ b.y) + __popc(a.z ^ b.z) + __popc(a.w ^ b.w);
 }
 
+// The bitmap bound of one source that passed the position test: does it still
+// need a merge?  q4: the query's bitmap (shared or global memory).
+__device__ __forceinline__ bool bitmap_keeps(const uint4* q4, const uint4* __restrict__ b4, uint32_t bmw, uint32_t S,
+                                             uint32_t im) {
+    uint32_t pc = popc_xor(q4[0], __ldg(b4)) + popc_xor(q4[1], __ldg(b4 + 1));
+    if (bmw == 4) pc += popc_xor(q4[2], __ldg(b4 + 2)) + popc_xor(q4[3], __ldg(b4 + 3));
+    return S >= 2 * im + pc;
+}
+
 // ------------------------------------------------- plain verification stage
 
-// Warp per candidate record (q, s, matches, last query position); the source
-// position is found by a search, q tokens are searched in global memory.
-// Writes the overlap (0 when it cannot reach floor(min overlap)).
-// A candidate whose bitmap bound (k_bitmaps) is below floor(min overlap) can
-// be no intersection and skips its merge, as in the batched method's kernel.
+// Candidate records (q, s, matches, last query position): a lane per record
+// checks the bitmap bound (k_bitmaps_mj; below floor(min overlap) it can be no
+// intersection), then the warp merges the records left one after another; the
+// source position is found by a search, query tokens are searched in global
+// memory.  Writes the overlap (0 when it cannot reach floor(min overlap)).  Nearly
+// every record fails the bound, so a warp per record spends its time on 31 idle
+// lanes: 17.8 M records of 100,000 titles at t = 0.7 took 2.1 ms, a lane each 0.22 ms.
+// A warp takes `per` <= 32 records, fewer where there are too few to give every
+// warp 32 (the merges of one warp's records are a serial chain: 500 titles at
+// t = 0.9 took 99 us at 32 a warp, 7 us at 1).
 static __global__ void k_verify(JoinArgs a, const uint4* __restrict__ cand, const uint64_t* __restrict__ d_nc,
-                                uint32_t* __restrict__ ov, const uint4* __restrict__ bmap, uint32_t bmw) {
+                                uint32_t per, uint32_t* __restrict__ ov, const uint4* __restrict__ bmap,
+                                uint32_t bmw) {
     const uint32_t nc = (uint32_t)*d_nc;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t lane = lane_id();
-    unsigned long long inter = 0, ver = 0;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc; i += warps) {
-        const uint4 r = cand[i];
-        const uint32_t q = r.x, s = r.y, c = r.z, jm = r.w;
-        const uint32_t lq = a.len[q], ls = a.len[s], S = lq + ls;
-        const uint32_t imin = a.inter_min[S];
-        // lanes 0..bmw-1 each xor one 128-bit word of the two bitmaps
-        uint32_t pc = lane < bmw ? popc_xor(__ldg(bmap + bmw * q + lane), __ldg(bmap + bmw * s + lane)) : 0u;
-        pc = warp_sum(pc);
-        uint32_t o = 0;
-        if (S >= 2 * imin + pc) {
-            const uint32_t* qt = a.tok + a.pos[q];
-            const uint32_t* st = a.tok + a.pos[s];
-            const uint32_t smx = warp_find(st, a.index[ls], __ldg(qt + jm));
-            o = warp_merge_count(qt, jm + 1, lq, st, smx + 1, ls, c, imin);
+    const uint64_t w0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x >> 5) * per;
+    unsigned long long inter = 0;
+    for (uint64_t i0 = w0 * per; i0 < nc; i0 += stride) {
+        const uint64_t i = i0 + lane;
+        const bool in = lane < per && i < nc;
+        const uint4 r = in ? cand[i] : make_uint4(0, 0, 0, 0);
+        uint32_t lq = 0, ls = 0, imin = 0;
+        bool left = false;
+        if (in) {
+            lq = a.len[r.x];
+            ls = a.len[r.y];
+            imin = a.inter_min[lq + ls];
+            left = bitmap_keeps(bmap + (uint64_t)bmw * r.x, bmap + (uint64_t)bmw * r.y, bmw, lq + ls, imin);
         }
-        const bool ok = o >= imin && o > 0;
-        if (lane == 0) {
+        uint32_t o = 0;
+        for (uint32_t m = __ballot_sync(kFull, left); m; m &= m - 1) {
+            const uint32_t l = __ffs(m) - 1;
+            const uint32_t s = __shfl_sync(kFull, r.y, l), c = __shfl_sync(kFull, r.z, l), jm = __shfl_sync(kFull, r.w, l);
+            const uint32_t n = __shfl_sync(kFull, ls, l);
+            const uint32_t* qt = a.tok + a.pos[__shfl_sync(kFull, r.x, l)];
+            const uint32_t* st = a.tok + a.pos[s];
+            const uint32_t smx = warp_find(st, a.index[n], __ldg(qt + jm));
+            const uint32_t x = warp_merge_count(qt, jm + 1, __shfl_sync(kFull, lq, l), st, smx + 1, n, c,
+                                                __shfl_sync(kFull, imin, l));
+            if (lane == l) o = x;
+        }
+        if (in) {
+            const bool ok = o >= imin && o > 0;
             ov[i] = ok ? o : 0;
-            ver++;
             inter += ok;
         }
     }
-    if (lane == 0) {
-        if (inter) atomicAdd(&a.stats[SS_INTERSECTIONS], inter);
-        if (ver) atomicAdd(&a.stats[SS_VERIFIED], ver);
-    }
+    inter = warp_sum(inter);
+    if (lane == 0 && inter) atomicAdd(&a.stats[SS_INTERSECTIONS], inter);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats[SS_VERIFIED], (unsigned long long)nc);
 }
 
 // Result flags for the compaction (block.cu:190-192 as an integer test).
@@ -1007,41 +860,29 @@ static __global__ void k_result_flags(JoinArgs a, const uint4* __restrict__ cand
 
 static __global__ void k_result_fill(const uint4* __restrict__ cand, const uint32_t* __restrict__ ov,
                               const uint32_t* __restrict__ flag, const uint32_t* __restrict__ off,
-                              const uint64_t* __restrict__ d_nc, uint64_t* __restrict__ key,
+                              const uint64_t* __restrict__ d_nc, uint32_t qb, uint64_t* __restrict__ key,
                               uint32_t* __restrict__ val) {
     const uint32_t nc = (uint32_t)*d_nc;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
         if (flag[i]) {
             uint4 r = cand[i];
             uint32_t d = off[i];
-            key[d] = ((uint64_t)r.x << 32) | r.y;
+            key[d] = ((uint64_t)r.x << qb) | r.y;
             val[d] = ov[i];
         }
     }
 }
 
-// Fused method: results (q, s, o) -> sort keys.
-static __global__ void k_result_keys(const uint32_t* __restrict__ rq, const uint32_t* __restrict__ rs,
-                              const uint32_t* __restrict__ ro, const uint32_t* __restrict__ d_cnt, uint32_t cap,
-                              uint64_t* __restrict__ key, uint32_t* __restrict__ val, uint64_t* __restrict__ d_n) {
-    const uint32_t n = min(*d_cnt, cap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *d_n = n;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        key[i] = ((uint64_t)rq[i] << 32) | rs[i];
-        val[i] = ro[i];
-    }
-}
-
 // Sorted keys -> output columns: q, s, id_q, id_s, overlap, sim.
 static __global__ void k_result_out(const uint64_t* __restrict__ key, const uint32_t* __restrict__ val,
-                             const uint64_t* __restrict__ d_n, const uint32_t* __restrict__ id,
+                             const uint64_t* __restrict__ d_n, uint32_t qb, const uint32_t* __restrict__ id,
                              const uint32_t* __restrict__ len, uint32_t* __restrict__ oq, uint32_t* __restrict__ os,
                              uint32_t* __restrict__ oidq, uint32_t* __restrict__ oids, uint32_t* __restrict__ oo,
                              float* __restrict__ osim) {
     const uint64_t n = *d_n;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t k = key[i];
-        uint32_t q = (uint32_t)(k >> 32), s = (uint32_t)k, o = val[i];
+        uint32_t q = (uint32_t)(k >> qb), s = (uint32_t)(k & ((1ull << qb) - 1)), o = val[i];
         oq[i] = q;
         os[i] = s;
         oidq[i] = id ? id[q] : q;

@@ -56,10 +56,14 @@ fgss_status fgss_model_train(fgss_ctx* ctx, const fgss_sets_view* sets, const fl
             fgss_join_opts o;
             fgss_join_opts_default(&o);
             o.threshold = thresholds[i];
-            join_setup(c, J, sets[i], o, 100);
-            join_index(c, J);
-            join_plain_filter_verify(c, J, false);
-            join_finish_status(c, J);
+            J.slot = 100;
+            Batch B;
+            batch_prep(c, B, {&J}, &sets[i], &o);
+            batch_index(c, B, B.E);
+            plain_filter_verify(c, B, false);
+            const uint64_t n_res = J.n_res;
+            batch_finish_status(c, B);
+            J.n_res = n_res;
             const uint64_t m = J.in.n_sets;
             if (!m) continue;
             uint32_t* rcnt = c.devT<uint32_t>("mt.rcnt", m + 1);

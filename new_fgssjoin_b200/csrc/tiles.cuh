@@ -14,7 +14,17 @@ struct TileMap {
     uint32_t nj;
     uint32_t tile;             // records per tile
     uint32_t ntiles;
+    uint32_t split;            // tiles per entry of tile_off's unit (finer_tiles)
 };
+
+// The same map in tiles of `tile` records, a divisor of m's.  (The parts of a
+// join's last tile beyond its records are empty: r1 <= r0.)
+inline TileMap finer_tiles(TileMap m, uint32_t tile) {
+    m.split *= m.tile / tile;
+    m.ntiles *= m.tile / tile;
+    m.tile = tile;
+    return m;
+}
 
 // The join of tile b: the last j with tile_off[j] <= b.
 __device__ __forceinline__ uint32_t tile_join(const TileMap& m, uint32_t b) {
@@ -33,8 +43,8 @@ struct TileRange {
 };
 __device__ __forceinline__ TileRange tile_range(const TileMap& m, uint32_t b) {
     TileRange t;
-    t.j = tile_join(m, b);
-    t.r0 = (b - __ldg(m.tile_off + t.j)) * m.tile;
+    t.j = tile_join(m, b / m.split);
+    t.r0 = (b - __ldg(m.tile_off + t.j) * m.split) * m.tile;
     const uint64_t n = __ldg(m.roff + t.j + 1) - __ldg(m.roff + t.j);
     t.r1 = (uint32_t)min((uint64_t)t.r0 + m.tile, n);
     return t;
