@@ -15,7 +15,6 @@
 
 namespace fgss {
 
-__global__ void k_widen(const uint32_t* in, uint64_t* out);
 static_assert(kFeatures == kFeat, "model feature rows");
 
 // Warp per record: the learned model's features of one join (training rows,
@@ -163,10 +162,11 @@ TileMap tiles_for(const TileMap& m, uint64_t want, uint32_t low) {
     return finer_tiles(m, tile);
 }
 
-// Tiles of the warp-per-record stages: small enough to give every SM 8 CTAs of 8 warps
-// as long as a warp still has a record (500 titles: k_windows_mj 40 -> 4.1 us,
+// Tiles of the warp-per-record stages.  Records come in descending size, so a tile of
+// the longest ones is the stage's critical path: small enough to give every resident CTA
+// (8 of 8 warps on an SM) 4 tiles, as long as a warp still has a record (500 titles: k_windows_mj 40 -> 4.1 us,
 // k_bitmaps_mj 32 -> 3.3, k_index_entries_mj 21 -> 2.9 with tiles of 8 instead of 256).
-TileMap warp_tiles(Ctx& c, const TileMap& m) { return tiles_for(m, (uint64_t)8 * c.num_sms, 8); }
+TileMap warp_tiles(Ctx& c, const TileMap& m) { return tiles_for(m, (uint64_t)32 * c.num_sms, 8); }
 
 // Items of the records in order: about 128 per CTA.
 ClaimItems items_in_order(Ctx& c, const TileMap& m) {
@@ -360,13 +360,13 @@ FusedArgs* batch_filters(Ctx& c, Batch& B, const Prepass& pp, uint32_t cap_entri
     FusedArgs* d_fargs = c.devT<FusedArgs>(p + "b.fargs", nj);
     FGSS_CK(cudaMemcpyAsync(d_fargs, hf, nj * sizeof(FusedArgs), cudaMemcpyHostToDevice, c.stream));
     unsigned long long* cused = c.devT<unsigned long long>(p + "b.cused", 1);
-    FGSS_CK(cudaMemsetAsync(cused, 0, 8, c.stream));
     if (R == 0) return d_fargs;
     const TileMap wt = warp_tiles(c, B.rec);
     const unsigned g = tile_grid(c, wt);
     k_bitmaps_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, wt);
     FGSS_LAUNCH_CK();
     if (!chunks) return d_fargs;  // no query for k_fused
+    FGSS_CK(cudaMemsetAsync(cused, 0, 8, c.stream));
     k_chunks_mj<<<g, 256, 0, c.stream>>>(B.d_args, d_fargs, wt, pp.wtot, cap_entries, cbuf, cbuf_cap, cused);
     FGSS_LAUNCH_CK();
     return d_fargs;
@@ -420,9 +420,13 @@ void batch_prep(Ctx& c, Batch& B, const std::vector<JoinState*>& js, const fgss_
     B.R = B.roff[nj];
     // per-record offsets are 32-bit: the caller splits larger batches
     if (T >= 0xffffffffull || B.R >= 0xffffffffull) fail(FGSS_ERR_UNSUPPORTED, "a batch of 2^32 or more tokens");
-    B.status = c.devT<uint32_t>(p + "b.status", nj * 8);
-    B.stats = c.devT<unsigned long long>(p + "b.stats", nj * SS_N);
-    B.d_e = c.devT<uint64_t>(p + "b.E", nj * 2);
+    // one block, cleared and read back as one
+    B.words = (nj * (4 + SS_N + 2) + 2) * 8;
+    uint64_t* words = c.devT<uint64_t>(p + "b.words", B.words / 8);
+    B.status = reinterpret_cast<uint32_t*>(words);
+    B.stats = reinterpret_cast<unsigned long long*>(words + nj * 4);
+    B.d_e = words + nj * (4 + SS_N);
+    B.tot = B.d_e + nj * 2;
     B.icnt = c.devT<uint32_t>(p + "b.icnt", B.R + 1);
     B.pcnt = c.devT<uint32_t>(p + "b.pcnt", B.R + 1);
     B.ioff = c.devT<uint32_t>(p + "b.ioff", B.R + 1);
@@ -430,8 +434,7 @@ void batch_prep(Ctx& c, Batch& B, const std::vector<JoinState*>& js, const fgss_
     B.send = c.devT<uint32_t>(p + "b.send", nj * 65537);
     B.heavy_q = c.devT<uint32_t>(p + "b.heavy_q", B.R + 1);
     B.d_args = c.devT<JoinArgs>(p + "b.args", nj);
-    FGSS_CK(cudaMemsetAsync(B.status, 0, nj * 32, c.stream));
-    FGSS_CK(cudaMemsetAsync(B.stats, 0, nj * SS_N * 8, c.stream));
+    FGSS_CK(cudaMemsetAsync(words, 0, B.words, c.stream));
     for (size_t j = 0; j < nj; j++) {
         JoinState& J = *js[j];
         J.status = B.status + 8 * j;
@@ -451,32 +454,33 @@ void batch_prep(Ctx& c, Batch& B, const std::vector<JoinState*>& js, const fgss_
     B.rec = upload_tiles(c, p + "b.rec", B.roff, kRecTile);
     upload_args(c, B, p + "b.ha0");
     if (B.R) {
-        k_prep_mj<<<tile_grid(c, B.rec), 256, 0, c.stream>>>(B.d_args, B.rec, B.icnt, B.pcnt);
+        const TileMap t = tiles_for(B.rec, (uint64_t)32 * c.num_sms, 8);
+        k_prep_mj<<<tile_grid(c, t, 8), 256, 0, c.stream>>>(B.d_args, t, B.icnt, B.pcnt);
         FGSS_LAUNCH_CK();
         k_send_mj<<<grid_for((uint64_t)nj << 16, 256, c.num_sms * 32), 256, 0, c.stream>>>(B.d_args, (uint32_t)nj,
                                                                                           B.send);
         FGSS_LAUNCH_CK();
         exclusive_scan<uint32_t>(c, B.icnt, B.ioff, B.R, nullptr, B.ioff + B.R, (p + "b.scan.i").c_str());
         exclusive_scan<uint32_t>(c, B.pcnt, B.poff, B.R, nullptr, B.poff + B.R, (p + "b.scan.p").c_str());
+        k_join_totals<<<grid_for(nj, 128), 128, 0, c.stream>>>(B.d_args, B.rec.roff, (uint32_t)nj, B.ioff, B.poff, B.d_e,
+                                                               B.tot);
+        FGSS_LAUNCH_CK();
     } else {
         FGSS_CK(cudaMemsetAsync(B.ioff, 0, 4, c.stream));
         FGSS_CK(cudaMemsetAsync(B.poff, 0, 4, c.stream));
     }
     // one wait for the whole batch: no kernel reads tokens through caller
     // offsets before they are validated
-    uint32_t* h = c.pinnedT<uint32_t>(p + "b.hprep", nj * 8 + 2);
-    FGSS_CK(cudaMemcpyAsync(h, B.status, nj * 32, cudaMemcpyDeviceToHost, c.stream));
-    FGSS_CK(cudaMemcpyAsync(h + nj * 8, B.ioff + B.R, 4, cudaMemcpyDeviceToHost, c.stream));
-    FGSS_CK(cudaMemcpyAsync(h + nj * 8 + 1, B.poff + B.R, 4, cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
+    const uint32_t* h = batch_read_status(c, B);
+    const uint64_t* tot = reinterpret_cast<const uint64_t*>(h) + (B.tot - words);
+    B.E = tot[0];
+    B.P = tot[1];
     B.keyed_possible = false;
-    B.status_host = nullptr;
+    B.status_host = nullptr;  // of the filter, not yet read
     for (size_t j = 0; j < nj; j++) {
         if (js[j]->in.n_sets) check_input_status(h[8 * j]);
         B.keyed_possible |= js[j]->lut.probe_max[std::min<uint32_t>(h[8 * j + 1], kMaxLen)] > kClaimPC;
     }
-    B.E = h[nj * 8];
-    B.P = h[nj * 8 + 1];
 }
 
 void batch_index(Ctx& c, Batch& B, uint64_t E_cap) {
@@ -518,15 +522,9 @@ void batch_index(Ctx& c, Batch& B, uint64_t E_cap) {
     // a join without entries keeps these zero offsets (empty lists)
     FGSS_CK(cudaMemsetAsync(list, 0, L * 4, c.stream));
     if (TB) FGSS_CK(cudaMemsetAsync(tab, 0, TB * 4, c.stream));
-    FGSS_CK(cudaMemsetAsync(B.d_e, 0, nj * 16, c.stream));
     if (B.R) {
-        uint64_t* d_E = c.devT<uint64_t>(p + "b.dE", 2);
-        k_widen<<<1, 1, 0, c.stream>>>(B.ioff + B.R, d_E);
-        FGSS_LAUNCH_CK();
-        k_join_entries<<<grid_for(nj, 128), 128, 0, c.stream>>>(B.rec.roff, (uint32_t)nj, B.ioff, B.d_e);
-        FGSS_LAUNCH_CK();
-        if (tbits + jbits <= 32) index_sort<uint32_t>(c, B, E_cap, tbits, jbits, d_E, d_loff, list, d_toff, tab, ent);
-        else index_sort<uint64_t>(c, B, E_cap, tbits, jbits, d_E, d_loff, list, d_toff, tab, ent);
+        if (tbits + jbits <= 32) index_sort<uint32_t>(c, B, E_cap, tbits, jbits, B.tot, d_loff, list, d_toff, tab, ent);
+        else index_sort<uint64_t>(c, B, E_cap, tbits, jbits, B.tot, d_loff, list, d_toff, tab, ent);
     }
 }
 
@@ -924,13 +922,8 @@ void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
 }
 
 const uint32_t* batch_read_status(Ctx& c, Batch& B) {
-    const size_t nj = B.js.size();
-    uint32_t* h = c.pinnedT<uint32_t>(c.bpfx + "b.hfin", nj * 8);
-    unsigned long long* hs = c.pinnedT<unsigned long long>(c.bpfx + "b.hfin.stats", nj * SS_N);
-    uint64_t* he = c.pinnedT<uint64_t>(c.bpfx + "b.hfin.E", nj * 2);
-    FGSS_CK(cudaMemcpyAsync(h, B.status, nj * 32, cudaMemcpyDeviceToHost, c.stream));
-    FGSS_CK(cudaMemcpyAsync(hs, B.stats, nj * SS_N * 8, cudaMemcpyDeviceToHost, c.stream));
-    FGSS_CK(cudaMemcpyAsync(he, B.d_e, nj * 16, cudaMemcpyDeviceToHost, c.stream));
+    uint32_t* h = c.pinnedT<uint32_t>(c.bpfx + "b.hwords", B.words / 4);
+    FGSS_CK(cudaMemcpyAsync(h, B.status, B.words, cudaMemcpyDeviceToHost, c.stream));
     c.sync();
     B.status_host = h;
     return h;
@@ -939,8 +932,9 @@ const uint32_t* batch_read_status(Ctx& c, Batch& B) {
 void batch_finish_status(Ctx& c, Batch& B) {
     const size_t nj = B.js.size();
     const uint32_t* h = B.status_host ? B.status_host : batch_read_status(c, B);
-    const unsigned long long* hs = c.pinnedT<unsigned long long>(c.bpfx + "b.hfin.stats", nj * SS_N);
-    const uint64_t* he = c.pinnedT<uint64_t>(c.bpfx + "b.hfin.E", nj * 2);
+    const uint64_t* w = reinterpret_cast<const uint64_t*>(h);
+    const unsigned long long* hs = reinterpret_cast<const unsigned long long*>(w + nj * 4);
+    const uint64_t* he = w + (B.d_e - reinterpret_cast<const uint64_t*>(B.status));
     for (size_t j = 0; j < nj; j++) {
         B.js[j]->n_entries = he[2 * j];
         B.js[j]->n_res = h[8 * j + 3];

@@ -12,17 +12,28 @@ namespace fgss {
 // k_prep for every join: counts into the batch arrays icnt / pcnt (record g).
 static __global__ void k_prep_mj(const JoinArgs* __restrict__ joins, TileMap m, uint32_t* __restrict__ icnt,
                                  uint32_t* __restrict__ pcnt) {
+    // a warp takes an eighth of the tile, at most 32 records
+    const uint32_t wid = threadIdx.x >> 5, lane = lane_id(), per = m.tile / 8;
+    uint32_t local_max = 0, bad = 0, cur = 0xffffffffu;
     for (uint32_t b = blockIdx.x; b < m.ntiles; b += gridDim.x) {
         const TileRange t = tile_range(m, b);
         const JoinArgs& a = joins[t.j];
         const uint64_t g0 = __ldg(m.roff + t.j);
-        uint32_t local_max = 0, bad = 0;
-        unsigned long long probe = 0;
-        for (uint32_t i = t.r0 + threadIdx.x; i < t.r1; i += blockDim.x)
-            prep_record(a, i, icnt + g0 + i, pcnt + g0 + i, local_max, bad, probe, 1);
-        prep_flush(a, a.status + 1, local_max, bad, probe);
+        if (t.j != cur) {
+            if (cur != 0xffffffffu) prep_flush(joins[cur], local_max, bad);
+            local_max = bad = 0;
+            cur = t.j;
+        }
+        const uint32_t i = t.r0 + wid * per + lane;
+        uint32_t l = 0, p = 0;
+        if (lane < per && i < t.r1) {
+            l = prep_record(a, i, icnt + g0 + i, pcnt + g0 + i, local_max, bad);
+            p = a.pos[i];
+        }
+        prep_tokens(a.tok, a.n_terms, p, l, bad);
         if (t.r0 == 0 && threadIdx.x == 0) prep_skip_test(a);
     }
+    if (cur != 0xffffffffu) prep_flush(joins[cur], local_max, bad);
 }
 
 // send[L] of every join for the query lengths L <= its longest record (the
@@ -113,15 +124,28 @@ __global__ void k_index_lists_mj(const JoinArgs* __restrict__ joins, const K* __
     }
 }
 
-// Number of index entries of every join (from the batch's entry offsets).
-static __global__ void k_join_entries(const uint64_t* __restrict__ roff, uint32_t nj,
-                                      const uint32_t* __restrict__ ioff, uint64_t* __restrict__ d_e_all) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nj; j += gridDim.x * blockDim.x)
-        d_e_all[2 * j] = (uint64_t)(ioff[roff[j + 1]] - ioff[roff[j]]);
+// Numbers of index entries and probe tokens of every join (from the batch's
+// offsets) and of the batch (tot).
+static __global__ void k_join_totals(const JoinArgs* __restrict__ joins, const uint64_t* __restrict__ roff, uint32_t nj,
+                                     const uint32_t* __restrict__ ioff, const uint32_t* __restrict__ poff,
+                                     uint64_t* __restrict__ d_e_all, uint64_t* __restrict__ tot) {
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nj; j += gridDim.x * blockDim.x) {
+        const uint64_t b = roff[j], e = roff[j + 1];
+        d_e_all[2 * j] = (uint64_t)(ioff[e] - ioff[b]);
+        joins[j].stats[SS_PROBE] = (uint64_t)(poff[e] - poff[b]);
+        if (j == nj - 1) {
+            tot[0] = ioff[e];
+            tot[1] = poff[e];
+        }
+    }
 }
 
 // Warp per record: the windows of every probe token (windows_query) of every join.
-static __global__ void k_windows_mj(const JoinArgs* __restrict__ joins, TileMap m, const uint32_t* __restrict__ poff,
+// Bound by the latency of its dependent searches, so by the warps in flight: at 8 CTAs
+// an SM (32 registers) 500,000 reads take 192 us, at 5 245; two or four searches per
+// lane side by side need the registers and lose (208 to 298 us; only 1,000,000
+// heavy-tailed records gain, 2.1 -> 1.5 ms).
+static __global__ void __launch_bounds__(256, 8) k_windows_mj(const JoinArgs* __restrict__ joins, TileMap m, const uint32_t* __restrict__ poff,
                                     uint2* __restrict__ win, uint32_t* __restrict__ wpre, uint32_t* __restrict__ wtot,
                                     uint4* __restrict__ meta, bool classes) {
     const uint32_t wid = threadIdx.x >> 5, nw = blockDim.x >> 5;

@@ -18,8 +18,6 @@ void upload(Ctx& c, T* dst, const std::vector<T>& v) {
 
 }  // namespace
 
-__global__ void k_widen(const uint32_t* in, uint64_t* out) { *out = *in; }
-
 int bits_for(uint64_t v) {
     int b = 1;
     while (b < 64 && (1ull << b) < v) b++;

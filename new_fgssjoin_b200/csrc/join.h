@@ -120,6 +120,8 @@ struct Batch {
     uint32_t *icnt = nullptr, *pcnt = nullptr;  // R + 1: index / probe prefix per record
     uint32_t *ioff = nullptr, *poff = nullptr;  // R + 1: their exclusive scans (totals at R)
     uint32_t* send = nullptr;          // nj x 65537
+    uint64_t* tot = nullptr;           // index entries and probe tokens of the batch
+    size_t words = 0;                  // bytes of status, stats, d_e and tot, one block
     uint32_t* heavy_q = nullptr;       // R + 1
     // output columns (batch_filter_verify): join j's at out_off[j]
     std::vector<uint64_t> out_off;

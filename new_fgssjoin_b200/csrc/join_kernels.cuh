@@ -195,49 +195,58 @@ __device__ __forceinline__ uint32_t warp_merge_count(const uint32_t* q, uint32_t
 // ------------------------------------------------------------- prefix stage
 
 // Per record: prefix lengths (data.cu:241-257), validation of the input
-// (sizes, order, tokens).  icnt / pcnt are the record's own slots.
-__device__ __forceinline__ void prep_record(const JoinArgs& a, uint32_t i, uint32_t* icnt, uint32_t* pcnt,
-                                            uint32_t& local_max, uint32_t& bad, unsigned long long& probe,
-                                            int check_tokens) {
+// (sizes, order).  icnt / pcnt are the record's own slots.  Returns how many
+// tokens are to be checked (prep_tokens): none where they may not be read.
+__device__ __forceinline__ uint32_t prep_record(const JoinArgs& a, uint32_t i, uint32_t* icnt, uint32_t* pcnt,
+                                                uint32_t& local_max, uint32_t& bad) {
     const uint32_t l = a.len[i];
     local_max = max(local_max, l);
     if ((uint64_t)a.pos[i] + l > a.n_tokens) {
         bad |= ST_BAD_OFFSETS;
         *icnt = 0;
         *pcnt = 0;
-        return;
+        return 0;
     }
     if (l > 65535u) {
         bad |= ST_TOO_LONG;
         *icnt = 0;
         *pcnt = 0;
-        return;
+        return 0;
     }
     if (i + 1 < a.n && a.len[i + 1] > l) bad |= ST_UNSORTED;
     *icnt = a.index[l];
     *pcnt = a.probe[l];
-    probe += a.probe[l];
-    if (check_tokens) {
-        const uint32_t* t = a.tok + a.pos[i];
-        uint32_t prev = 0;
-        for (uint32_t j = 0; j < l; j++) {
-            const uint32_t v = t[j];
-            if (v >= a.n_terms || (j > 0 && v <= prev)) bad |= ST_BAD_TOKENS;
-            prev = v;
-        }
+    return l;
+}
+
+// Warp-collective: every lane's l tokens at tok + pos ascend and the last is a term.
+// The warp reads one record after another: a lane per record takes fewer
+// instructions on short ones, but waits for its longest (150,000 heavy-tailed
+// records: 201 -> 47 us, 500,000 reads of about 135 tokens 98 -> 77 us; 48 joins of
+// 600,000 titles together 76 -> 98 us).
+__device__ __forceinline__ void prep_tokens(const uint32_t* __restrict__ tok, uint32_t n_terms, uint32_t pos, uint32_t l,
+                                            uint32_t& bad) {
+    if (l && __ldg(tok + pos + l - 1) >= n_terms) bad |= ST_BAD_TOKENS;
+    for (uint32_t m = __ballot_sync(kFull, l > 1); m; m &= m - 1) {
+        const uint32_t r = __ffs(m) - 1;
+        const uint32_t n = __shfl_sync(kFull, l, r);
+        const uint32_t* __restrict__ t = tok + __shfl_sync(kFull, pos, r);
+        bool up = true;
+#pragma unroll 4
+        for (uint32_t j = lane_id() + 1; j < n; j += 32) up &= __ldg(t + j - 1) < __ldg(t + j);
+        if (!up) bad |= ST_BAD_TOKENS;
     }
 }
 
-// Warp-collective: the warp's maximum size, status bits and probe-token count to the join.
-__device__ __forceinline__ void prep_flush(const JoinArgs& a, uint32_t* maxlen, uint32_t local_max, uint32_t bad,
-                                           unsigned long long probe) {
+// Warp-collective: the warp's maximum size and status bits to the join.  (The word
+// is looked at first: the maximum is in the first records, and thousands of warps'
+// atomics on one address would take longer than their records.)
+__device__ __forceinline__ void prep_flush(const JoinArgs& a, uint32_t local_max, uint32_t bad) {
     local_max = __reduce_max_sync(kFull, local_max);
     bad = __reduce_or_sync(kFull, bad);
-    probe = warp_sum(probe);
     if (lane_id() == 0) {
-        if (local_max) atomicMax(maxlen, local_max);
+        if (local_max > *(volatile uint32_t*)(a.status + 1)) atomicMax(a.status + 1, local_max);
         if (bad) atomicOr(a.status, bad);
-        if (probe) atomicAdd(&a.stats[SS_PROBE], probe);
     }
 }
 
@@ -761,7 +770,18 @@ __device__ __forceinline__ void bitmap_record(const JoinArgs& a, uint32_t r, uin
     __syncwarp();
     const uint32_t l = a.len[r];
     const uint32_t* t = a.tok + a.pos[r];
-    for (uint32_t j = lane; j < l; j += 32) {
+    uint32_t j = lane;
+    for (; j + 96 < l; j += 128) {  // four tokens of a long record in flight
+        uint32_t v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldg(t + j + 32 * u);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t b = (v[u] * 0x9E3779B1u) >> shift;
+            atomicOr(&sw[b >> 5], 1u << (b & 31));
+        }
+    }
+    for (; j < l; j += 32) {
         const uint32_t b = (__ldg(t + j) * 0x9E3779B1u) >> shift;
         atomicOr(&sw[b >> 5], 1u << (b & 31));
     }
