@@ -176,7 +176,10 @@ ClaimItems items_in_order(Ctx& c, const TileMap& m) {
 
 template <int MODE>
 void tiny_launch(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const TileMap& m, bool sided) {
-    const TileMap t = tiles_for(finer_tiles(m, 32), (uint64_t)8 * c.num_sms, kTinyWarps);
+    // 4 tiles for each of the 16 CTAs an SM is given, down to a record per warp: the first
+    // tiles hold the longest records (150,000 heavy-tailed ones 450 us at half a tile each,
+    // 330 at 4, 315 at 8, where 500,000 reads lose: 765 -> 825; more CTAs lose everywhere)
+    const TileMap t = tiles_for(finer_tiles(m, 32), (uint64_t)64 * c.num_sms, kTinyWarps);
     const unsigned grid = std::min<unsigned>(t.ntiles, (unsigned)c.num_sms * 16);
     if (sided) k_tiny<MODE, true><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, t);
     else k_tiny<MODE, false><<<grid, kTinyWarps * 32, 0, c.stream>>>(d_args, d_fargs, t);

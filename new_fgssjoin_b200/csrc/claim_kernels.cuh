@@ -621,8 +621,12 @@ constexpr uint32_t kTinyWarps = 8;
 // k_claim would leave most of its 256 threads without an entry), in rows of 32 in the
 // lanes' registers in (probe position, source) order.  The claim of k_claim
 // within the warp: entry f writes f into its source's slot, the number w that
-// stays leads the source, the largest number is the last match.  CTAs take 32
-// consecutive records of a join (an eighth of a 256-record tile).
+// stays leads the source, the largest number is the last match.  CTAs take tiles of
+// 8 to 32 consecutive records of a join.  Bound by the latency of a query's chain of
+// loads (windows, entries, bounds, bitmaps, merges; 0.8 instructions a cycle):
+// 64 registers for 4 CTAs an SM, the queries' bounds and offsets and four chunks
+// of a merge's tokens fetched at once (500,000 reads at t = 0.8 1.05 -> 0.77 ms,
+// 48 joins of titles 0.57 -> 0.47; at 3 CTAs 0.94 and 0.55, at 5 0.81 and 0.61).
 struct TinyShared {
     uint32_t at[kTinyMax];    // entry of number f
     uint32_t src[kTinyMax];
@@ -633,7 +637,7 @@ struct TinyShared {
 };
 
 template <int MODE, bool SIDED>
-__global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __restrict__ joins,
+__global__ void __launch_bounds__(kTinyWarps * 32, 4) k_tiny(const JoinArgs* __restrict__ joins,
                                                           const FusedArgs* __restrict__ fargs, TileMap m) {
     __shared__ TinyShared s_all[kTinyWarps];
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, lt = lanemask_lt();
@@ -658,15 +662,19 @@ __global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __rest
         // warp w takes records r0 + w, r0 + w + 8, ...
         const uint32_t rec = r0 + wid + lane * kTinyWarps;
         const uint4 mt = lane < 32 / kTinyWarps && rec < t.r1 ? fa.meta[rec] : make_uint4(0, 0, QC_NONE << 16, 0);
+        uint32_t qp0 = 0, po0 = 0;  // of each lane's query: their loads are in flight together
+        if ((mt.z >> 16) == QC_TINY) {
+            qp0 = a.probe[mt.y];
+            po0 = fa.poff[rec];
+        }
 #pragma unroll 1
         for (uint32_t todo = __ballot_sync(kFull, (mt.z >> 16) == QC_TINY); todo; todo &= todo - 1) {
             const uint32_t ln = __ffs(todo) - 1, q = r0 + wid + ln * kTinyWarps;
             const uint32_t lq = __shfl_sync(kFull, mt.y, ln), W = __shfl_sync(kFull, mt.w, ln);
             const uint32_t* __restrict__ qt = a.tok + __shfl_sync(kFull, mt.x, ln);
-            const uint32_t qp = a.probe[lq], po = fa.poff[q];
+            const uint32_t qp = __shfl_sync(kFull, qp0, ln), po = __shfl_sync(kFull, po0, ln);
             for (uint32_t j = lane; j < qp; j += 32) {
                 const uint2 w = __ldg(fa.win + po + j);
-                if (w.x == w.y) continue;
                 uint32_t p = __ldg(fa.wpre + po + j);
                 for (uint32_t x = w.x; x < w.y; x++, p++) {
                     sh.at[p] = x;
@@ -755,7 +763,7 @@ __global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __rest
                     plain_take<MODE>(a, q, i0 + lane < nv, sh.src[f], sh.agg[f].y);
                 } else {
                     bool check = false;
-                    uint32_t s0 = 0, y0 = 0, cj0 = 0, im0 = 0;
+                    uint32_t s0 = 0, y0 = 0, cj0 = 0, im0 = 0, at0 = 0;
                     if (i0 + lane < nv) {
                         const uint32_t f = sh.vl[i0 + lane];
                         const uint2 g = sh.agg[f];
@@ -763,6 +771,7 @@ __global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __rest
                         y0 = g.x;
                         cj0 = g.y;
                         im0 = __ldg(&smin[y0 >> 16].y);
+                        at0 = fa.meta[s0].x;
                         check = bitmap_keeps(fa.bmap + (uint64_t)fa.bmw * q, fa.bmap + (uint64_t)fa.bmw * s0, fa.bmw,
                                              lq + (y0 >> 16), im0);
                     }
@@ -773,14 +782,22 @@ __global__ void __launch_bounds__(kTinyWarps * 32) k_tiny(const JoinArgs* __rest
                         const uint32_t s = __shfl_sync(kFull, s0, l), y = __shfl_sync(kFull, y0, l);
                         const uint32_t cj = __shfl_sync(kFull, cj0, l), im = __shfl_sync(kFull, im0, l);
                         const uint32_t ls = y >> 16, c = cj & 0xffffu, j = cj >> 16, qrest = lq - j - 1, k0 = (y & 0xffffu) + 1;
-                        const uint32_t* st = a.tok + fa.meta[s].x;
+                        const uint32_t* st = a.tok + __shfl_sync(kFull, at0, l);
                         uint32_t k = k0, cnt = c;
 #pragma unroll 1
                         while (k < ls && cnt + min(ls - k, qrest - (cnt - c)) >= im) {
-                            const uint32_t kk = k + lane;
-                            const bool hit = kk < ls && contains_gen(qt, j + 1, lq, __ldg(st + kk));
-                            cnt += __popc(__ballot_sync(kFull, hit));
-                            k = min(k + 32u, ls);
+                            uint32_t tk[4];  // four chunks of 32 source tokens in flight
+#pragma unroll
+                            for (uint32_t u = 0; u < 4; u++) tk[u] = k + 32 * u + lane < ls ? __ldg(st + k + 32 * u + lane) : 0u;
+#pragma unroll 1
+                            for (uint32_t u = 0; u < 4 && k < ls && cnt + min(ls - k, qrest - (cnt - c)) >= im; u++) {
+                                const bool hit = k + lane < ls && contains_gen(qt, j + 1, lq, tk[0]);
+                                cnt += __popc(__ballot_sync(kFull, hit));
+                                k = min(k + 32u, ls);
+                                tk[0] = tk[1];
+                                tk[1] = tk[2];
+                                tk[2] = tk[3];
+                            }
                         }
                         if (lane == 0) {
                             ctr.merged += k - k0;
