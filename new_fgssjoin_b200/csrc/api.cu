@@ -133,7 +133,10 @@ void export_pairs(Ctx& c, JoinState& J, const fgss_join_opts& o, fgss_pairs* out
         out->on_device = 1;
     } else {
         alloc_host_pairs(out, R);
-        if (R) {
+        if (R && out->priv) {  // both sides are six columns of one block: one copy
+            const size_t col = (char*)out->s - (char*)out->q;
+            FGSS_CK(cudaMemcpy2DAsync(out->q, col, J.oq, J.out_col * 4, R * 4, 6, cudaMemcpyDeviceToHost, c.stream));
+        } else if (R) {
             FGSS_CK(cudaMemcpyAsync(out->q, J.oq, R * 4, cudaMemcpyDeviceToHost, c.stream));
             FGSS_CK(cudaMemcpyAsync(out->s, J.os, R * 4, cudaMemcpyDeviceToHost, c.stream));
             FGSS_CK(cudaMemcpyAsync(out->id_q, J.oidq, R * 4, cudaMemcpyDeviceToHost, c.stream));
@@ -163,10 +166,8 @@ void export_batch(Ctx& c, Batch& B, const fgss_join_opts* opts, fgss_pairs* outs
     }
     const uint64_t oc = B.out_cap;
     uint32_t* st = c.pinnedT<uint32_t>("b.stage", 6 * oc + 1);
-    const void* cols[6] = {B.oq, B.os, B.oidq, B.oids, B.oo, B.osim};
     if (oc) {
-        for (int k = 0; k < 6; k++)
-            FGSS_CK(cudaMemcpyAsync(st + k * oc, cols[k], oc * 4, cudaMemcpyDeviceToHost, c.stream));
+        FGSS_CK(cudaMemcpy2DAsync(st, oc * 4, B.oq, B.out_col * 4, oc * 4, 6, cudaMemcpyDeviceToHost, c.stream));
         c.sync();
     }
     for (size_t j = 0; j < nj; j++) {

@@ -750,15 +750,18 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     for (size_t i = 0; i < nj; i++) B.out_off[i + 1] = B.out_off[i] + rcap[i];
     B.out_cap = B.out_off[nj];
     const uint64_t oc = B.out_cap;
-    B.oq = c.devT<uint32_t>(p + "b.o.q", oc + 1);
-    B.os = c.devT<uint32_t>(p + "b.o.s", oc + 1);
-    B.oidq = c.devT<uint32_t>(p + "b.o.idq", oc + 1);
-    B.oids = c.devT<uint32_t>(p + "b.o.ids", oc + 1);
-    B.oo = c.devT<uint32_t>(p + "b.o.o", oc + 1);
-    B.osim = c.devT<float>(p + "b.o.sim", oc + 1);
+    B.out_col = out_column(oc);
+    uint32_t* o6 = c.devT<uint32_t>(p + "b.o", 6 * B.out_col);
+    B.oq = o6;
+    B.os = o6 + B.out_col;
+    B.oidq = o6 + 2 * B.out_col;
+    B.oids = o6 + 3 * B.out_col;
+    B.oo = o6 + 4 * B.out_col;
+    B.osim = reinterpret_cast<float*>(o6 + 5 * B.out_col);
     for (size_t i = 0; i < nj; i++) {
         JoinState& J = *joins[i];
         const uint64_t o = B.out_off[i];
+        J.out_col = B.out_col;
         J.oq = B.oq + o;
         J.os = B.os + o;
         J.oidq = B.oidq + o;

@@ -162,12 +162,13 @@ HeavyScratch heavy_scratch(Ctx& c, const std::string& prefix, uint64_t n, uint32
 
 void join_output(Ctx& c, JoinState& J, uint64_t* keys, uint32_t* vals, const uint64_t* d_n, uint64_t n_cap) {
     const uint64_t n = J.in.n_sets;
-    J.oq = c.devT<uint32_t>(J.pfx("o.q"), n_cap + 1);
-    J.os = c.devT<uint32_t>(J.pfx("o.s"), n_cap + 1);
-    J.oidq = c.devT<uint32_t>(J.pfx("o.idq"), n_cap + 1);
-    J.oids = c.devT<uint32_t>(J.pfx("o.ids"), n_cap + 1);
-    J.oo = c.devT<uint32_t>(J.pfx("o.o"), n_cap + 1);
-    J.osim = c.devT<float>(J.pfx("o.sim"), n_cap + 1);
+    J.out_col = out_column(n_cap);
+    J.oq = c.devT<uint32_t>(J.pfx("o"), 6 * J.out_col);
+    J.os = J.oq + J.out_col;
+    J.oidq = J.oq + 2 * J.out_col;
+    J.oids = J.oq + 3 * J.out_col;
+    J.oo = J.oq + 4 * J.out_col;
+    J.osim = reinterpret_cast<float*>(J.oq + 5 * J.out_col);
     if (n_cap == 0) return;
     const int qb = bits_for(n);  // keys are q << qb | s
     radix_sort<uint64_t, uint32_t>(c, keys, vals, n_cap, d_n, 0, 2 * qb, J.pfx("rsort").c_str());

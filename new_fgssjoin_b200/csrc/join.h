@@ -30,6 +30,9 @@ constexpr int kFeat = 8;
 
 int bits_for(uint64_t v);  // bits needed to hold values < v (at least 1)
 
+// Words of an output column of n results: six lie in one device block.
+inline uint64_t out_column(uint64_t n) { return (n + 64) & ~uint64_t(63); }
+
 // Everything one join keeps on the device between stages.
 struct JoinState {
     int slot = 0;              // buffer-name prefix (joins of a batch use different slots)
@@ -50,6 +53,7 @@ struct JoinState {
     uint64_t* d_nres = nullptr;
     uint32_t *oq = nullptr, *os = nullptr, *oidq = nullptr, *oids = nullptr, *oo = nullptr;
     float* osim = nullptr;
+    uint64_t out_col = 0;  // words from one of the six to the next: one block, one copy to the host
     uint64_t n_res = 0;
     uint64_t n_entries = ~0ull;  // index entries once read back (batched method)
     uint64_t res_cap_hint = 0;   // exact result count after an overflow
@@ -116,18 +120,19 @@ struct Batch {
     JoinArgs* d_args = nullptr;        // nj
     uint32_t* status = nullptr;        // nj x 8 (ST_* bits, longest record, heavy count, result count)
     unsigned long long* stats = nullptr;  // nj x SS_N
+    uint64_t* tot = nullptr;           // index entries and probe tokens of the batch
+    size_t words = 0;                  // bytes of status, stats, d_e and tot, one block
     uint64_t* d_e = nullptr;           // nj x 2: index entries per join
     uint32_t *icnt = nullptr, *pcnt = nullptr;  // R + 1: index / probe prefix per record
     uint32_t *ioff = nullptr, *poff = nullptr;  // R + 1: their exclusive scans (totals at R)
     uint32_t* send = nullptr;          // nj x 65537
-    uint64_t* tot = nullptr;           // index entries and probe tokens of the batch
-    size_t words = 0;                  // bytes of status, stats, d_e and tot, one block
     uint32_t* heavy_q = nullptr;       // R + 1
     // output columns (batch_filter_verify): join j's at out_off[j]
     std::vector<uint64_t> out_off;
     uint64_t out_cap = 0;
     uint32_t *oq = nullptr, *os = nullptr, *oidq = nullptr, *oids = nullptr, *oo = nullptr;
     float* osim = nullptr;
+    uint64_t out_col = 0;  // words from one of the six to the next: one block, one copy to the host
 };
 
 // Host-side decisions of one batched run, recorded eagerly and reused when the

@@ -27,15 +27,16 @@ int bits_needed(uint64_t v) {  // bits to hold values < v
     return b;
 }
 
-// Union sort keys: (0xffff - min(len, 0xffff)) << 32 | side << 31 | index.
+// Union sort keys: (0xffff - min(len, 0xffff)) << 32 | side << 31 | index.  (They
+// are written in the order of the low 32 bits, so the stable sort only takes the
+// sizes: two passes instead of six.)
 __global__ void k_rs_keys(const uint32_t* __restrict__ rlen, uint32_t nr, const uint32_t* __restrict__ slen,
-                          uint32_t ns, uint64_t* __restrict__ key, uint32_t* __restrict__ val) {
+                          uint32_t ns, uint64_t* __restrict__ key) {
     const uint32_t n = nr + ns;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t side = i >= nr, idx = side ? i - nr : i;
         const uint32_t len = side ? slen[idx] : rlen[idx];
         key[i] = ((uint64_t)(0xffffu - min(len, 0xffffu)) << 32) | ((uint64_t)side << 31) | idx;
-        val[i] = i;
     }
 }
 
@@ -59,28 +60,28 @@ __global__ void k_rs_union(const uint64_t* __restrict__ key, uint32_t n, const u
     }
 }
 
-// Union-index pairs (sorted by (q, s)) -> keys r << 32 | s in the sides' own
+// Union-index pairs (sorted by (q, s)) -> keys r << sb | s in the sides' own
 // indices, value = the pair's position.
 __global__ void k_rs_remap(const uint32_t* __restrict__ oq, const uint32_t* __restrict__ os, uint64_t n,
-                           const uint8_t* __restrict__ side, const uint32_t* __restrict__ orig,
+                           const uint8_t* __restrict__ side, const uint32_t* __restrict__ orig, uint32_t sb,
                            uint64_t* __restrict__ key, uint32_t* __restrict__ val) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t a = oq[i], b = os[i];
         const bool a_is_r = side[a] == 0;
         const uint32_t r = orig[a_is_r ? a : b], s = orig[a_is_r ? b : a];
-        key[i] = ((uint64_t)r << 32) | s;
+        key[i] = ((uint64_t)r << sb) | s;
         val[i] = (uint32_t)i;
     }
 }
 
-__global__ void k_rs_out(const uint64_t* __restrict__ key, const uint32_t* __restrict__ val, uint64_t n,
+__global__ void k_rs_out(const uint64_t* __restrict__ key, const uint32_t* __restrict__ val, uint64_t n, uint32_t sb,
                          const uint32_t* __restrict__ rid, const uint32_t* __restrict__ sid,
                          const uint32_t* __restrict__ oo, const float* __restrict__ osim, uint32_t* __restrict__ q,
                          uint32_t* __restrict__ s, uint32_t* __restrict__ idq, uint32_t* __restrict__ ids,
                          uint32_t* __restrict__ o, float* __restrict__ sim) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t k = key[i];
-        const uint32_t r = (uint32_t)(k >> 32), x = (uint32_t)k, v = val[i];
+        const uint32_t r = (uint32_t)(k >> sb), x = (uint32_t)(k & ((1ull << sb) - 1)), v = val[i];
         q[i] = r;
         s[i] = x;
         idq[i] = rid ? rid[r] : r;
@@ -145,11 +146,10 @@ RsInput rs_union(Ctx& c, const fgss_sets_view& r_in, const fgss_sets_view& s_in)
         FGSS_CK(cudaMemcpyAsync(utok + r.n_tokens, s.tokens, s.n_tokens * 4, cudaMemcpyDeviceToDevice, c.stream));
     if (n) {
         uint64_t* key = c.devT<uint64_t>("rs.u.key", n + 1);
-        uint32_t* val = c.devT<uint32_t>("rs.u.val", n + 1);
         k_rs_keys<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(r.len, (uint32_t)u.nr, s.len,
-                                                                        (uint32_t)u.ns, key, val);
+                                                                        (uint32_t)u.ns, key);
         FGSS_LAUNCH_CK();
-        radix_sort<uint64_t, uint32_t>(c, key, val, n, nullptr, 0, 48, "rs.u.sort");
+        radix_sort<uint64_t, uint32_t>(c, key, nullptr, n, nullptr, 32, 48, "rs.u.sort");
         k_rs_union<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(
             key, (uint32_t)n, r.pos, r.len, r.n_tokens, s.pos, s.len, s.n_tokens, upos, ulen, u.side, u.orig, bad);
         FGSS_LAUNCH_CK();
@@ -171,23 +171,23 @@ RsInput rs_union(Ctx& c, const fgss_sets_view& r_in, const fgss_sets_view& s_in)
 
 void rs_output(Ctx& c, JoinState& J, const RsInput& u) {
     const uint64_t n = J.n_res;
-    uint32_t* q = c.devT<uint32_t>("rs.o.q", n + 1);
-    uint32_t* s = c.devT<uint32_t>("rs.o.s", n + 1);
-    uint32_t* idq = c.devT<uint32_t>("rs.o.idq", n + 1);
-    uint32_t* ids = c.devT<uint32_t>("rs.o.ids", n + 1);
-    uint32_t* o = c.devT<uint32_t>("rs.o.o", n + 1);
-    float* sim = c.devT<float>("rs.o.sim", n + 1);
+    const uint64_t col = out_column(n);
+    uint32_t* q = c.devT<uint32_t>("rs.o", 6 * col);
+    uint32_t *s = q + col, *idq = q + 2 * col, *ids = q + 3 * col, *o = q + 4 * col;
+    float* sim = reinterpret_cast<float*>(q + 5 * col);
     if (n) {
         uint64_t* key = c.devT<uint64_t>("rs.o.key", n + 1);
         uint32_t* val = c.devT<uint32_t>("rs.o.val", n + 1);
-        k_rs_remap<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(J.oq, J.os, n, u.side, u.orig, key, val);
+        const int sb = bits_needed(u.ns);
+        k_rs_remap<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(J.oq, J.os, n, u.side, u.orig, (uint32_t)sb,
+                                                                          key, val);
         FGSS_LAUNCH_CK();
-        radix_sort<uint64_t, uint32_t>(c, key, val, n, nullptr, 0, bits_needed(u.ns), "rs.o.sort.lo");
-        radix_sort<uint64_t, uint32_t>(c, key, val, n, nullptr, 32, 32 + bits_needed(u.nr), "rs.o.sort.hi");
-        k_rs_out<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(key, val, n, u.rid, u.sid, J.oo, J.osim, q, s,
-                                                                        idq, ids, o, sim);
+        radix_sort<uint64_t, uint32_t>(c, key, val, n, nullptr, 0, sb + bits_needed(u.nr), "rs.o.sort");
+        k_rs_out<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(key, val, n, (uint32_t)sb, u.rid, u.sid, J.oo,
+                                                                        J.osim, q, s, idq, ids, o, sim);
         FGSS_LAUNCH_CK();
     }
+    J.out_col = col;
     J.oq = q;
     J.os = s;
     J.oidq = idq;
