@@ -1,8 +1,9 @@
 // batch.cu -- the batched method: every join of a batch in one launch per
-// stage (per-record counts, index, windows, bitmaps, chunk splits, features,
-// learned estimates, work-item costs, items, one persistent fused
-// filter+verify launch, one global-accumulator launch, result keys, sort,
-// output), presized result buffers with an exact re-run on overflow.
+// stage (per-record counts, index, windows, bitmaps; where they are needed
+// features, learned estimates, work-item costs, items, chunk splits; one
+// filter+verify launch per class of queries, one global-accumulator launch,
+// result keys, sort, output), presized result buffers with an exact re-run on
+// overflow; and the plain method's filter and verification of one join.
 #include <string.h>
 
 #include <algorithm>
@@ -130,29 +131,35 @@ void fused_launch(Ctx& c, const TuneEntry& te, const JoinArgs* d_args, const Fus
 
 namespace {
 
-// k_claim's shape: 256 consumer threads with 8 entries each and 8192 claim
-// slots, 3 CTAs per SM (56 KB of shared memory each, which leaves the L1 about
-// 60 KB).  Measured on 1,000,000 heavy-tailed records at t = 0.7 / 100,000
-// titles at t = 0.5: 93.5 / 4.36 ms; 6 entries 98.5 / 4.29; 4 entries and 4
-// CTAs 105 / 4.74; 512 threads and 2 CTAs 103 / 4.90.
-using Claim = ClaimShape<256, 8, 13>;
+// k_claim's shapes: 256 consumer threads, 8192 claim slots, 6 entries a thread or 8
+// (wide), 3 CTAs per SM (53 and 59 KB of shared memory each: at 66 KB and more the L1
+// that is left costs 10 %).  The wide shape has fewer steps, the other no spills and
+// less to lay out for a short step.  6 / 8 entries, kernel time: 1,000,000
+// heavy-tailed records at t = 0.7 (5,350 window entries a query) 99.9 / 94.9 ms;
+// 100,000 titles at t = 0.5 (3,356) 4.14 / 4.24; R-S of 2 x 60,000 titles at t = 0.6
+// 3.44 / 3.47; 150,000 heavy-tailed records at t = 0.85 (86) 0.54 / 0.58; 100,000 titles
+// at t = 0.7, plain 1.53 / 1.83.  (5 entries: 104.7, 4.14, 3.36, 0.52, 1.55; 4096 slots: 103.0,
+// 4.40, 3.46, 0.56, 1.58 with 6; 4 CTAs of 56 registers lose everywhere.)
+using Claim = ClaimShape<256, 6, 13>;
+using ClaimWide = ClaimShape<256, 8, 13>;
 constexpr int kClaimCtas = 3;
+constexpr uint64_t kClaimWideCost = 4096;  // average cost (k_cost_mj) of k_claim's queries from which it is wide
 
-template <int MODE, bool SIDED>
+template <class Shape, int MODE, bool SIDED>
 void claim_launch_as(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const ClaimItems& items,
                      uint32_t* counter) {
-    FGSS_CK(cudaFuncSetAttribute(k_claim<Claim, kClaimCtas, MODE, SIDED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Claim::bytes));
+    FGSS_CK(cudaFuncSetAttribute(k_claim<Shape, kClaimCtas, MODE, SIDED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)Shape::bytes));
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)kClaimCtas * c.num_sms, items.n);
-    k_claim<Claim, kClaimCtas, MODE, SIDED><<<grid, Claim::NT, Claim::bytes, c.stream>>>(d_args, d_fargs, items, counter);
+    k_claim<Shape, kClaimCtas, MODE, SIDED><<<grid, Shape::NT, Shape::bytes, c.stream>>>(d_args, d_fargs, items, counter);
     FGSS_LAUNCH_CK();
 }
 
-template <int MODE>
+template <int MODE, class Shape = Claim>
 void claim_launch(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const ClaimItems& items, uint32_t* counter,
                   bool sided) {
-    if (sided) claim_launch_as<MODE, true>(c, d_args, d_fargs, items, counter);
-    else claim_launch_as<MODE, false>(c, d_args, d_fargs, items, counter);
+    if (sided) claim_launch_as<Shape, MODE, true>(c, d_args, d_fargs, items, counter);
+    else claim_launch_as<Shape, MODE, false>(c, d_args, d_fargs, items, counter);
 }
 
 // m in tiles small enough to make at least `want` of them, but not below `low` records.
@@ -576,6 +583,7 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     std::vector<uint32_t> K[2] = {std::vector<uint32_t>(nj, 0), std::vector<uint32_t>(nj, 0)};
     uint64_t nitems[2] = {0, 0};
     bool tiny = classes && B.R != 0;
+    bool wide = capture && plan->wide;  // (light: the costs are not known)
     uint64_t* hsum = c.pinnedT<uint64_t>(p + "b.hsum", std::max<size_t>(pp.n_sums, 1));
     if (light) {
         // nothing to read back
@@ -595,6 +603,11 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
         const uint64_t* count = hsum + 2 * nj;  // queries per class
         for (int k = 0; k < 2; k++) {
             if (k == QC_CLAIM && !classes) continue;
+            if (k == QC_CLAIM) {
+                uint64_t cost = 0;
+                for (size_t i = 0; i < nj; i++) cost += hsum[nj + i];
+                wide = count[k] != 0 && cost / count[k] >= kClaimWideCost;
+            }
             if (count[k] == 0 && !plan) continue;
             uint64_t grand = 0;
             for (size_t i = 0; i < nj; i++) grand += hsum[k * nj + i];
@@ -673,7 +686,8 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
         upload_args(c, B, p + "b.ha2");
         FGSS_CK(cudaMemsetAsync(counter, 0, (4 + nj) * 4, c.stream));
         FGSS_CK(cudaEventRecordWithFlags(c.ev[4], c.stream, rec_flags));
-        if (claims.n) claim_launch<MODE_FUSED>(c, B.d_args, d_fargs, claims, counter + 1, sided);
+        if (claims.n && wide) claim_launch<MODE_FUSED, ClaimWide>(c, B.d_args, d_fargs, claims, counter + 1, sided);
+        else if (claims.n) claim_launch<MODE_FUSED>(c, B.d_args, d_fargs, claims, counter + 1, sided);
         if (nitems[QC_KEYED])
             fused_launch(c, te, B.d_args, d_fargs, items[QC_KEYED], (uint32_t)nitems[QC_KEYED], counter, sided);
         if (tiny) tiny_launch<MODE_FUSED>(c, B.d_args, d_fargs, B.rec, sided);
@@ -723,6 +737,7 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     }
     if (plan && !capture) {
         plan->te = te;
+        plan->wide = wide;
         for (int k = 0; k < 2; k++) plan->K[k] = K[k];
         for (int k = 0; k < 2; k++) plan->nitems[k] = nitems[k];
         plan->heavy_slots = slots;

@@ -1,5 +1,5 @@
-// claim_kernels.cuh -- the batched method's filter + verify kernels: k_claim (a
-// CTA per query) and k_tiny (a warp per query of few window entries).  Same
+// claim_kernels.cuh -- the filter + verify kernels (the plain method's filter
+// passes too): k_claim (a CTA per query) and k_tiny (a warp per query of few window entries).  Same
 // semantics as k_fused (fused_kernels.cuh), whose keyed slot table remains for
 // the strategies a caller asks for, tuned keyed shapes and probe prefixes above
 // kClaimPC tokens.
@@ -13,8 +13,9 @@
 // every query, instead of a binary search per query, probe token and
 // range.  Measured (filter kernels of a call, chunk splits included): 1,000,000
 // heavy-tailed records at t = 0.7 177 -> 95 ms, 100,000 titles at t = 0.5
-// 12.1 -> 4.4 ms, 2 x 60,000 titles R-S at t = 0.6 6.3 -> 4.3 ms, 500,000
-// reads at t = 0.8 2.8 -> 1.4 ms.
+// 12.1 -> 4.2 ms, 2 x 60,000 titles R-S at t = 0.6 6.3 -> 3.5 ms, 500,000
+// reads at t = 0.8 2.8 -> 0.95 ms, 100,000 titles at t = 0.7 with the plain method's
+// two passes 8.4 -> 1.6 ms.
 #pragma once
 
 #include "fused_kernels.cuh"
@@ -67,7 +68,7 @@ struct ClaimShape {
     static constexpr uint32_t PC = kClaimPC;
     static constexpr uint32_t JE = NTC * U;   // entries of a step
     static constexpr uint32_t JW = JE / 32;   // their groups of 32
-    static constexpr uint32_t QC = 512;       // query tokens staged
+    static constexpr uint32_t QC = 256;       // query tokens staged (longer: read from global memory)
     static constexpr uint32_t BW = 1024;      // membership words: one bit per term up to 32768 terms
     static constexpr uint32_t MC = 256;       // merge list
     static constexpr size_t off_agg = 0;                          // uint2[JE]

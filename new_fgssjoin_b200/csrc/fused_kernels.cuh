@@ -1,4 +1,5 @@
-// fused_kernels.cuh -- the batched method's filter + verify kernel.
+// fused_kernels.cuh -- the batched method's pre-pass per query and its keyed
+// filter + verify kernel (queries of class QC_KEYED).
 //
 // Same semantics as the plain stages (join_kernels.cuh; reference
 // filtering.cu:76-141, checking.cu:93-175, block.cu:184-197), organised for

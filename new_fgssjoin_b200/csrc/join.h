@@ -141,6 +141,7 @@ struct BatchPlan {
     bool capture = false;             // issue device work only, with these decisions
     TuneEntry te;
     uint64_t E_cap = 0, P_cap = 0;    // index entries, probe windows the buffers hold
+    bool wide = false;                // k_claim's shape
     bool light = false;               // every query is the claim kernels', whose items are the records in order
     std::vector<uint32_t> K[2];       // work items per join (k_fused, k_claim)
     uint64_t nitems[2] = {0, 0};

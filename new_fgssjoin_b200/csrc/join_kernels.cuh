@@ -9,12 +9,13 @@
 //   verification       src/fgssjoin/checking.cu:93-175 (thread per candidate merge)
 //   compaction/output  src/fgssjoin/checking.cu:556-595, block.cu:184-197
 //
-// B200 design.  No block x block score matrix: a CTA owns one query at a time
-// and accumulates its candidates in a shared-memory hash table (a
-// global-memory dense accumulator for the few queries too large for it).
+// B200 design.  No block x block score matrix: a CTA (or a warp) owns one query
+// at a time and accumulates its candidates in shared memory: claim slots
+// (claim_kernels.cuh), and for long probe prefixes a keyed hash table (k_probe
+// here, k_fused) or a global-memory dense accumulator.
 // Sources are limited to an id window [q+1, send) found by binary search in
 // each inverted list (lists are sorted by source id, sources by descending
-// size), so entries outside the size filter are never read.  Each hash slot
+// size), so entries outside the size filter are never read.  A keyed slot
 // keeps (source, matches, last match position): the number of prefix matches
 // is the reference's partial score, the last match reproduces its positional
 // filter exactly (the bound it tests at every match is non-increasing, so it
@@ -798,6 +799,15 @@ inline uint32_t bitmap_words(uint64_t n_tokens, uint64_t n_sets) {
     return n_tokens > 96ull * (n_sets ? n_sets : 1) ? 4u : 2u;
 }
 
+// 32 bytes of global memory from a 32-byte boundary in one load: the lanes' bitmaps
+// lie at random, and two 16-byte loads take two turns per lane in the L1 (k_claim
+// 2 to 3 % of its time).
+__device__ __forceinline__ void load32(const uint4* p, uint4& x, uint4& y) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w), "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w)
+                 : "l"(p));
+}
+
 __device__ __forceinline__ uint32_t popc_xor(uint4 a, uint4 b) {
     return __popc(a.x ^ b.x) + __popc(a.y ^ b.y) + __popc(a.z ^ b.z) + __popc(a.w ^ b.w);
 }
@@ -806,8 +816,13 @@ __device__ __forceinline__ uint32_t popc_xor(uint4 a, uint4 b) {
 // need a merge?  q4: the query's bitmap (shared or global memory).
 __device__ __forceinline__ bool bitmap_keeps(const uint4* q4, const uint4* __restrict__ b4, uint32_t bmw, uint32_t S,
                                              uint32_t im) {
-    uint32_t pc = popc_xor(q4[0], __ldg(b4)) + popc_xor(q4[1], __ldg(b4 + 1));
-    if (bmw == 4) pc += popc_xor(q4[2], __ldg(b4 + 2)) + popc_xor(q4[3], __ldg(b4 + 3));
+    uint4 x, y;
+    load32(b4, x, y);
+    uint32_t pc = popc_xor(q4[0], x) + popc_xor(q4[1], y);
+    if (bmw == 4) {
+        load32(b4 + 2, x, y);
+        pc += popc_xor(q4[2], x) + popc_xor(q4[3], y);
+    }
     return S >= 2 * im + pc;
 }
 

@@ -105,3 +105,16 @@ def test_replay_after_records_grew(ctx):
             c.copy_(torch.from_numpy(np.asarray(x).astype(np.int32)))
         torch.cuda.synchronize()
         _check(ctx.selfjoin(v, 0.5, method="batched"), s, 0.5)
+
+
+@pytest.mark.parametrize("n", [1500, 5000])
+def test_claim_shapes(ctx, n):
+    """One record with a probe prefix beyond 640, so the costs are read back: below and above an
+    average of 4,096 window entries a query the claim kernel's two shapes run (about 1,800 and 6,000)."""
+    rng = np.random.default_rng(n)
+    recs = [np.sort(rng.choice(5000, 2600, replace=False))]
+    recs += [np.sort(rng.choice(40, 24, replace=False)) for _ in range(n)]
+    s = _sets(recs, 5000)
+    got = ctx.selfjoin(s, 0.7, method="batched")
+    assert (got.stats["window_entries"] / n >= 4096) == (n == 5000)
+    _check(got, s, 0.7)
