@@ -38,6 +38,7 @@ namespace {
 // call queued are done before it returns.
 void settle(fgss_ctx* ctx) {
     if (ctx && ctx->c.stream && cudaStreamSynchronize(ctx->c.stream) != cudaSuccess) (void)cudaGetLastError();
+    if (ctx && ctx->c.copy_stream && cudaStreamSynchronize(ctx->c.copy_stream) != cudaSuccess) (void)cudaGetLastError();
 }
 
 template <typename F>
@@ -638,6 +639,9 @@ void fgss_destroy(fgss_ctx* ctx) {
     for (auto& e : c.ev)
         if (e) cudaEventDestroy(e);
     if (c.err_host) cudaFreeHost(c.err_host);
+    for (auto& e : c.copy_ev)
+        if (e) cudaEventDestroy(e);
+    if (c.copy_stream) cudaStreamDestroy(c.copy_stream);
     if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);
     delete c.model;
     delete ctx;

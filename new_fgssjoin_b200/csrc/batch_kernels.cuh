@@ -9,7 +9,7 @@
 
 namespace fgss {
 
-// k_prep for every join: counts into the batch arrays icnt / pcnt (record g).
+// Prefix lengths and input checks of every join's records: counts into the batch arrays icnt / pcnt (record g).
 static __global__ void k_prep_mj(const JoinArgs* __restrict__ joins, TileMap m, uint32_t* __restrict__ icnt,
                                  uint32_t* __restrict__ pcnt) {
     // a warp takes an eighth of the tile, at most 32 records

@@ -53,6 +53,17 @@ struct Ctx {
     struct GraphCache* graphs = nullptr;  // captured batched pipelines (api.cu)
     fgss_model* model = nullptr;
     cudaEvent_t ev[8] = {};
+    // Copies to the host beside the kernels of later parts (tokenize.cu): made on
+    // first use; a call that used it waits for it before it returns.
+    static constexpr int kCopyParts = 4;
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t copy_ev[kCopyParts + 1] = {};
+    void copy_lane() {
+        if (copy_stream) return;
+        for (auto& e : copy_ev)
+            if (!e) FGSS_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        FGSS_CK(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
+    }
     bool probe_timed = false;  // ev[4]..ev[5] bracket the last fused filter+verify launch
     bool heavy_timed = false;  // ev[6]..ev[7] bracket the last global-accumulator launch
 

@@ -346,6 +346,7 @@ constexpr uint32_t kMaxLineGrams = 8192;   // grams of a line of tokenize_lines
 // Classes of lines by grams (a warp each; tables of 512 and 2048 slots at eight and
 // four warps per CTA, beyond that of twice the longest line at one warp per CTA) and
 // of records by tokens (a warp, 256 and 1024 threads each).
+constexpr uint64_t kPartTokens = 1 << 20;  // tokens from which a result is copied in parts
 constexpr uint32_t kSmallLine = 256, kMidLine = 1024;
 
 // Counters of one call, read back together.
@@ -679,13 +680,13 @@ __device__ __forceinline__ void sort_shared(S* v, uint32_t n, uint32_t t, uint32
     }
 }
 
-// Records of (lo, hi] tokens: tokens sorted by id, written at the record's
+// Records [first, end) of (lo, hi] tokens: tokens sorted by id, written at the record's
 // place (records are in descending size, so each class is a run of them).  S:
 // id << pb | position, 32 bits where that fits.  WARP: a warp per record, else a CTA.
 template <typename S, bool WARP>
 __global__ void k_records(const uint32_t* __restrict__ mline, const uint32_t* __restrict__ mlen,
-                          const uint32_t* __restrict__ moff, uint32_t nrec, uint32_t lo, uint32_t hi,
-                          const uint32_t* __restrict__ loff, const uint32_t* __restrict__ id,
+                          const uint32_t* __restrict__ moff, uint32_t first, uint32_t end, uint32_t lo,
+                          uint32_t hi, const uint32_t* __restrict__ loff, const uint32_t* __restrict__ id,
                           const uint32_t* __restrict__ pos, int pb, uint32_t* __restrict__ otok,
                           uint32_t* __restrict__ oloc) {
     extern __shared__ __align__(16) unsigned char s_rec[];
@@ -697,7 +698,7 @@ __global__ void k_records(const uint32_t* __restrict__ mline, const uint32_t* __
         else __syncthreads();
     };
     const S pm = ((S)1 << pb) - 1;
-    for (uint32_t i = blockIdx.x * nw + wid; i < nrec; i += gridDim.x * nw) {
+    for (uint32_t i = first + blockIdx.x * nw + wid; i < end; i += gridDim.x * nw) {
         const uint32_t n = mlen[i];
         if (n <= lo) break;  // shorter ones only from here on
         if (n > hi) continue;
@@ -824,28 +825,78 @@ void tokenize_terms(Ctx& c, const unsigned char* dtext, const uint32_t* lstart, 
     uint32_t* otok = c.devT<uint32_t>("tl.otok", (uint64_t)T + 1);
     uint32_t* oloc = c.devT<uint32_t>("tl.oloc", (uint64_t)T + 1);
     const int pb = bits_for32((uint64_t)h.max_grams + 1);
-    auto records = [&](auto tag) {
+    auto records = [&](auto tag, uint32_t a, uint32_t b) {
         using S = decltype(tag);
-        k_records<S, true><<<grid_for(nrec, 8, c.num_sms * 16), 256, 8 * kSmallLine * sizeof(S), c.stream>>>(
-            mline, mlen, moff, nrec, 0, kSmallLine, loff, id, pos, pb, otok, oloc);
+        k_records<S, true><<<grid_for(b - a, 8, c.num_sms * 16), 256, 8 * kSmallLine * sizeof(S), c.stream>>>(
+            mline, mlen, moff, a, b, 0, kSmallLine, loff, id, pos, pb, otok, oloc);
         FGSS_LAUNCH_CK();
-        if (h.max_size > kSmallLine) {
-            k_records<S, false><<<grid_for(h.n_mid + h.n_long, 1, c.num_sms * 8), 256, kMidLine * sizeof(S), c.stream>>>(
-                mline, mlen, moff, nrec, kSmallLine, kMidLine, loff, id, pos, pb, otok, oloc);
+        // (sizes descend: the longer ones are among the first)
+        if (h.max_size > kSmallLine && a < h.n_mid + h.n_long) {
+            k_records<S, false><<<grid_for(h.n_mid + h.n_long - a, 1, c.num_sms * 8), 256, kMidLine * sizeof(S), c.stream>>>(
+                mline, mlen, moff, a, b, kSmallLine, kMidLine, loff, id, pos, pb, otok, oloc);
             FGSS_LAUNCH_CK();
         }
-        if (h.max_size > kMidLine) {
+        if (h.max_size > kMidLine && a < h.n_long) {
             const size_t smem = (size_t)h.max_size * sizeof(S);
             FGSS_CK(cudaFuncSetAttribute(k_records<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(kMaxLineGrams * sizeof(S))));
-            k_records<S, false><<<grid_for(h.n_long, 1, c.num_sms * 2), 1024, smem, c.stream>>>(
-                mline, mlen, moff, nrec, kMidLine, h.max_size, loff, id, pos, pb, otok, oloc);
+            k_records<S, false><<<grid_for(h.n_long - a, 1, c.num_sms * 2), 1024, smem, c.stream>>>(
+                mline, mlen, moff, a, b, kMidLine, h.max_size, loff, id, pos, pb, otok, oloc);
             FGSS_LAUNCH_CK();
         }
     };
-    if (bits_for32((uint64_t)V + 1) + pb <= 32) records(uint32_t());
-    else records(uint64_t());
-    copy_out(c, out, nrec, T, V, mid, mlen, moff, otok, oloc);
+    const bool narrow = bits_for32((uint64_t)V + 1) + pb <= 32;
+    auto part = [&](uint32_t a, uint32_t b) {
+        if (narrow) records(uint32_t(), a, b);
+        else records(uint64_t(), a, b);
+    };
+    // A large result goes to the host in parts, each while the next one's records are sorted:
+    // 200,000 reads of 27 M tokens 11.3 -> 10.2 ms of the call, 200,000 titles 4.85 -> 4.28, 60,000
+    // heavy-tailed texts 4.13 -> 3.72 (in four equal parts, the first the longest: 10.6, 4.33, 3.92).
+    // Below 2^20 tokens (8 MB) the copies take no longer than the extra launches and events.
+    if (T < kPartTokens || nrec < Ctx::kCopyParts) {
+        part(0, nrec);
+        copy_out(c, out, nrec, T, V, mid, mlen, moff, otok, oloc);
+        return;
+    }
+    out->n_sets = nrec;
+    out->n_tokens = T;
+    out->n_terms = V;
+    alloc_host_sets(out, nrec, T, true);
+    c.copy_lane();
+    struct Settle {  // no copy is in flight when the call returns or fails
+        Ctx& c;
+        ~Settle() {
+            if (cudaStreamSynchronize(c.copy_stream) != cudaSuccess) (void)cudaGetLastError();
+        }
+    } settle{c};
+    constexpr int kParts = Ctx::kCopyParts;
+    uint32_t cut[kParts + 1], *hcut = c.pinnedT<uint32_t>("tl.hcut", kParts + 1);
+    // the first part's sort is the one that no copy hides, and its records are the longest
+    for (int i = 0; i <= kParts; i++) cut[i] = (uint32_t)((uint64_t)nrec * ((1u << i) - 1) / ((1u << kParts) - 1));
+    for (int i = 1; i < kParts; i++)
+        FGSS_CK(cudaMemcpyAsync(hcut + i, moff + cut[i], 4, cudaMemcpyDeviceToHost, c.stream));
+    FGSS_CK(cudaEventRecord(c.copy_ev[kParts], c.stream));
+    for (int i = 0; i < kParts; i++) {
+        part(cut[i], cut[i + 1]);
+        FGSS_CK(cudaEventRecord(c.copy_ev[i], c.stream));
+    }
+    FGSS_CK(cudaEventSynchronize(c.copy_ev[kParts]));
+    hcut[0] = 0;
+    hcut[kParts] = T;
+    cudaStream_t cs = c.copy_stream;
+    FGSS_CK(cudaMemcpyAsync(out->id, mid, (uint64_t)nrec * 4, cudaMemcpyDeviceToHost, cs));
+    FGSS_CK(cudaMemcpyAsync(out->len, mlen, (uint64_t)nrec * 4, cudaMemcpyDeviceToHost, cs));
+    FGSS_CK(cudaMemcpyAsync(out->pos, moff, (uint64_t)nrec * 4, cudaMemcpyDeviceToHost, cs));
+    for (int i = 0; i < kParts; i++) {
+        const uint64_t o = hcut[i], n = hcut[i + 1] - o;
+        FGSS_CK(cudaStreamWaitEvent(cs, c.copy_ev[i], 0));
+        FGSS_CK(cudaMemcpyAsync(out->tokens + o, otok + o, n * 4, cudaMemcpyDeviceToHost, cs));
+        FGSS_CK(cudaMemcpyAsync(out->loc + o, oloc + o, n * 4, cudaMemcpyDeviceToHost, cs));
+    }
+    FGSS_CK(cudaStreamSynchronize(cs));
+    c.sync();
+    out->max_len = out->len[0];  // descending sizes
 }
 
 void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokParams& p, fgss_sets* out);

@@ -59,3 +59,13 @@ def test_kmers(ctx, k):
 def test_text_layout(ctx, text):
     _check(ctx, text, q=3, pad=True, suffix=False, lower=True)
     _check(ctx, text, q=3, pad=False, suffix=True, lower=True)
+
+
+@pytest.mark.parametrize("sizes", [[256] * 4096, [256] * 4095 + [255], [8192] * 128,
+                                   [8000] * 3 + [1000] * 40 + [500] * 200 + [60] * 15500],
+                         ids=["2^20", "2^20-1", "long", "mixed"])
+def test_result_in_parts(ctx, sizes):
+    """Results of 2^20 tokens and more go to the host in parts of 1, 2, 4 and 8 fifteenths of the records."""
+    rng = np.random.default_rng(len(sizes))
+    lines = [_line(rng, n + 2, b"abcdefghijklmnopqrstuvwxyz ") for n in rng.permutation(sizes)]
+    _check(ctx, b"\n".join(lines), q=3, pad=False, suffix=True, lower=True)
