@@ -25,6 +25,9 @@ struct DevBounds {
 };
 DevBounds device_bounds(Ctx& c, float t, int mode);
 
+// v's host arrays in the device buffer `name`.
+fgss_sets_view sets_to_device(Ctx& c, const std::string& name, const fgss_sets_view& v);
+
 // Per-query features of the learned cost model (one row per record).
 constexpr int kFeat = 8;
 

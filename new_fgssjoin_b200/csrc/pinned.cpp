@@ -85,6 +85,16 @@ bool pinned_give(void* b) {
     return true;
 }
 
+bool pinned_holds(const void* p, size_t bytes) {
+    PinnedPool& P = pinned_pool();
+    std::lock_guard<std::mutex> lk(P.mu);
+    auto it = P.sizes.upper_bound(const_cast<void*>(p));
+    if (it == P.sizes.begin()) return false;
+    --it;
+    const char* b = static_cast<const char*>(it->first);
+    return static_cast<const char*>(p) + bytes <= b + it->second;
+}
+
 void alloc_host_sets(fgss_sets* s, uint64_t n, uint64_t T, bool loc) {
     const size_t nc = ((n + 1) * 4 + 255) & ~size_t(255), tc = ((T + 1) * 4 + 255) & ~size_t(255);
     if (char* b = static_cast<char*>(pinned_take(3 * nc + (loc ? 2 : 1) * tc))) {

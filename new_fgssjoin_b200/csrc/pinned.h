@@ -12,6 +12,9 @@ void* pinned_take(size_t bytes);
 // Gives a block of the pool back (true), or returns false for other memory.
 bool pinned_give(void* b);
 
+// Does one block of the pool hold the `bytes` bytes from p?
+bool pinned_holds(const void* p, size_t bytes);
+
 // Columns of n records and T tokens (freed by fgss_sets_free): one page-locked
 // block of 256-byte aligned columns that starts with `id`, so the copies from
 // the device, and to it when the sets are joined, run at the link's rate; or

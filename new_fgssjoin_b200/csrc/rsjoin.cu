@@ -94,28 +94,9 @@ __global__ void k_rs_out(const uint64_t* __restrict__ key, const uint32_t* __res
 // A side's arrays on the device (copied when the caller's are host memory).
 fgss_sets_view rs_side_on_device(Ctx& c, const fgss_sets_view& v, const char* tag) {
     if (v.on_device) return v;
-    fgss_sets_view d = v;
-    const std::string t(tag);
-    uint32_t* pos = c.devT<uint32_t>("rs." + t + ".pos", v.n_sets + 1);
-    uint32_t* len = c.devT<uint32_t>("rs." + t + ".len", v.n_sets + 1);
-    uint32_t* tok = c.devT<uint32_t>("rs." + t + ".tok", v.n_tokens + 1);
-    uint32_t* id = v.id ? c.devT<uint32_t>("rs." + t + ".id", v.n_sets + 1) : nullptr;
-    if (v.n_sets) {
-        if (!v.pos || !v.len) fail(FGSS_ERR_INVALID, "null record arrays");
-        FGSS_CK(cudaMemcpyAsync(pos, v.pos, v.n_sets * 4, cudaMemcpyHostToDevice, c.stream));
-        FGSS_CK(cudaMemcpyAsync(len, v.len, v.n_sets * 4, cudaMemcpyHostToDevice, c.stream));
-        if (id) FGSS_CK(cudaMemcpyAsync(id, v.id, v.n_sets * 4, cudaMemcpyHostToDevice, c.stream));
-    }
-    if (v.n_tokens) {
-        if (!v.tokens) fail(FGSS_ERR_INVALID, "null token array");
-        FGSS_CK(cudaMemcpyAsync(tok, v.tokens, v.n_tokens * 4, cudaMemcpyHostToDevice, c.stream));
-    }
-    d.pos = pos;
-    d.len = len;
-    d.tokens = tok;
-    d.id = id;
-    d.on_device = 1;
-    return d;
+    if (v.n_sets && (!v.pos || !v.len)) fail(FGSS_ERR_INVALID, "null record arrays");
+    if (v.n_tokens && !v.tokens) fail(FGSS_ERR_INVALID, "null token array");
+    return sets_to_device(c, std::string("rs.") + tag, v);
 }
 
 }  // namespace
