@@ -753,8 +753,13 @@ void launch_lines(Ctx& c, const unsigned char* text, const uint32_t* lstart, con
     uint32_t slots = 64;
     while (slots < 2 * grams) slots <<= 1;
     const size_t smem = (size_t)warps * slots * (sizeof(K) + 4);
+    // Every launch sets the largest table of any class, not its own: the limit belongs to the
+    // function, which all contexts of a device share, and a thread that lowered it between
+    // another one's setting and launch would have that launch refused.
+    constexpr int kMost = (int)(2 * kMaxLineGrams * (sizeof(K) + 4));
+    static_assert(8 * 2 * kSmallLine <= 2 * kMaxLineGrams && 4 * 2 * kMidLine <= 2 * kMaxLineGrams, "largest table");
     if (smem + 1024 > 48 * 1024)  // (with the static code table)
-        FGSS_CK(cudaFuncSetAttribute(k_lines<K, KO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        FGSS_CK(cudaFuncSetAttribute(k_lines<K, KO>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
     k_lines<K, KO><<<grid_for(n, warps, c.num_sms * 16), warps * 32, smem, c.stream>>>(
         text, lstart, lend, list, n, p, lut, cb, slots, fill, ob, lsz, loff, key, num, pos, cnt);
     FGSS_LAUNCH_CK();
