@@ -15,6 +15,7 @@
 #include <thread>
 #include <vector>
 
+#include "guard.h"
 #include "join.h"
 #include "model.h"
 #include "pinned.h"
@@ -33,39 +34,6 @@ void set_thread_error(const std::string& msg) { g_err = msg; }
 }  // namespace fgss
 
 namespace {
-
-// After an error: copies from or to the caller's page-locked arrays that the
-// call queued are done before it returns.
-void settle(fgss_ctx* ctx) {
-    if (ctx && ctx->c.stream && cudaStreamSynchronize(ctx->c.stream) != cudaSuccess) (void)cudaGetLastError();
-    if (ctx && ctx->c.copy_stream && cudaStreamSynchronize(ctx->c.copy_stream) != cudaSuccess) (void)cudaGetLastError();
-}
-
-template <typename F>
-fgss_status guard(fgss_ctx* ctx, F&& f) {
-    try {
-        f();
-        if (ctx && ctx->c.err_host && *(volatile uint32_t*)ctx->c.err_host) {
-            *ctx->c.err_host = 0;
-            fail(FGSS_ERR_TIMEOUT, "a device wait of a scan or sort gave up");
-        }
-        if (ctx) ctx->c.last_error.clear();
-        return FGSS_OK;
-    } catch (const Error& e) {
-        settle(ctx);
-        if (ctx) ctx->c.last_error = e.msg;
-        g_err = e.msg;
-        return e.st;
-    } catch (const std::bad_alloc&) {
-        settle(ctx);
-        if (ctx) ctx->c.last_error = "host allocation failed";
-        return FGSS_ERR_NOMEM;
-    } catch (...) {
-        settle(ctx);
-        if (ctx) ctx->c.last_error = "unknown error";
-        return FGSS_ERR_CUDA;
-    }
-}
 
 struct PairsPriv {
     bool host_owned;
@@ -118,6 +86,7 @@ void export_pairs(Ctx& c, JoinState& J, const fgss_join_opts& o, fgss_pairs* out
     const uint64_t R = J.n_res;
     out->n = R;
     if (o.out_on_device) {
+        out->on_device = 1;
         // hand out library buffers: copies so the context can be reused
         auto dup = [&](const void* src, size_t bytes) -> void* {
             void* p = nullptr;
@@ -131,7 +100,6 @@ void export_pairs(Ctx& c, JoinState& J, const fgss_join_opts& o, fgss_pairs* out
         out->id_s = (uint32_t*)dup(J.oids, R * 4);
         out->overlap = (uint32_t*)dup(J.oo, R * 4);
         out->sim = (float*)dup(J.osim, R * 4);
-        out->on_device = 1;
     } else {
         alloc_host_pairs(out, R);
         if (R && out->priv) {  // both sides are six columns of one block: one copy
@@ -145,7 +113,6 @@ void export_pairs(Ctx& c, JoinState& J, const fgss_join_opts& o, fgss_pairs* out
             FGSS_CK(cudaMemcpyAsync(out->overlap, J.oo, R * 4, cudaMemcpyDeviceToHost, c.stream));
             FGSS_CK(cudaMemcpyAsync(out->sim, J.osim, R * 4, cudaMemcpyDeviceToHost, c.stream));
         }
-        out->on_device = 0;
     }
     if (!J.cand_host.empty() || o.want_candidates) {
         out->n_cand = J.cand_host.size() / 3;
@@ -369,10 +336,8 @@ bool replay_graph(Ctx& c, GraphEntry& g, const fgss_sets_view* sets, const fgss_
     return true;
 }
 
-void run_joins(Ctx& c, const fgss_sets_view* sets, const fgss_join_opts* opts, int n, fgss_pairs* outs,
-               fgss_stats* stats) {
-    if (n <= 0) return;
-    if (!sets || !opts || !outs) fail(FGSS_ERR_INVALID, "null argument");
+void joins_of_call(Ctx& c, const fgss_sets_view* sets, const fgss_join_opts* opts, int n, fgss_pairs* outs,
+                   fgss_stats* stats) {
     bool batched = false;
     for (int i = 0; i < n; i++) batched |= opts[i].method == FGSS_METHOD_BATCHED;
     if (batched && opts[0].want_candidates) fail(FGSS_ERR_INVALID, "want_candidates needs the plain method");
@@ -533,6 +498,19 @@ void run_joins(Ctx& c, const fgss_sets_view* sets, const fgss_join_opts* opts, i
     c.bpfx.clear();
 }
 
+// A failed call hands out nothing: the pairs of its joins that were done are freed.
+void run_joins(Ctx& c, const fgss_sets_view* sets, const fgss_join_opts* opts, int n, fgss_pairs* outs,
+               fgss_stats* stats) {
+    if (n <= 0) return;
+    if (!sets || !opts || !outs) fail(FGSS_ERR_INVALID, "null argument");
+    memset(outs, 0, sizeof(fgss_pairs) * (size_t)n);
+    or_undo(
+        c, [&] { joins_of_call(c, sets, opts, n, outs, stats); },
+        [&] {
+            for (int i = 0; i < n; i++) fgss_pairs_free(&outs[i]);
+        });
+}
+
 }  // namespace
 
 extern "C" {
@@ -685,12 +663,8 @@ fgss_status fgss_tokenize(fgss_ctx* ctx, const char* text, uint64_t n_bytes, con
         if (opts) o = *opts;
         TokParams p{o.q, o.mode, o.pad, o.pad_char, o.suffix, o.lower};
         FGSS_CK(cudaSetDevice(ctx->c.device));
-        try {
-            tokenize_device(ctx->c, text, n_bytes, p, out);
-        } catch (...) {
-            fgss_sets_free(out);
-            throw;
-        }
+        or_undo(
+            ctx->c, [&] { tokenize_device(ctx->c, text, n_bytes, p, out); }, [&] { fgss_sets_free(out); });
     });
 }
 
@@ -718,7 +692,7 @@ fgss_status fgss_tokenize_dual(fgss_ctx* ctx, const char* text_r, uint64_t n_r, 
         if (n_s) text.append(text_s, n_s);
         fgss_sets all;
         memset(&all, 0, sizeof all);
-        try {
+        auto split = [&] {
             tokenize_device(ctx->c, text.data(), text.size(), p, &all);
             fgss_sets* outs[2] = {out_r, out_s};
             uint64_t cnt[2] = {0, 0}, tok[2] = {0, 0};
@@ -747,12 +721,12 @@ fgss_status fgss_tokenize_dual(fgss_ctx* ctx, const char* text_r, uint64_t n_r, 
                 d.max_len = std::max<uint32_t>(d.max_len, (uint32_t)l);
                 ti[sd] += l;
             }
-        } catch (...) {
+        };
+        or_undo(ctx->c, split, [&] {
             fgss_sets_free(&all);
             fgss_sets_free(out_r);
             fgss_sets_free(out_s);
-            throw;
-        }
+        });
         fgss_sets_free(&all);
     });
 }
@@ -794,10 +768,16 @@ fgss_status fgss_rsjoin(fgss_ctx* ctx, const fgss_sets_view* r, const fgss_sets_
             J.n_res = n_res;
         }
         rs_output(c, J, u);
-        export_pairs(c, J, *opts, out);
-        Times t;
-        add_times(c, t);
-        report_stats(c, v, stats, launch_counter() - launches0, 1, t);
+        memset(out, 0, sizeof *out);
+        or_undo(
+            c,
+            [&] {
+                export_pairs(c, J, *opts, out);
+                Times t;
+                add_times(c, t);
+                report_stats(c, v, stats, launch_counter() - launches0, 1, t);
+            },
+            [&] { fgss_pairs_free(out); });
     });
 }
 
