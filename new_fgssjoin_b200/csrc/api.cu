@@ -657,6 +657,7 @@ void fgss_sets_free(fgss_sets* s) {
 fgss_status fgss_tokenize(fgss_ctx* ctx, const char* text, uint64_t n_bytes, const fgss_tok_opts* opts,
                           fgss_sets* out) {
     if (!ctx || !out || (!text && n_bytes)) return FGSS_ERR_INVALID;
+    memset(out, 0, sizeof *out);
     return guard(ctx, [&] {
         fgss_tok_opts o;
         fgss_tok_opts_default(&o);
