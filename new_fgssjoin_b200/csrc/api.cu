@@ -159,6 +159,7 @@ void add_times(Ctx& c, Times& t) {
     cudaEvent_t* ev = c.ev;
     FGSS_CK(cudaEventRecord(ev[3], c.stream));
     FGSS_CK(cudaEventSynchronize(ev[3]));
+    c.check_waits();
     float a = 0, b = 0, d = 0, e = 0;
     FGSS_CK(cudaEventElapsedTime(&a, ev[0], ev[1]));
     FGSS_CK(cudaEventElapsedTime(&b, ev[1], ev[2]));

@@ -106,12 +106,24 @@ struct Ctx {
     T* pinnedT(const std::string& name, size_t count) {
         return static_cast<T*>(pinned(name, count * sizeof(T)));
     }
-    void sync() { FGSS_CK(cudaStreamSynchronize(stream)); }
+    void sync() {
+        FGSS_CK(cudaStreamSynchronize(stream));
+        check_waits();
+    }
     // Error word the kernels' bounded waits set (mapped page-locked memory, so
     // reading it after a wait costs no copy); made with the context.
     uint32_t* err_host = nullptr;
     uint32_t* err_dev = nullptr;
     uint32_t* dev_err() const { return err_dev; }
+    // Throws when a device wait gave up: what the stream's kernels left is not to
+    // be read.  To be called after every wait of the host for them.
+    void check_waits() const {
+        if (err_host && *(volatile uint32_t*)err_host) fail(FGSS_ERR_TIMEOUT, "a device wait of a scan or sort gave up");
+    }
+    // After a failed call, nothing in flight.
+    void clear_waits() {
+        if (err_host) *(volatile uint32_t*)err_host = 0;
+    }
     // Frees every pooled device buffer whose name starts with `prefix`.
     void release_prefix(const std::string& prefix) {
         for (auto it = bufs.begin(); it != bufs.end();) {

@@ -32,31 +32,35 @@ void or_undo(Ctx& c, F&& f, U&& undo) {
     }
 }
 
-// Runs f and returns its status.
+// Runs f and returns its status.  A wait of a scan or sort that gave up is looked
+// at wherever the call waits for the stream (Ctx::sync), before anything read back
+// is used, and here once more; every failed call, whatever its reason, leaves the
+// words clear for the next one.
 template <typename F>
 fgss_status guard(fgss_ctx* ctx, F&& f) {
+    fgss_status st = FGSS_ERR_CUDA;
+    std::string msg;
     try {
         f();
-        if (ctx && ctx->c.err_host && *(volatile uint32_t*)ctx->c.err_host) {
-            *ctx->c.err_host = 0;
-            fail(FGSS_ERR_TIMEOUT, "a device wait of a scan or sort gave up");
-        }
+        if (ctx) ctx->c.check_waits();
         if (ctx) ctx->c.last_error.clear();
         return FGSS_OK;
     } catch (const Error& e) {
-        if (ctx) settle(ctx->c);
-        if (ctx) ctx->c.last_error = e.msg;
+        st = e.st;
+        msg = e.msg;
         set_thread_error(e.msg);
-        return e.st;
     } catch (const std::bad_alloc&) {
-        if (ctx) settle(ctx->c);
-        if (ctx) ctx->c.last_error = "host allocation failed";
-        return FGSS_ERR_NOMEM;
+        st = FGSS_ERR_NOMEM;
+        msg = "host allocation failed";
     } catch (...) {
-        if (ctx) settle(ctx->c);
-        if (ctx) ctx->c.last_error = "unknown error";
-        return FGSS_ERR_CUDA;
+        msg = "unknown error";
     }
+    if (ctx) {
+        settle(ctx->c);
+        ctx->c.clear_waits();
+        ctx->c.last_error = msg;
+    }
+    return st;
 }
 
 }  // namespace fgss

@@ -8,6 +8,7 @@
 #include <memory>
 #include <vector>
 
+#include "guard.h"
 #include "join.h"
 #include "model.h"
 #include "prims.cuh"
@@ -43,7 +44,7 @@ extern "C" {
 fgss_status fgss_model_train(fgss_ctx* ctx, const fgss_sets_view* sets, const float* thresholds, int n, int epochs,
                              float lr, uint64_t seed, float* final_loss) {
     if (!ctx || !sets || !thresholds || n <= 0 || epochs <= 0) return FGSS_ERR_INVALID;
-    try {
+    return guard(ctx, [&] {
         Ctx& c = ctx->c;
         FGSS_CK(cudaSetDevice(c.device));
         uint64_t total = 0;
@@ -99,13 +100,7 @@ fgss_status fgss_model_train(fgss_ctx* ctx, const fgss_sets_view* sets, const fl
         FGSS_CK(cudaMemcpyAsync(c.model->dev, c.model->host.data(), kParamsAll * 4, cudaMemcpyHostToDevice, c.stream));
         c.sync();
         if (final_loss) *final_loss = loss;
-        c.last_error.clear();
-        return FGSS_OK;
-    } catch (const Error& e) {
-        if (cudaStreamSynchronize(ctx->c.stream) != cudaSuccess) (void)cudaGetLastError();  // copies from the caller's arrays
-        ctx->c.last_error = e.msg;
-        return e.st;
-    }
+    });
 }
 
 int fgss_model_num_params(void) { return kParams; }

@@ -887,6 +887,7 @@ void tokenize_terms(Ctx& c, const unsigned char* dtext, const uint32_t* lstart, 
         FGSS_CK(cudaEventRecord(c.copy_ev[i], c.stream));
     }
     FGSS_CK(cudaEventSynchronize(c.copy_ev[kParts]));
+    c.check_waits();  // before the parts' bounds are used
     hcut[0] = 0;
     hcut[kParts] = T;
     cudaStream_t cs = c.copy_stream;

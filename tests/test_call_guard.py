@@ -54,3 +54,36 @@ int main() {
         assert st == status
         assert events[:4] == ["copy", "sync-main", "sync-copy", "free"], line
     assert out[3].split() == ["0", "copy"]
+
+
+def test_a_wait_that_gave_up_fails_its_call_only(tmp_path):
+    """The word that a device wait sets stops the call at its next wait, before anything read back is
+    used, and is clear for the next call whatever the failed one ended with."""
+    out = fake_util.run(tmp_path, FAKES + r"""
+int main() {
+    uint32_t word = 0;
+    ctx.c.stream = (cudaStream_t)1;
+    ctx.c.err_host = &word;
+    auto good = [&] { return (int)guard(&ctx, [&] { ctx.c.sync(); }); };
+    int used = 0;
+    int st = guard(&ctx, [&] { word = 1; ctx.c.sync(); used = 1; });
+    printf("at a wait %d used %d word %u next %d\n", st, used, word, good());
+    st = guard(&ctx, [&] { word = 1; });
+    printf("at the end %d word %u next %d\n", st, word, good());
+    st = guard(&ctx, [&] { word = 1; fail(FGSS_ERR_NOMEM, "other"); });
+    printf("other reason %d word %u next %d\n", st, word, good());
+    st = guard(&ctx, [&] { word = 1; throw std::bad_alloc(); });
+    printf("host memory %d word %u next %d\n", st, word, good());
+    printf("message '%s'\n", ctx.c.last_error.c_str());
+}
+""")
+    assert out.splitlines() == ["at a wait 7 used 0 word 0 next 0", "at the end 7 word 0 next 0",
+                                "other reason 3 word 0 next 0", "host memory 3 word 0 next 0", "message ''"]
+
+
+def test_training_runs_under_the_guard():
+    """fgss_model_train joins on the device like the joins' own entry points."""
+    import os
+    src = open(os.path.join(fake_util.CSRC, "model_api.cu")).read()
+    body = src[src.index("fgss_status fgss_model_train("):src.index("int fgss_model_num_params")]
+    assert "return guard(ctx," in body
