@@ -347,6 +347,14 @@ fgss_status fgss_overlap_table(float threshold, int bounds, uint32_t max_sum, ui
  * Replaces exclusive_scan<unsigned int> (include/fgssjoin/scan.cuh:39-105). */
 fgss_status fgss_dev_exclusive_scan_u32(fgss_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n);
 
+/* The same with the caller's limit on the polls of one wait between the scan's
+ * tiles of 4,096 elements (every scan and sort of the library has one of about
+ * a second).  A wait that reaches it gives up: FGSS_ERR_TIMEOUT, out then
+ * incomplete, the context usable.  With 0 every scan of more than one tile
+ * does. */
+fgss_status fgss_dev_exclusive_scan_u32_polls(fgss_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n,
+                                              uint32_t polls);
+
 /* Exclusive prefix sum of n uint32 values that allocates no device memory,
  * for callers that cannot call cudaMalloc: a host that pre-allocates all
  * device memory up front and forbids later allocations, or a latency-critical

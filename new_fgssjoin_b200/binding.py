@@ -22,7 +22,8 @@ EXPORTED_SYMBOLS = [
     "fgss_join_opts_default", "fgss_selfjoin", "fgss_selfjoin_batch", "fgss_rsjoin", "fgss_pairs_free",
     "fgss_pairs_print", "fgss_selfjoin_to_file",
     "fgss_model_train", "fgss_model_save", "fgss_model_load", "fgss_model_grad", "fgss_model_num_params",
-    "fgss_autotune", "fgss_bounds_table", "fgss_overlap_table", "fgss_query_costs", "fgss_dev_exclusive_scan_u32", "fgss_dev_sort_pairs_u64",
+    "fgss_autotune", "fgss_bounds_table", "fgss_overlap_table", "fgss_query_costs", "fgss_dev_exclusive_scan_u32",
+    "fgss_dev_exclusive_scan_u32_polls", "fgss_dev_sort_pairs_u64",
     "fgss_dev_exclusive_scan_u32_noalloc",
 ]
 
@@ -130,6 +131,7 @@ def load_library():
     L.fgss_model_grad.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p,
                                   ctypes.c_void_p, P(ctypes.c_float)]
     L.fgss_dev_exclusive_scan_u32.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64]
+    L.fgss_dev_exclusive_scan_u32_polls.argtypes = L.fgss_dev_exclusive_scan_u32.argtypes + [ctypes.c_uint32]
     L.fgss_dev_sort_pairs_u64.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64,
                                           ctypes.c_int, ctypes.c_int]
     L.fgss_dev_exclusive_scan_u32_noalloc.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64,
@@ -518,6 +520,10 @@ class Context:
     # ---------------------------------------------------- device primitives
     def dev_exclusive_scan_u32(self, d_in, d_out, n):
         _check(self._L, self._ctx, self._L.fgss_dev_exclusive_scan_u32(self._ctx, d_in, d_out, n))
+
+    def dev_exclusive_scan_u32_polls(self, d_in, d_out, n, polls):
+        """The scan with a limit on the polls of a wait between its tiles (FGSS_ERR_TIMEOUT beyond it)."""
+        _check(self._L, self._ctx, self._L.fgss_dev_exclusive_scan_u32_polls(self._ctx, d_in, d_out, n, polls))
 
     def dev_sort_pairs_u64(self, d_keys, d_vals, n, begin_bit=0, end_bit=64):
         _check(self._L, self._ctx, self._L.fgss_dev_sort_pairs_u64(self._ctx, d_keys, d_vals, n, begin_bit, end_bit))

@@ -590,7 +590,9 @@ fgss_status fgss_create(fgss_ctx** out, const fgss_options* opt) {
         for (auto& e : c.ev) FGSS_CK(cudaEventCreate(&e));
         FGSS_CK(cudaHostAlloc((void**)&c.err_host, 4, cudaHostAllocMapped));
         *c.err_host = 0;
-        FGSS_CK(cudaHostGetDevicePointer((void**)&c.err_dev, c.err_host, 0));
+        FGSS_CK(cudaHostGetDevicePointer((void**)&c.err_map, c.err_host, 0));
+        FGSS_CK(cudaMalloc(&c.err_dev, 4));
+        FGSS_CK(cudaMemsetAsync(c.err_dev, 0, 4, c.stream));
         tune_load(c);
         c.graphs = new GraphCache();
     });
@@ -618,6 +620,7 @@ void fgss_destroy(fgss_ctx* ctx) {
     for (auto& e : c.ev)
         if (e) cudaEventDestroy(e);
     if (c.err_host) cudaFreeHost(c.err_host);
+    if (c.err_dev) cudaFree(c.err_dev);
     for (auto& e : c.copy_ev)
         if (e) cudaEventDestroy(e);
     if (c.copy_stream) cudaStreamDestroy(c.copy_stream);
@@ -1104,6 +1107,16 @@ fgss_status fgss_dev_exclusive_scan_u32(fgss_ctx* ctx, const uint32_t* in, uint3
     return guard(ctx, [&] {
         FGSS_CK(cudaSetDevice(ctx->c.device));
         if (n) exclusive_scan<uint32_t>(ctx->c, in, out, n, nullptr, (uint32_t*)nullptr, "api.scan");
+        ctx->c.sync();
+    });
+}
+
+fgss_status fgss_dev_exclusive_scan_u32_polls(fgss_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n,
+                                              uint32_t polls) {
+    if (!ctx || (n && (!in || !out))) return FGSS_ERR_INVALID;
+    return guard(ctx, [&] {
+        FGSS_CK(cudaSetDevice(ctx->c.device));
+        if (n) exclusive_scan<uint32_t>(ctx->c, in, out, n, nullptr, (uint32_t*)nullptr, "api.scan", polls);
         ctx->c.sync();
     });
 }

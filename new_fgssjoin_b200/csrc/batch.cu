@@ -26,10 +26,12 @@ __global__ void k_features(JoinArgs a, float* __restrict__ feat) {
         features_record(a, q, feat + (uint64_t)q * kFeatures);
 }
 
+// (By an order that a sort gave up on, the items stay as they are.)
 __global__ void k_permute_items(const uint4* __restrict__ items, const uint32_t* __restrict__ order, uint64_t n,
-                                uint4* __restrict__ out) {
+                                uint4* __restrict__ out, const uint32_t* __restrict__ err) {
+    const bool as_is = gave_up(err);
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = items[order[i]];
+        out[i] = items[as_is ? i : order[i]];
 }
 
 template <int NT, int HLOG, int RT>
@@ -248,7 +250,7 @@ void index_sort(Ctx& c, Batch& B, uint64_t E_cap, int tbits, int jbits, const ui
     FGSS_LAUNCH_CK();
     radix_sort<K, uint64_t>(c, key, val, E_cap, d_E, 0, tbits + jbits, (p + "b.ixsort").c_str());
     k_index_lists_mj<K><<<grid_for(E_cap, 256, c.num_sms * 32), 256, 0, c.stream>>>(
-        B.d_args, key, val, d_E, (uint32_t)tbits, d_loff, list, d_toff, tab, ent);
+        B.d_args, key, val, d_E, (uint32_t)tbits, d_loff, list, d_toff, tab, ent, c.err_dev);
     FGSS_LAUNCH_CK();
 }
 
@@ -330,7 +332,7 @@ uint4* batch_items(Ctx& c, Batch& B, const Prepass& pp, int cls, const std::vect
         // longest-processing-time order: sort items by descending cost
         uint4* sorted = c.devT<uint4>(p + "items2", nitems + 1);
         radix_sort<uint32_t, uint32_t>(c, ikey, ival, nitems, nullptr, 0, 16, (p + "sort").c_str());
-        k_permute_items<<<grid_for(nitems, 128), 128, 0, c.stream>>>(items, ival, nitems, sorted);
+        k_permute_items<<<grid_for(nitems, 128), 128, 0, c.stream>>>(items, ival, nitems, sorted, c.err_dev);
         FGSS_LAUNCH_CK();
         items = sorted;
     }
@@ -799,7 +801,7 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     FGSS_LAUNCH_CK();
     radix_sort<uint64_t, uint32_t>(c, key, val, oc, d_n, 0, 2 * qb + jb, (p + "b.rsort").c_str());
     k_result_out_mj<<<grid_for(oc, 256, c.num_sms * 32), 256, 0, c.stream>>>(
-        B.d_args, key, val, d_n, resoff, rt.roff, (uint32_t)qb, B.oq, B.os, B.oidq, B.oids, B.oo, B.osim);
+        B.d_args, key, val, d_n, resoff, rt.roff, (uint32_t)qb, B.oq, B.os, B.oidq, B.oids, B.oo, B.osim, c.err_dev);
     FGSS_LAUNCH_CK();
 }
 
@@ -933,8 +935,8 @@ void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
     uint64_t* keys = c.devT<uint64_t>(J.pfx("rkey"), R + 1);
     uint32_t* vals = c.devT<uint32_t>(J.pfx("rval"), R + 1);
     if (R) {
-        k_result_fill<<<grid_for(C, 256, c.num_sms * 32), 256, 0, c.stream>>>(cand, ov, flag, off, d_nc,
-                                                                              (uint32_t)bits_for(n), keys, vals);
+        k_result_fill<<<grid_for(C, 256, c.num_sms * 32), 256, 0, c.stream>>>(
+            cand, ov, flag, off, d_nc, (uint32_t)bits_for(n), keys, vals, c.err_dev);
         FGSS_LAUNCH_CK();
     }
     join_output(c, J, keys, vals, J.d_nres, R);

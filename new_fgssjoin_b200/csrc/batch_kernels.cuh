@@ -87,7 +87,9 @@ __global__ void k_index_lists_mj(const JoinArgs* __restrict__ joins, const K* __
                                         const uint64_t* __restrict__ val, const uint64_t* __restrict__ d_e,
                                         uint32_t tbits, const uint64_t* __restrict__ loff,
                                         uint32_t* __restrict__ list_all, const uint64_t* __restrict__ toff,
-                                        uint32_t* __restrict__ tab_all, uint2* __restrict__ ent) {
+                                        uint32_t* __restrict__ tab_all, uint2* __restrict__ ent,
+                                        const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;  // (the cleared offsets stay: every list is empty)
     const uint64_t E = *d_e;
     const uint64_t tmask = (1ull << tbits) - 1;
     for (uint64_t k0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; k0 < E;
@@ -407,7 +409,9 @@ static __global__ void k_result_out_mj(const JoinArgs* __restrict__ joins, const
                                        const uint64_t* __restrict__ resoff, const uint64_t* __restrict__ capoff,
                                        uint32_t qb, uint32_t* __restrict__ oq, uint32_t* __restrict__ os,
                                        uint32_t* __restrict__ oidq, uint32_t* __restrict__ oids,
-                                       uint32_t* __restrict__ oo, float* __restrict__ osim) {
+                                       uint32_t* __restrict__ oo, float* __restrict__ osim,
+                                       const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     const uint64_t n = *d_n;
     const uint64_t qmask = (1ull << qb) - 1;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {

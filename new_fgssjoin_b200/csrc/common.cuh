@@ -39,6 +39,20 @@ inline unsigned long long& launch_counter() {
         FGSS_CK(cudaGetLastError());     \
     } while (0)
 
+// How a kernel's bounded wait reports that it gave up (Ctx::waits).  What such a
+// kernel leaves is not finished: a kernel that uses it as positions or sizes first
+// looks at *word and writes nothing where it is set (gave_up), until the host, which
+// looks at its own word after every wait, ends the call.
+struct WaitErr {
+    static constexpr uint32_t kPolls = 1u << 21;  // of one status word: a second or so
+    uint32_t* word;
+    uint32_t* host;
+    uint32_t polls;
+};
+// The same in every thread of a kernel that does not wait itself: the word is set
+// by earlier kernels of the stream.
+__device__ __forceinline__ bool gave_up(const uint32_t* word) { return *word != 0; }
+
 constexpr int kWarp = 32;
 constexpr uint32_t kFull = 0xffffffffu;
 

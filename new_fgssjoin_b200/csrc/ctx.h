@@ -110,11 +110,14 @@ struct Ctx {
         FGSS_CK(cudaStreamSynchronize(stream));
         check_waits();
     }
-    // Error word the kernels' bounded waits set (mapped page-locked memory, so
-    // reading it after a wait costs no copy); made with the context.
+    // The words that a kernel's bounded wait sets when it gives up, made with the
+    // context: one in mapped page-locked memory (err_host, at err_map for kernels), which
+    // the host reads without a copy, and one in device memory (err_dev), which the
+    // kernels that follow look at first (WaitErr::word).
     uint32_t* err_host = nullptr;
+    uint32_t* err_map = nullptr;
     uint32_t* err_dev = nullptr;
-    uint32_t* dev_err() const { return err_dev; }
+    WaitErr waits(uint32_t polls = WaitErr::kPolls) const { return {err_dev, err_map, polls}; }
     // Throws when a device wait gave up: what the stream's kernels left is not to
     // be read.  To be called after every wait of the host for them.
     void check_waits() const {
@@ -122,7 +125,11 @@ struct Ctx {
     }
     // After a failed call, nothing in flight.
     void clear_waits() {
-        if (err_host) *(volatile uint32_t*)err_host = 0;
+        if (!err_host || !*(volatile uint32_t*)err_host) return;
+        *(volatile uint32_t*)err_host = 0;
+        if (!err_dev) return;
+        if (cudaMemsetAsync(err_dev, 0, 4, stream) != cudaSuccess) (void)cudaGetLastError();
+        if (cudaStreamSynchronize(stream) != cudaSuccess) (void)cudaGetLastError();
     }
     // Frees every pooled device buffer whose name starts with `prefix`.
     void release_prefix(const std::string& prefix) {

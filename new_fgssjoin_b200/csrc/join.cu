@@ -191,7 +191,7 @@ void join_output(Ctx& c, JoinState& J, uint64_t* keys, uint32_t* vals, const uin
     const int qb = bits_for(n);  // keys are q << qb | s
     radix_sort<uint64_t, uint32_t>(c, keys, vals, n_cap, d_n, 0, 2 * qb, J.pfx("rsort").c_str());
     k_result_out<<<grid_for(n_cap, 256, c.num_sms * 32), 256, 0, c.stream>>>(
-        keys, vals, d_n, (uint32_t)qb, J.id, J.in.len, J.oq, J.os, J.oidq, J.oids, J.oo, J.osim);
+        keys, vals, d_n, (uint32_t)qb, J.id, J.in.len, J.oq, J.os, J.oidq, J.oids, J.oo, J.osim, c.err_dev);
     FGSS_LAUNCH_CK();
 }
 

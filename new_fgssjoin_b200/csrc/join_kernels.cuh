@@ -896,7 +896,8 @@ static __global__ void k_result_flags(JoinArgs a, const uint4* __restrict__ cand
 static __global__ void k_result_fill(const uint4* __restrict__ cand, const uint32_t* __restrict__ ov,
                               const uint32_t* __restrict__ flag, const uint32_t* __restrict__ off,
                               const uint64_t* __restrict__ d_nc, uint32_t qb, uint64_t* __restrict__ key,
-                              uint32_t* __restrict__ val) {
+                              uint32_t* __restrict__ val, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     const uint32_t nc = (uint32_t)*d_nc;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
         if (flag[i]) {
@@ -913,7 +914,8 @@ static __global__ void k_result_out(const uint64_t* __restrict__ key, const uint
                              const uint64_t* __restrict__ d_n, uint32_t qb, const uint32_t* __restrict__ id,
                              const uint32_t* __restrict__ len, uint32_t* __restrict__ oq, uint32_t* __restrict__ os,
                              uint32_t* __restrict__ oidq, uint32_t* __restrict__ oids, uint32_t* __restrict__ oo,
-                             float* __restrict__ osim) {
+                             float* __restrict__ osim, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     const uint64_t n = *d_n;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t k = key[i];

@@ -93,26 +93,31 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_add(T* out, const T* __re
 // Status word of a tile (or of a tile's digit): 0 = nothing yet, else the sum of
 // the tile alone (kLbSum) or of everything up to it (kLbAll).
 constexpr uint64_t kLbSum = 1ull << 62, kLbAll = 2ull << 62, kLbValue = (1ull << 62) - 1;
-constexpr uint32_t kLbPolls = 1u << 21;  // polls of one word (a second or so) before a tile gives up
 
-// Waits for the status word *p; 0 when it gave up (or another tile did): the
-// caller then returns without writing anything, *abort and *err (host memory,
-// Ctx::dev_err) are set, and the call fails with FGSS_ERR_TIMEOUT.
-__device__ __forceinline__ uint64_t lb_wait(const volatile uint64_t* p, volatile uint64_t* abort, volatile uint32_t* err) {
-    for (uint32_t i = 0; i < kLbPolls; i++) {
+// A tile gives up: the others of its kernel stop waiting (*abort), the kernels that
+// follow write nothing by what it leaves and the call fails with FGSS_ERR_TIMEOUT.
+__device__ __forceinline__ void lb_give_up(volatile uint64_t* abort, const WaitErr& err) {
+    *abort = 1;
+    *(volatile uint32_t*)err.word = 1;
+    *(volatile uint32_t*)err.host = 1;
+}
+
+// Waits for the status word *p, err.polls times at most; 0 when it gave up (or
+// another tile did): the caller then returns without writing anything.
+__device__ __forceinline__ uint64_t lb_wait(const volatile uint64_t* p, volatile uint64_t* abort, const WaitErr& err) {
+    for (uint32_t i = 0; i < err.polls; i++) {
         const uint64_t v = *p;
         if (v) return v;
         if ((i & 255u) == 255u && *abort) return 0;
     }
-    *abort = 1;
-    *err = 1;
+    lb_give_up(abort, err);
     return 0;
 }
 
 // state: u64 [0] tile counter, [1] abort, [2 ..] tile statuses; zero at launch.
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) k_scan_pass(const T* in, T* out, uint64_t n_cap, const uint64_t* d_n,
-                                                             uint64_t* state, T* grand_total, uint32_t* err) {
+                                                             uint64_t* state, T* grand_total, WaitErr err) {
     __shared__ T wsum[33];
     __shared__ uint64_t s_tile, s_pre;
     __shared__ bool s_stop;
@@ -192,16 +197,17 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_pass(const T* in, T* out,
 
 // Exclusive scan of n_cap (or *d_n) elements (out may alias in); optional grand
 // total to `total` (device).  Sums below 2^62 (of 32-bit elements: any, modulo 2^32).
+// polls: see WaitErr.
 template <typename T>
 void exclusive_scan(Ctx& c, const T* in, T* out, uint64_t n_cap, const uint64_t* d_n, T* total,
-                    const char* tag = "scan") {
+                    const char* tag = "scan", uint32_t polls = WaitErr::kPolls) {
     const uint64_t ntiles = n_cap == 0 ? 1 : (n_cap + kScanTile - 1) / kScanTile;
     uint64_t* state = nullptr;
     if (ntiles > 1) {
         state = c.devT<uint64_t>(std::string(tag) + ".lb", ntiles + 2);
         FGSS_CK(cudaMemsetAsync(state, 0, (ntiles + 2) * 8, c.stream));
     }
-    k_scan_pass<T><<<(unsigned)ntiles, kScanThreads, 0, c.stream>>>(in, out, n_cap, d_n, state, total, c.dev_err());
+    k_scan_pass<T><<<(unsigned)ntiles, kScanThreads, 0, c.stream>>>(in, out, n_cap, d_n, state, total, c.waits(polls));
     FGSS_LAUNCH_CK();
 }
 
@@ -330,7 +336,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_sort_pass(const K* __restri
                                                             const unsigned long long* __restrict__ hist,
                                                             const uint32_t* __restrict__ offs, uint64_t n_cap,
                                                             const uint64_t* d_n, int shift, uint64_t* state,
-                                                            uint32_t* err) {
+                                                            WaitErr err) {
     constexpr size_t kElem = sizeof(K) > sizeof(V) ? sizeof(K) : sizeof(V);
     extern __shared__ __align__(16) unsigned char s_buf[];  // kSortTile x kElem
     (void)kElem;
@@ -339,10 +345,13 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_sort_pass(const K* __restri
     __shared__ unsigned long long s_wsum[33];
     __shared__ uint64_t s_tile;
     const uint64_t n = d_n ? min(*d_n, n_cap) : n_cap;
+    // Nothing is written by counts or positions of a scan, or of this sort's earlier passes, that
+    // gave up.  (One thread looks where tiles of this kernel may give up: the same for its block.)
     if (LOOK) {
-        if (threadIdx.x == 0) s_tile = atomicAdd((unsigned long long*)state, 1ull);
+        if (threadIdx.x == 0) s_tile = gave_up(err.word) ? ~0ull : atomicAdd((unsigned long long*)state, 1ull);
         __syncthreads();
     }
+    if (LOOK ? s_tile == ~0ull : gave_up(err.word)) return;
     const uint64_t tile = LOOK ? s_tile : blockIdx.x, base = tile * kSortTile;
     if (base >= n) return;
     const uint32_t n_tile = (uint32_t)min((uint64_t)kSortTile, n - base);
@@ -385,10 +394,9 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_sort_pass(const K* __restri
                 t -= got;
                 if (got == 0) {
                     polls++;
-                    if (polls > kLbPolls || ((polls & 255u) == 0 && *(volatile uint64_t*)(state + 1))) {
+                    if (polls > err.polls || ((polls & 255u) == 0 && *(volatile uint64_t*)(state + 1))) {
                         stop = true;
-                        *(volatile uint64_t*)(state + 1) = 1;
-                        *(volatile uint32_t*)err = 1;
+                        lb_give_up(state + 1, err);
                         break;
                     }
                 }
@@ -511,7 +519,7 @@ void radix_sort(Ctx& c, K* keys, V* values, uint64_t n_cap, const uint64_t* d_n,
         for (int p = 0; p < passes; p++) {
             k_sort_pass<K, V, true><<<ntiles, kSortThreads, smem, c.stream>>>(
                 ka, kb, va, vb, hist + 256 * p, nullptr, n_cap, d_n, begin_bit + 8 * p, work + passes * 256 + p * per,
-                c.dev_err());
+                c.waits());
             FGSS_LAUNCH_CK();
             std::swap(ka, kb);
             std::swap(va, vb);
@@ -523,7 +531,7 @@ void radix_sort(Ctx& c, K* keys, V* values, uint64_t n_cap, const uint64_t* d_n,
             FGSS_LAUNCH_CK();
             exclusive_scan<uint32_t>(c, cnt, cnt, 256ull * ntiles, nullptr, (uint32_t*)nullptr, (t + ".hs").c_str());
             k_sort_pass<K, V, false><<<ntiles, kSortThreads, smem, c.stream>>>(
-                ka, kb, va, vb, nullptr, cnt, n_cap, d_n, begin_bit + 8 * p, nullptr, nullptr);
+                ka, kb, va, vb, nullptr, cnt, n_cap, d_n, begin_bit + 8 * p, nullptr, c.waits());
             FGSS_LAUNCH_CK();
             std::swap(ka, kb);
             std::swap(va, vb);

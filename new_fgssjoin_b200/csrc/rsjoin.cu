@@ -46,7 +46,8 @@ __global__ void k_rs_union(const uint64_t* __restrict__ key, uint32_t n, const u
                            const uint32_t* __restrict__ rlen, uint64_t tr, const uint32_t* __restrict__ spos,
                            const uint32_t* __restrict__ slen, uint64_t ts, uint32_t* __restrict__ upos,
                            uint32_t* __restrict__ ulen, uint8_t* __restrict__ side, uint32_t* __restrict__ orig,
-                           uint32_t* __restrict__ bad) {
+                           uint32_t* __restrict__ bad, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint64_t x = key[k];
         const uint32_t sd = (uint32_t)(x >> 31) & 1u, idx = (uint32_t)x & 0x7fffffffu;
@@ -78,7 +79,8 @@ __global__ void k_rs_out(const uint64_t* __restrict__ key, const uint32_t* __res
                          const uint32_t* __restrict__ rid, const uint32_t* __restrict__ sid,
                          const uint32_t* __restrict__ oo, const float* __restrict__ osim, uint32_t* __restrict__ q,
                          uint32_t* __restrict__ s, uint32_t* __restrict__ idq, uint32_t* __restrict__ ids,
-                         uint32_t* __restrict__ o, float* __restrict__ sim) {
+                         uint32_t* __restrict__ o, float* __restrict__ sim, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t k = key[i];
         const uint32_t r = (uint32_t)(k >> sb), x = (uint32_t)(k & ((1ull << sb) - 1)), v = val[i];
@@ -132,7 +134,8 @@ RsInput rs_union(Ctx& c, const fgss_sets_view& r_in, const fgss_sets_view& s_in)
         FGSS_LAUNCH_CK();
         radix_sort<uint64_t, uint32_t>(c, key, nullptr, n, nullptr, 32, 48, "rs.u.sort");
         k_rs_union<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(
-            key, (uint32_t)n, r.pos, r.len, r.n_tokens, s.pos, s.len, s.n_tokens, upos, ulen, u.side, u.orig, bad);
+            key, (uint32_t)n, r.pos, r.len, r.n_tokens, s.pos, s.len, s.n_tokens, upos, ulen, u.side, u.orig, bad,
+            c.err_dev);
         FGSS_LAUNCH_CK();
         uint32_t* h = c.pinnedT<uint32_t>("rs.h.bad", 1);
         FGSS_CK(cudaMemcpyAsync(h, bad, 4, cudaMemcpyDeviceToHost, c.stream));
@@ -165,7 +168,7 @@ void rs_output(Ctx& c, JoinState& J, const RsInput& u) {
         FGSS_LAUNCH_CK();
         radix_sort<uint64_t, uint32_t>(c, key, val, n, nullptr, 0, sb + bits_needed(u.nr), "rs.o.sort");
         k_rs_out<<<grid_for(n, 256, c.num_sms * 16), 256, 0, c.stream>>>(key, val, n, (uint32_t)sb, u.rid, u.sid, J.oo,
-                                                                        J.osim, q, s, idq, ids, o, sim);
+                                                                        J.osim, q, s, idq, ids, o, sim, c.err_dev);
         FGSS_LAUNCH_CK();
     }
     J.out_col = col;

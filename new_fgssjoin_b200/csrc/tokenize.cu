@@ -215,7 +215,8 @@ __global__ void k_compact_tok(const uint64_t* __restrict__ key, const uint64_t* 
 
 // tag (line << 32 | pos) -> global gram index (monotone in (line, pos)) for the first-occurrence order
 __global__ void k_tag_index(const uint64_t* __restrict__ tag, const uint32_t* __restrict__ goff, uint64_t n,
-                            uint32_t* __restrict__ gidx) {
+                            uint32_t* __restrict__ gidx, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t t = tag[i];
         gidx[i] = goff[t >> 32] + (uint32_t)t;
@@ -231,7 +232,8 @@ __global__ void k_run_flags(const uint64_t* __restrict__ key, uint64_t n, uint32
 // Run id of every element (exclusive scan of the run-start flags) and the
 // start index of every run.
 __global__ void k_run_start(const uint32_t* __restrict__ flag, uint32_t* __restrict__ rid, uint64_t n,
-                            uint32_t* __restrict__ rstart) {
+                            uint32_t* __restrict__ rstart, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t r = rid[i] + flag[i] - 1;
         rid[i] = r;
@@ -251,7 +253,9 @@ __global__ void k_run_keys2(const uint32_t* __restrict__ rstart, const uint32_t*
 }
 
 // rank of every run after the (df, first) sort -> term id per run
-__global__ void k_run_ids(const uint32_t* __restrict__ rval_sorted, uint32_t nruns, uint32_t* __restrict__ id_of_run) {
+__global__ void k_run_ids(const uint32_t* __restrict__ rval_sorted, uint32_t nruns, uint32_t* __restrict__ id_of_run,
+                          const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nruns; k += gridDim.x * blockDim.x)
         id_of_run[rval_sorted[k]] = k;
 }
@@ -269,7 +273,8 @@ __global__ void k_line_id_keys(const uint32_t* __restrict__ rid, const uint32_t*
 
 // tokens per line (sorted by line): sizes via run boundaries
 __global__ void k_line_bounds2(const uint64_t* __restrict__ k2, uint64_t n, uint32_t* __restrict__ lend,
-                               uint32_t* __restrict__ loff) {
+                               uint32_t* __restrict__ loff, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t l = (uint32_t)(k2[i] >> 32);
         if (i == 0 || (uint32_t)(k2[i - 1] >> 32) != l) loff[l] = (uint32_t)i;
@@ -296,7 +301,8 @@ __global__ void k_rec_keys(const uint32_t* __restrict__ lsz, uint32_t nlines, ui
 // (empty records sort first in file order and are cut off at the end)
 __global__ void k_rec_out(const uint32_t* __restrict__ rv_sorted, const uint32_t* __restrict__ lsz, uint32_t nlines,
                           uint32_t nempty, uint32_t* __restrict__ mline, uint32_t* __restrict__ mid,
-                          uint32_t* __restrict__ mlen) {
+                          uint32_t* __restrict__ mlen, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     const uint32_t nrec = nlines - nempty;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nrec; i += gridDim.x * blockDim.x) {
         uint32_t l = rv_sorted[nlines - 1 - i];
@@ -309,7 +315,9 @@ __global__ void k_rec_out(const uint32_t* __restrict__ rv_sorted, const uint32_t
 __global__ void k_gather_rec(const uint32_t* __restrict__ mline, const uint32_t* __restrict__ moff, uint32_t nrec,
                              const uint32_t* __restrict__ loff, const uint32_t* __restrict__ lsz,
                              const uint64_t* __restrict__ k2, const uint32_t* __restrict__ pos,
-                             uint32_t* __restrict__ otok, uint32_t* __restrict__ oloc) {
+                             uint32_t* __restrict__ otok, uint32_t* __restrict__ oloc,
+                             const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nrec; i += warps) {
         uint32_t l = mline[i], src = loff[l], n = lsz[l], dst = moff[i];
@@ -409,8 +417,9 @@ __global__ void __launch_bounds__(256) k_text_count(const unsigned char* __restr
 // Bounds of the non-empty lines (the k-th start belongs to the k-th end).
 __global__ void __launch_bounds__(256) k_text_lines(const unsigned char* __restrict__ text, uint64_t n,
                                                     const uint32_t* __restrict__ tile_off, uint32_t* __restrict__ lstart,
-                                                    uint32_t* __restrict__ lend) {
+                                                    uint32_t* __restrict__ lend, const uint32_t* __restrict__ err) {
     __shared__ uint32_t s_wsum[33];
+    if (gave_up(err)) return;
     const uint64_t base = (uint64_t)blockIdx.x * kTextTile + threadIdx.x * 16;
     uint32_t w[4], starts, ends, total;
     line_flags(text, base, n, w, starts, ends);
@@ -431,7 +440,9 @@ __device__ __forceinline__ uint32_t line_grams(uint32_t len, const TokParams& p)
 // The largest line, and the lists of the lines of more than kSmallLine grams (mid
 // from the front, long ones from the back).
 __global__ void k_line_classes(const uint32_t* __restrict__ lstart, const uint32_t* __restrict__ lend, TokParams p,
-                               TokCounts* cnt, uint32_t* __restrict__ list, uint32_t list_cap) {
+                               TokCounts* cnt, uint32_t* __restrict__ list, uint32_t list_cap,
+                               const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     const uint32_t nl = cnt->n_lines;
     uint32_t mx = 0;
     for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < nl; l += gridDim.x * blockDim.x) {
@@ -631,7 +642,8 @@ __global__ void k_nonzero(const uint32_t* __restrict__ mark, uint32_t n, uint32_
 // Terms in first-occurrence order: their df and run.
 __global__ void k_term_order(const uint32_t* __restrict__ mark, const uint32_t* __restrict__ rank, uint32_t n,
                              const uint32_t* __restrict__ rstart, uint32_t nruns, uint32_t* __restrict__ df,
-                             uint32_t* __restrict__ run) {
+                             uint32_t* __restrict__ run, const uint32_t* __restrict__ err) {
+    if (gave_up(err)) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (mark[i] == 0) continue;
         const uint32_t r = mark[i] - 1, e = r + 1 < nruns ? rstart[r + 1] : n;
@@ -688,8 +700,9 @@ __global__ void k_records(const uint32_t* __restrict__ mline, const uint32_t* __
                           const uint32_t* __restrict__ moff, uint32_t first, uint32_t end, uint32_t lo,
                           uint32_t hi, const uint32_t* __restrict__ loff, const uint32_t* __restrict__ id,
                           const uint32_t* __restrict__ pos, int pb, uint32_t* __restrict__ otok,
-                          uint32_t* __restrict__ oloc) {
+                          uint32_t* __restrict__ oloc, const uint32_t* __restrict__ err) {
     extern __shared__ __align__(16) unsigned char s_rec[];
+    if (gave_up(err)) return;
     const uint32_t nw = WARP ? blockDim.x >> 5 : 1, wid = WARP ? threadIdx.x >> 5 : 0;
     const uint32_t t = WARP ? lane_id() : threadIdx.x, nt = WARP ? 32 : blockDim.x;
     S* v = reinterpret_cast<S*>(s_rec) + (size_t)wid * hi;
@@ -790,7 +803,7 @@ void tokenize_terms(Ctx& c, const unsigned char* dtext, const uint32_t* lstart, 
     k_key_flags<KO><<<gT, 256, 0, c.stream>>>(key, T, flag);
     FGSS_LAUNCH_CK();
     exclusive_scan<uint32_t>(c, flag, rid, T, nullptr, tot, "tl.s.run");
-    k_run_start<<<gT, 256, 0, c.stream>>>(flag, rid, T, rstart);
+    k_run_start<<<gT, 256, 0, c.stream>>>(flag, rid, T, rstart, c.err_dev);
     FGSS_LAUNCH_CK();
     const uint32_t V = read_u32(c, tot);
     // term ids: first-occurrence order, then a stable sort by document frequency
@@ -805,10 +818,10 @@ void tokenize_terms(Ctx& c, const unsigned char* dtext, const uint32_t* lstart, 
     k_nonzero<<<gT, 256, 0, c.stream>>>(mark, T, flag);
     FGSS_LAUNCH_CK();
     exclusive_scan<uint32_t>(c, flag, flag, T, nullptr, (uint32_t*)nullptr, "tl.s.first");
-    k_term_order<<<gT, 256, 0, c.stream>>>(mark, flag, T, rstart, V, df, run);
+    k_term_order<<<gT, 256, 0, c.stream>>>(mark, flag, T, rstart, V, df, run, c.err_dev);
     FGSS_LAUNCH_CK();
     radix_sort<uint32_t, uint32_t>(c, df, run, V, nullptr, 0, bits_for32((uint64_t)nl + 1), "tl.dfsort");
-    k_run_ids<<<gV, 256, 0, c.stream>>>(run, V, id_of_run);
+    k_run_ids<<<gV, 256, 0, c.stream>>>(run, V, id_of_run, c.err_dev);
     FGSS_LAUNCH_CK();
     uint32_t* id = mark;  // (the marks are done with)
     k_token_ids<<<gT, 256, 0, c.stream>>>(rid, id_of_run, num, T, id);
@@ -824,7 +837,7 @@ void tokenize_terms(Ctx& c, const unsigned char* dtext, const uint32_t* lstart, 
     uint32_t* mid = c.devT<uint32_t>("tl.mid", (uint64_t)nrec + 1);
     uint32_t* mlen = c.devT<uint32_t>("tl.mlen", (uint64_t)nrec + 1);
     uint32_t* moff = c.devT<uint32_t>("tl.moff", (uint64_t)nrec + 1);
-    k_rec_out<<<grid_for(nrec, 256), 256, 0, c.stream>>>(rv, lsz, nl, h.n_empty, mline, mid, mlen);
+    k_rec_out<<<grid_for(nrec, 256), 256, 0, c.stream>>>(rv, lsz, nl, h.n_empty, mline, mid, mlen, c.err_dev);
     FGSS_LAUNCH_CK();
     exclusive_scan<uint32_t>(c, mlen, moff, nrec, nullptr, (uint32_t*)nullptr, "tl.s.rec");
     uint32_t* otok = c.devT<uint32_t>("tl.otok", (uint64_t)T + 1);
@@ -833,12 +846,12 @@ void tokenize_terms(Ctx& c, const unsigned char* dtext, const uint32_t* lstart, 
     auto records = [&](auto tag, uint32_t a, uint32_t b) {
         using S = decltype(tag);
         k_records<S, true><<<grid_for(b - a, 8, c.num_sms * 16), 256, 8 * kSmallLine * sizeof(S), c.stream>>>(
-            mline, mlen, moff, a, b, 0, kSmallLine, loff, id, pos, pb, otok, oloc);
+            mline, mlen, moff, a, b, 0, kSmallLine, loff, id, pos, pb, otok, oloc, c.err_dev);
         FGSS_LAUNCH_CK();
         // (sizes descend: the longer ones are among the first)
         if (h.max_size > kSmallLine && a < h.n_mid + h.n_long) {
             k_records<S, false><<<grid_for(h.n_mid + h.n_long - a, 1, c.num_sms * 8), 256, kMidLine * sizeof(S), c.stream>>>(
-                mline, mlen, moff, a, b, kSmallLine, kMidLine, loff, id, pos, pb, otok, oloc);
+                mline, mlen, moff, a, b, kSmallLine, kMidLine, loff, id, pos, pb, otok, oloc, c.err_dev);
             FGSS_LAUNCH_CK();
         }
         if (h.max_size > kMidLine && a < h.n_long) {
@@ -846,7 +859,7 @@ void tokenize_terms(Ctx& c, const unsigned char* dtext, const uint32_t* lstart, 
             FGSS_CK(cudaFuncSetAttribute(k_records<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(kMaxLineGrams * sizeof(S))));
             k_records<S, false><<<grid_for(h.n_long - a, 1, c.num_sms * 2), 1024, smem, c.stream>>>(
-                mline, mlen, moff, a, b, kMidLine, h.max_size, loff, id, pos, pb, otok, oloc);
+                mline, mlen, moff, a, b, kMidLine, h.max_size, loff, id, pos, pb, otok, oloc, c.err_dev);
             FGSS_LAUNCH_CK();
         }
     };
@@ -922,9 +935,10 @@ bool tokenize_lines(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokPa
     k_text_count<<<ntiles, 256, 0, c.stream>>>(dtext, nb, p.mode == 0 && p.lower, toff, cnt);
     FGSS_LAUNCH_CK();
     exclusive_scan<uint32_t>(c, toff, toff, ntiles, nullptr, &cnt->n_lines, "tl.s.tile");
-    k_text_lines<<<ntiles, 256, 0, c.stream>>>(dtext, nb, toff, lstart, lend);
+    k_text_lines<<<ntiles, 256, 0, c.stream>>>(dtext, nb, toff, lstart, lend, c.err_dev);
     FGSS_LAUNCH_CK();
-    k_line_classes<<<grid_for(lcap, 256, c.num_sms * 8), 256, 0, c.stream>>>(lstart, lend, p, cnt, list, lcap);
+    k_line_classes<<<grid_for(lcap, 256, c.num_sms * 8), 256, 0, c.stream>>>(lstart, lend, p, cnt, list, lcap,
+                                                                                c.err_dev);
     FGSS_LAUNCH_CK();
     FGSS_CK(cudaMemcpyAsync(h, cnt, sizeof(TokCounts), cudaMemcpyDeviceToHost, c.stream));
     c.sync();
@@ -1080,7 +1094,7 @@ void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokP
     const int kb2 = suffix ? kb + 16 : kb;
     radix_sort<uint64_t, uint64_t>(c, tkey, ttag, Tn, nullptr, 0, kb2 > 64 ? 64 : kb2, "tk.sortC");
     uint32_t* gidx = c.devT<uint32_t>("tk.gidx", Tn + 1);
-    k_tag_index<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(ttag, goff, Tn, gidx);
+    k_tag_index<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(ttag, goff, Tn, gidx, c.err_dev);
     FGSS_LAUNCH_CK();
     uint32_t* rflag = c.devT<uint32_t>("tk.rflag", Tn + 1);
     uint32_t* rid = c.devT<uint32_t>("tk.rid", Tn + 1);
@@ -1089,7 +1103,7 @@ void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokP
     exclusive_scan<uint32_t>(c, rflag, rid, Tn, nullptr, tot + 4, "tk.s5");
     const uint32_t V = read_u32(c, tot + 4);
     uint32_t* rstart = c.devT<uint32_t>("tk.rstart", (uint64_t)V + 1);
-    k_run_start<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(rflag, rid, Tn, rstart);
+    k_run_start<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(rflag, rid, Tn, rstart, c.err_dev);
     FGSS_LAUNCH_CK();
     uint64_t* rkey = c.devT<uint64_t>("tk.rkey", (uint64_t)V + 1);
     uint32_t* rval = c.devT<uint32_t>("tk.rval", (uint64_t)V + 1);
@@ -1097,7 +1111,7 @@ void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokP
     FGSS_LAUNCH_CK();
     radix_sort<uint64_t, uint32_t>(c, rkey, rval, V, nullptr, 0, 32 + bits_for32((uint64_t)nlines + 1), "tk.sortD");
     uint32_t* id_of_run = c.devT<uint32_t>("tk.idrun", (uint64_t)V + 1);
-    k_run_ids<<<grid_for(V, 256, c.num_sms * 32), 256, 0, c.stream>>>(rval, V, id_of_run);
+    k_run_ids<<<grid_for(V, 256, c.num_sms * 32), 256, 0, c.stream>>>(rval, V, id_of_run, c.err_dev);
     FGSS_LAUNCH_CK();
     // 5. (line, id) order
     uint64_t* k2 = c.devT<uint64_t>("tk.k2", Tn + 1);
@@ -1112,7 +1126,7 @@ void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokP
     uint32_t* lend = c.devT<uint32_t>("tk.lend", nlines + 1);
     FGSS_CK(cudaMemsetAsync(loff, 0, (uint64_t)nlines * 4, c.stream));
     FGSS_CK(cudaMemsetAsync(lend, 0, (uint64_t)nlines * 4, c.stream));
-    k_line_bounds2<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(k2, Tn, lend, loff);
+    k_line_bounds2<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(k2, Tn, lend, loff, c.err_dev);
     FGSS_LAUNCH_CK();
     k_line_sizes<<<grid_for(nlines, 256, c.num_sms * 8), 256, 0, c.stream>>>(lend, loff, nlines, lsz);
     FGSS_LAUNCH_CK();
@@ -1131,7 +1145,7 @@ void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokP
     uint32_t* mlen = c.devT<uint32_t>("tk.mlen", nrec + 1);
     uint32_t* moff = c.devT<uint32_t>("tk.moff", nrec + 1);
     if (nrec) {
-        k_rec_out<<<grid_for(nrec, 256), 256, 0, c.stream>>>(rv, lsz, nlines, nempty, mline, mid, mlen);
+        k_rec_out<<<grid_for(nrec, 256), 256, 0, c.stream>>>(rv, lsz, nlines, nempty, mline, mid, mlen, c.err_dev);
         FGSS_LAUNCH_CK();
         exclusive_scan<uint32_t>(c, mlen, moff, nrec, nullptr, tot + 6, "tk.s6");
     }
@@ -1139,7 +1153,7 @@ void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokP
     uint32_t* oloc = c.devT<uint32_t>("tk.oloc", Tn + 1);
     if (nrec) {
         k_gather_rec<<<grid_for((uint64_t)nrec * 32, 256, c.num_sms * 32), 256, 0, c.stream>>>(
-            mline, moff, nrec, loff, lsz, k2, pos, otok, oloc);
+            mline, moff, nrec, loff, lsz, k2, pos, otok, oloc, c.err_dev);
         FGSS_LAUNCH_CK();
     }
     copy_out(c, out, nrec, Tn, V, mid, mlen, moff, otok, oloc);
