@@ -15,6 +15,7 @@
 #include <thread>
 #include <vector>
 
+#include "columns.h"
 #include "guard.h"
 #include "join.h"
 #include "model.h"
@@ -102,9 +103,9 @@ void export_pairs(Ctx& c, JoinState& J, const fgss_join_opts& o, fgss_pairs* out
         out->sim = (float*)dup(J.osim, R * 4);
     } else {
         alloc_host_pairs(out, R);
-        if (R && out->priv) {  // both sides are six columns of one block: one copy
+        if (R && out->priv) {  // both sides are six columns of one block
             const size_t col = (char*)out->s - (char*)out->q;
-            FGSS_CK(cudaMemcpy2DAsync(out->q, col, J.oq, J.out_col * 4, R * 4, 6, cudaMemcpyDeviceToHost, c.stream));
+            columns_to_host(out->q, col, J.oq, J.out_col * 4, R * 4, 6, c.max_pitch, c.stream);
         } else if (R) {
             FGSS_CK(cudaMemcpyAsync(out->q, J.oq, R * 4, cudaMemcpyDeviceToHost, c.stream));
             FGSS_CK(cudaMemcpyAsync(out->s, J.os, R * 4, cudaMemcpyDeviceToHost, c.stream));
@@ -122,8 +123,8 @@ void export_pairs(Ctx& c, JoinState& J, const fgss_join_opts& o, fgss_pairs* out
     c.sync();
 }
 
-// Pairs of every join of a batch: host outputs through one pinned staging
-// copy per column of the batch's output range, then a host copy per join.
+// Pairs of every join of a batch: host outputs through a pinned staging copy
+// of the batch's output range, then a host copy per join.
 void export_batch(Ctx& c, Batch& B, const fgss_join_opts* opts, fgss_pairs* outs) {
     const size_t nj = B.js.size();
     bool staged = nj > 1;
@@ -135,7 +136,7 @@ void export_batch(Ctx& c, Batch& B, const fgss_join_opts* opts, fgss_pairs* outs
     const uint64_t oc = B.out_cap;
     uint32_t* st = c.pinnedT<uint32_t>("b.stage", 6 * oc + 1);
     if (oc) {
-        FGSS_CK(cudaMemcpy2DAsync(st, oc * 4, B.oq, B.out_col * 4, oc * 4, 6, cudaMemcpyDeviceToHost, c.stream));
+        columns_to_host(st, oc * 4, B.oq, B.out_col * 4, oc * 4, 6, c.max_pitch, c.stream);
         c.sync();
     }
     for (size_t j = 0; j < nj; j++) {
@@ -578,6 +579,7 @@ fgss_status fgss_create(fgss_ctx** out, const fgss_options* opt) {
         if (prop.major != 10) fail(FGSS_ERR_UNSUPPORTED, "libfgss is built for sm_100a (B200) only");
         c.num_sms = prop.multiProcessorCount;
         c.smem_optin = prop.sharedMemPerBlockOptin;
+        c.max_pitch = prop.memPitch;
         c.verbose = o.verbose;
         if (o.tune_cache_path) c.tune_path = o.tune_cache_path;
         if (o.stream) {

@@ -39,6 +39,7 @@ struct Ctx {
     int verbose = 0;
     int num_sms = 148;
     size_t smem_optin = 227 * 1024;
+    size_t max_pitch = 0;  // of a 2-D copy (columns.h)
     std::string last_error;
     std::string tune_path;
     std::map<std::string, DevBuf> bufs;
