@@ -156,10 +156,14 @@ enum { FGSS_METHOD_PLAIN = 0,     /* per-stage launches, exact two-pass counts *
  * verification); every one gives the same pairs and counters.  The
  * reference's live filter is a thread per query (src/fgssjoin/filtering.cu:76-141);
  * its dead variants a CTA per query (filtering.cu:300-407). */
-enum { FGSS_FILTER_AUTO = 0,      /* the autotuner's choice for the join's workload class */
-       FGSS_FILTER_WARP = 1,      /* fused kernel, one warp per query (32-thread CTAs, small slot table) */
-       FGSS_FILTER_CTA = 2,       /* fused kernel, one 128-thread CTA per query (large slot table) */
+enum { FGSS_FILTER_AUTO = 0,      /* the autotuner's choice for the join's workload class; without one the
+                                     claim kernels: a warp per query of few window entries, else a CTA, and
+                                     the keyed kernel for probe prefixes above 640 tokens */
+       FGSS_FILTER_WARP = 1,      /* keyed kernel, one warp per query (32-thread CTAs, small slot table) */
+       FGSS_FILTER_CTA = 2,       /* keyed kernel, one 128-thread CTA per query (large slot table) */
        FGSS_FILTER_GLOBAL = 3 };  /* every query on the dense global-memory accumulator kernel */
+/* A strategy that fgss_autotune reported for the join's workload class runs the
+ * variant it had timed (fgss_tune_result). */
 
 typedef struct fgss_join_opts {
     float threshold;        /* Jaccard threshold in (0, 1) (fgssjoin_cli.cu:31-35) */
@@ -268,18 +272,21 @@ fgss_status fgss_selfjoin_to_file(fgss_ctx* ctx, const fgss_sets_view* sets, con
 /* ------------------------------------------------------------- autotuner */
 
 typedef struct fgss_tune_result {
-    int threads;       /* CTA size of the fused filter+verify kernel */
-    int hash_log2;     /* shared-memory slot table size (log2) */
-    int regs_rt;       /* resident threads per SM the register budget is sized for */
+    int threads;       /* CTA size of the keyed kernel */
+    int hash_log2;     /* its shared-memory slot table size (log2) */
+    int regs_rt;       /* resident threads per SM its register budget is sized for */
     int ctas_per_sm;   /* resident CTAs per SM (0 = as many as fit) */
     float ms;          /* best filter+verify time measured (device) */
     char key[64];      /* workload class the choice is cached under */
-    int filter;        /* the winning strategy: FGSS_FILTER_WARP / _CTA / _GLOBAL */
+    int filter;        /* the winning strategy: FGSS_FILTER_WARP / _CTA / _GLOBAL (_CTA also for the claim
+                          kernels, which have no shape to choose: the keyed shape is then the one of the
+                          queries they do not take) */
 } fgss_tune_result;
 
 /* Times every filter strategy of the batched method on this join -- each launch
- * shape of the fused kernel (one warp or one CTA per query) and the dense
- * global-memory accumulator for every query -- (reps runs each, best kept)
+ * shape of the keyed kernel (one warp or one CTA per query), the dense
+ * global-memory accumulator for every query and the claim kernels -- (reps runs
+ * each, best kept)
  * and caches the fastest for its workload class
  * (threshold, record-count and average-size buckets), in the context and in
  * the JSON file of fgss_options.tune_cache_path when one was given.  Later

@@ -100,7 +100,7 @@ TuneEntry filter_entry(int filter) {
     return te;
 }
 
-// The strategy a tuned entry amounts to.
+// The strategy a tuned entry amounts to (the claim kernels: a CTA per query, but for few entries).
 int filter_of(const TuneEntry& te) {
     return te.heavy_min_probe == 1 ? FGSS_FILTER_GLOBAL : te.threads == 32 ? FGSS_FILTER_WARP : FGSS_FILTER_CTA;
 }
@@ -386,15 +386,24 @@ FusedArgs* batch_filters(Ctx& c, Batch& B, const Prepass& pp, uint32_t cap_entri
 
 // The batch's launch shape: the tuned shape of its most expensive join (the
 // lowest threshold, then the most records), or the one of a requested strategy.
-TuneEntry batch_shape(Ctx& c, const Batch& B) {
+// A request for the strategy that the autotuner reported for the workload class runs
+// the entry it had timed (*as_tuned), which may be the claim kernels: 20,000 titles at
+// t = 0.5 0.36 ms, the keyed shape of that strategy 0.63 ms.
+TuneEntry batch_shape(Ctx& c, const Batch& B, bool* as_tuned = nullptr) {
+    if (as_tuned) *as_tuned = false;
     if (c.tune_force) return *c.tune_force;
     size_t lead = 0;
     for (size_t i = 1; i < B.js.size(); i++)
         if (B.js[i]->t < B.js[lead]->t || (B.js[i]->t == B.js[lead]->t && B.js[i]->in.n_sets > B.js[lead]->in.n_sets))
             lead = i;
     const JoinState& L = *B.js[lead];
-    if (L.filter != FGSS_FILTER_AUTO) return filter_entry(L.filter);
-    return tune_lookup(c, tune_key(L.in.n_sets, L.in.n_tokens, L.t));
+    const std::string key = tune_key(L.in.n_sets, L.in.n_tokens, L.t);
+    if (L.filter != FGSS_FILTER_AUTO) {
+        const auto it = c.tune.find(key);
+        if (it == c.tune.end() || filter_of(it->second) != L.filter) return filter_entry(L.filter);
+        if (as_tuned) *as_tuned = true;
+    }
+    return tune_lookup(c, key);
 }
 
 }  // namespace
@@ -562,14 +571,18 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     std::vector<JoinState*>& joins = B.js;
     const bool capture = plan && plan->capture;
     const std::string& p = c.bpfx;
-    const TuneEntry te = capture ? plan->te : batch_shape(c, B);
+    bool as_tuned = false;
+    const TuneEntry te = capture ? plan->te : batch_shape(c, B, &as_tuned);
+    if (capture) as_tuned = plan->as_tuned;
+    else if (plan) plan->as_tuned = as_tuned;
     const uint32_t cap_entries = (1u << te.hash_log2) / 4 * 3;  // chunk capacity of the chosen kernel shape
     const uint64_t P_cap = plan ? plan->P_cap : B.P;
     if (P_cap < B.P) fail(FGSS_ERR_CUDA, "window buffers below the batch's probe-token count");
     const bool model = use_model && c.model;
     // the caller's own choice of a strategy, a tuned keyed shape and the global accumulator take every query
     bool classes = te.heavy_min_probe == 0 && !te.keyed;
-    for (size_t i = 0; i < nj; i++) classes &= joins[i]->filter == FGSS_FILTER_AUTO;
+    for (size_t i = 0; i < nj; i++)
+        classes &= joins[i]->filter == FGSS_FILTER_AUTO || (as_tuned && joins[i]->filter == filter_of(te));
     // light: no query can be k_fused's and there is no learned estimate to order them by, so
     // k_claim takes the records in order and the costs, items and their sort, and the wait
     // for their counts, are left out (1,000 titles: 60 us of 450)

@@ -143,6 +143,7 @@ struct Batch {
 struct BatchPlan {
     bool capture = false;             // issue device work only, with these decisions
     TuneEntry te;
+    bool as_tuned = false;            // a requested strategy runs its tuned entry (batch_shape)
     uint64_t E_cap = 0, P_cap = 0;    // index entries, probe windows the buffers hold
     bool wide = false;                // k_claim's shape
     bool light = false;               // every query is the claim kernels', whose items are the records in order
