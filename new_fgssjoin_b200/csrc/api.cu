@@ -665,10 +665,7 @@ fgss_status fgss_tokenize(fgss_ctx* ctx, const char* text, uint64_t n_bytes, con
     if (!ctx || !out || (!text && n_bytes)) return FGSS_ERR_INVALID;
     memset(out, 0, sizeof *out);
     return guard(ctx, [&] {
-        fgss_tok_opts o;
-        fgss_tok_opts_default(&o);
-        if (opts) o = *opts;
-        TokParams p{o.q, o.mode, o.pad, o.pad_char, o.suffix, o.lower};
+        const TokParams p = tok_params(opts);
         FGSS_CK(cudaSetDevice(ctx->c.device));
         or_undo(
             ctx->c, [&] { tokenize_device(ctx->c, text, n_bytes, p, out); }, [&] { fgss_sets_free(out); });
@@ -681,10 +678,7 @@ fgss_status fgss_tokenize_dual(fgss_ctx* ctx, const char* text_r, uint64_t n_r, 
     memset(out_r, 0, sizeof *out_r);
     memset(out_s, 0, sizeof *out_s);
     return guard(ctx, [&] {
-        fgss_tok_opts o;
-        fgss_tok_opts_default(&o);
-        if (opts) o = *opts;
-        TokParams p{o.q, o.mode, o.pad, o.pad_char, o.suffix, o.lower};
+        const TokParams p = tok_params(opts);
         FGSS_CK(cudaSetDevice(ctx->c.device));
         // one text: R's lines, then S's; record ids count the non-empty lines
         std::string text(text_r ? text_r : "", n_r);
