@@ -213,13 +213,16 @@ __global__ void k_compact_tok(const uint64_t* __restrict__ key, const uint64_t* 
         }
 }
 
-// tag (line << 32 | pos) -> global gram index (monotone in (line, pos)) for the first-occurrence order
-__global__ void k_tag_index(const uint64_t* __restrict__ tag, const uint32_t* __restrict__ goff, uint64_t n,
-                            uint32_t* __restrict__ gidx, const uint32_t* __restrict__ err) {
+// tag (line << 32 | pos) -> a 32-bit number that ascends with (line, pos), for the
+// first-occurrence order: the gram's index, but of k-mers the window's place in the text (ls:
+// the lines' starts; windows with other bytes are skipped, so goff does not count positions).
+__global__ void k_tag_index(const uint64_t* __restrict__ tag, const uint32_t* __restrict__ goff,
+                            const uint64_t* __restrict__ ls, int kmers, uint64_t n, uint32_t* __restrict__ gidx,
+                            const uint32_t* __restrict__ err) {
     if (gave_up(err)) return;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t t = tag[i];
-        gidx[i] = goff[t >> 32] + (uint32_t)t;
+        gidx[i] = (kmers ? (uint32_t)ls[t >> 32] : goff[t >> 32]) + (uint32_t)t;
     }
 }
 
@@ -1094,7 +1097,8 @@ void tokenize_sorted(Ctx& c, const unsigned char* dtext, uint64_t nb, const TokP
     const int kb2 = suffix ? kb + 16 : kb;
     radix_sort<uint64_t, uint64_t>(c, tkey, ttag, Tn, nullptr, 0, kb2 > 64 ? 64 : kb2, "tk.sortC");
     uint32_t* gidx = c.devT<uint32_t>("tk.gidx", Tn + 1);
-    k_tag_index<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(ttag, goff, Tn, gidx, c.err_dev);
+    k_tag_index<<<grid_for(Tn, 256, c.num_sms * 32), 256, 0, c.stream>>>(ttag, goff, ls, p.mode, Tn, gidx,
+                                                                             c.err_dev);
     FGSS_LAUNCH_CK();
     uint32_t* rflag = c.devT<uint32_t>("tk.rflag", Tn + 1);
     uint32_t* rid = c.devT<uint32_t>("tk.rid", Tn + 1);
