@@ -177,10 +177,20 @@ TileMap tiles_for(const TileMap& m, uint64_t want, uint32_t low) {
 // k_bitmaps_mj 32 -> 3.3, k_index_entries_mj 21 -> 2.9 with tiles of 8 instead of 256).
 TileMap warp_tiles(Ctx& c, const TileMap& m) { return tiles_for(m, (uint64_t)32 * c.num_sms, 8); }
 
-// Items of the records in order: about 128 per CTA.
-ClaimItems items_in_order(Ctx& c, const TileMap& m) {
-    const TileMap t = tiles_for(m, (uint64_t)128 * kClaimCtas * c.num_sms, 1);
-    return {nullptr, t, t.ntiles};
+// Items of the records in order: about 128 per CTA.  Of one join, its query range
+// only: an item costs a CTA an atomic and its records' classes even where it has no
+// query (one query of 100,000 records: k_claim 237 us over all of them).
+ClaimItems items_in_order(Ctx& c, const Batch& B) {
+    const uint64_t want = (uint64_t)128 * kClaimCtas * c.num_sms;
+    if (B.js.size() > 1) {
+        const TileMap t = tiles_for(B.rec, want, 1);
+        return {nullptr, t, 0, t.ntiles};
+    }
+    const JoinArgs& a = B.js[0]->args;
+    uint32_t tile = B.rec.tile;
+    while (tile > 1 && (a.q_hi - a.q_lo) / tile < want) tile >>= 1;
+    const uint32_t first = a.q_lo / tile, end = (uint32_t)(((uint64_t)a.q_hi + tile - 1) / tile);
+    return {nullptr, finer_tiles(B.rec, tile), first, end - first};
 }
 
 template <int MODE>
@@ -648,8 +658,8 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     const uint4* items[2] = {nullptr, nullptr};
     for (int k = 0; k < 2; k++)
         if (nitems[k]) items[k] = batch_items(c, B, pp, k, K[k], nitems[k]);
-    const ClaimItems claims = light ? items_in_order(c, B.rec)
-                                    : ClaimItems{items[QC_CLAIM], B.rec, (uint32_t)nitems[QC_CLAIM]};
+    const ClaimItems claims = light ? items_in_order(c, B)
+                                    : ClaimItems{items[QC_CLAIM], B.rec, 0, (uint32_t)nitems[QC_CLAIM]};
 
     bool sided = false;
     for (size_t i = 0; i < nj; i++) sided |= joins[i]->args.side != nullptr;
@@ -848,7 +858,7 @@ void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
     // ---- pre-pass: windows and classes of the queries; k_claim takes the records in order
     const Prepass pp = batch_prepass(c, B, 1u << 30, B.P, false, true, true);
     const bool keyed = B.keyed_possible, sided = a.side != nullptr;
-    const ClaimItems claims = items_in_order(c, B.rec);
+    const ClaimItems claims = items_in_order(c, B);
     FusedArgs* d_fargs = batch_filters(c, B, pp, 1u << 30, 0, false);
     const FusedArgs& fa = c.pinnedT<FusedArgs>(p + "b.hf", 1)[0];
     a.meta = pp.meta;

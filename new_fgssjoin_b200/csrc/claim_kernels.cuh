@@ -86,17 +86,17 @@ struct ClaimShape {
     static_assert(MC <= 32 * NWC, "a warp's share of the merge list fits its lanes");
 };
 
-// Work items of k_claim: a list of (join, first query, end), or without one the
-// tiles of the map in order -- records come in descending size, so the costly
-// queries still come first.
+// Work items of k_claim: a list of (join, first query, end), or without one n
+// tiles of the map in order from `first` -- records come in descending size, so the
+// costly queries still come first.
 struct ClaimItems {
     const uint4* list;
     TileMap m;
-    uint32_t n;
+    uint32_t first, n;
 };
 __device__ __forceinline__ uint4 claim_item(const ClaimItems& I, uint32_t it) {
     if (I.list) return I.list[it];
-    const TileRange t = tile_range(I.m, it);
+    const TileRange t = tile_range(I.m, I.first + it);
     return make_uint4(t.j, t.r0, t.r1, 0);
 }
 
