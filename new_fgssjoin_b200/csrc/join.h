@@ -116,6 +116,7 @@ struct Batch {
     uint64_t R = 0;                    // records of the batch
     uint64_t E = 0, P = 0;             // index entries, probe windows (read back by batch_prep)
     uint32_t n_max = 0;                // records of the largest join
+    uint32_t len_max = 0;              // longest record of any join (read back by batch_prep)
     bool keyed_possible = false;       // a record's probe prefix may exceed kClaimPC (read back by batch_prep)
     const uint32_t* status_host = nullptr;  // status words, once read back after the filter (batch_read_status)
     uint32_t terms_max = 0;

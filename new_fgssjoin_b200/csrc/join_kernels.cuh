@@ -837,17 +837,23 @@ __device__ __forceinline__ bool bitmap_keeps(const uint4* q4, const uint4* __res
 // lanes: 17.8 M records of 100,000 titles at t = 0.7 took 2.1 ms, a lane each 0.22 ms.
 // A warp takes `per` <= 32 records, fewer where there are too few to give every
 // warp 32 (the merges of one warp's records are a serial chain: 500 titles at
-// t = 0.9 took 99 us at 32 a warp, 7 us at 1).
+// t = 0.9 took 99 us at 32 a warp, 7 us at 1), in groups of `group` consecutive ones
+// that lie as far apart as there are warps: the records left come in runs, those of
+// one query's near-duplicates, and long records' merges (40 us each at 4,000 tokens)
+// are not to be one warp's.  20,000 records of 5 to 40 tokens and 20 of 3,000 to 5,000
+// at t = 0.6: a call 1.88 ms with 32 consecutive records a warp, 1.07 in groups of 4,
+// 1.10 of 8; but 100,000 titles at t = 0.6 (144 tokens at most) 4.93, 5.06 and 4.98,
+// whose queries' bitmaps a warp then reads more of: groups where records are long.
 static __global__ void k_verify(JoinArgs a, const uint4* __restrict__ cand, const uint64_t* __restrict__ d_nc,
-                                uint32_t per, uint32_t* __restrict__ ov, const uint4* __restrict__ bmap,
-                                uint32_t bmw) {
+                                uint32_t per, uint32_t group, uint32_t* __restrict__ ov,
+                                const uint4* __restrict__ bmap, uint32_t bmw) {
     const uint32_t nc = (uint32_t)*d_nc;
     const uint32_t lane = lane_id();
     const uint64_t w0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x >> 5) * per;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     unsigned long long inter = 0;
-    for (uint64_t i0 = w0 * per; i0 < nc; i0 += stride) {
-        const uint64_t i = i0 + lane;
+    for (uint64_t i0 = 0; i0 < nc; i0 += warps * per) {
+        const uint64_t i = i0 + (lane / group * warps + w0) * group + lane % group;
         const bool in = lane < per && i < nc;
         const uint4 r = in ? cand[i] : make_uint4(0, 0, 0, 0);
         uint32_t lq = 0, ls = 0, imin = 0;
