@@ -265,8 +265,7 @@ void index_sort(Ctx& c, Batch& B, uint64_t E_cap, int tbits, int jbits, const ui
 }
 
 // The batch's pre-pass, first part (index built): windows of every probe
-// token (exact per-query work), the class of every query (classes; else all
-// QC_KEYED), the learned model's estimates (model) and the work-item costs
+// token (exact per-query work), the class of every query (pc: windows_query), the learned model's estimates (model) and the work-item costs
 // (k_cost_mj).  d_sums: k_cost_mj's 2 nj + 4 sums, then the joins' predicted
 // results (nj) and candidates (nj).
 struct Prepass {
@@ -281,7 +280,7 @@ struct Prepass {
 };
 
 // light: the windows and classes only.
-Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bool model, bool classes, bool light = false) {
+Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bool model, uint32_t pc, bool light = false) {
     const size_t nj = B.js.size();
     const std::string& p = c.bpfx;
     const uint64_t R = B.R;
@@ -294,7 +293,7 @@ Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bo
     const unsigned wg = tile_grid(c, wt);
     if (light) {
         if (R) {
-            k_windows_mj<<<wg, 256, 0, c.stream>>>(B.d_args, wt, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, classes);
+            k_windows_mj<<<wg, 256, 0, c.stream>>>(B.d_args, wt, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, pc);
             FGSS_LAUNCH_CK();
         }
         return pp;
@@ -307,7 +306,7 @@ Prepass batch_prepass(Ctx& c, Batch& B, uint32_t cap_entries, uint64_t P_cap, bo
     pp.d_sums = c.devT<uint64_t>(p + "b.sums", pp.n_sums);
     FGSS_CK(cudaMemsetAsync(pp.d_sums, 0, pp.n_sums * 8, c.stream));
     if (R == 0) return pp;
-    k_windows_mj<<<wg, 256, 0, c.stream>>>(B.d_args, wt, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, classes);
+    k_windows_mj<<<wg, 256, 0, c.stream>>>(B.d_args, wt, B.poff, pp.win, pp.wpre, pp.wtot, pp.meta, pc);
     FGSS_LAUNCH_CK();
     if (model) {
         pp.pred = pred;
@@ -564,7 +563,7 @@ void batch_index(Ctx& c, Batch& B, uint64_t E_cap) {
 void batch_query_costs(Ctx& c, Batch& B, bool use_model, uint64_t* out) {
     if (B.R == 0) return;
     const TuneEntry te = batch_shape(c, B);
-    const Prepass pp = batch_prepass(c, B, (1u << te.hash_log2) / 4 * 3, B.P, use_model && c.model, false);
+    const Prepass pp = batch_prepass(c, B, (1u << te.hash_log2) / 4 * 3, B.P, use_model && c.model, 0);
     k_query_costs_mj<<<tile_grid(c, B.rec), 256, 0, c.stream>>>(B.d_args, B.rec, pp.wtot, pp.pred, pp.cost[0]);
     FGSS_LAUNCH_CK();
     FGSS_CK(cudaMemcpyAsync(out, pp.cost[0], B.R * 8, cudaMemcpyDeviceToHost, c.stream));
@@ -600,7 +599,7 @@ void batched_filter_verify(Ctx& c, Batch& B, bool use_model, BatchPlan* plan) {
     // for their counts, are left out (1,000 titles: 60 us of 450)
     const bool light = capture ? plan->light : classes && !model && !B.keyed_possible && B.R != 0;
     if (plan && !capture) plan->light = light;
-    const Prepass pp = batch_prepass(c, B, cap_entries, P_cap, model, classes, light);
+    const Prepass pp = batch_prepass(c, B, cap_entries, P_cap, model, classes ? kClaimPC : 0, light);
 
     // work items per class of k_fused and k_claim: ~256 per resident CTA over
     // the whole batch (a few queries per item at 100k records), split by cost
@@ -841,11 +840,35 @@ __global__ void k_sum_u32(const uint32_t* __restrict__ in, uint64_t n, unsigned 
 }
 
 template <int MODE, int NT, int HLOG>
-void probe_launch(Ctx& c, const JoinArgs* d_args, uint64_t n) {
+void probe_launch(Ctx& c, const JoinArgs* d_args, uint64_t n, cudaStream_t stream) {
     FGSS_CK(cudaFuncSetAttribute(k_probe<MODE, NT, HLOG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ProbeLayout<MODE, HLOG>::bytes));
-    k_probe<MODE, NT, HLOG><<<(unsigned)n, NT, ProbeLayout<MODE, HLOG>::bytes, c.stream>>>(d_args);
+    k_probe<MODE, NT, HLOG><<<(unsigned)n, NT, ProbeLayout<MODE, HLOG>::bytes, stream>>>(d_args);
     FGSS_LAUNCH_CK();
+}
+
+// Probe tokens up to which a query of a join that runs k_probe anyway is k_claim's.  A
+// step of k_claim costs its producer two bounds for every probe token, so from about
+// 400 of them on the consumers wait for it and k_probe is the faster one.  Calls with
+// the line at 640 / 384 / 256 (k_probe beside k_claim): 2,100 records of 700 to 1,400
+// tokens at t = 0.5 4.69 / 3.48 / 3.47 ms, 6,000 of 200 to 1,800 17.4 / 16.2 / 16.3;
+// 20,000 of 100 to 700 and 20 longer ones 46 / 46 / 57.
+constexpr uint32_t kPlainPC = 384;
+
+// k_probe on the copies' stream, beside the claim kernels, whose queries are others:
+// both leave the chip idle at their ends, together less (with the line at 384, 2,100
+// records as above 3.64 -> 3.48 ms, 6,000 of 900 to 1,800 38.9 -> 35.7).  The context's
+// stream goes on behind both.
+template <int MODE, typename F>
+void probe_beside(Ctx& c, const JoinArgs* d_args, uint64_t n, bool keyed, F&& claims) {
+    if (!keyed) return claims();
+    c.copy_lane();
+    FGSS_CK(cudaEventRecord(c.copy_ev[0], c.stream));
+    FGSS_CK(cudaStreamWaitEvent(c.copy_stream, c.copy_ev[0], 0));
+    probe_launch<MODE, 256, 12>(c, d_args, n, c.copy_stream);
+    FGSS_CK(cudaEventRecord(c.copy_ev[1], c.copy_stream));
+    claims();
+    FGSS_CK(cudaStreamWaitEvent(c.stream, c.copy_ev[1], 0));
 }
 
 }  // namespace
@@ -858,8 +881,8 @@ void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
     if (n == 0) return;
     const std::string& p = c.bpfx;
     // ---- pre-pass: windows and classes of the queries; k_claim takes the records in order
-    const Prepass pp = batch_prepass(c, B, 1u << 30, B.P, false, true, true);
     const bool keyed = B.keyed_possible, sided = a.side != nullptr;
+    const Prepass pp = batch_prepass(c, B, 1u << 30, B.P, false, keyed ? kPlainPC : kClaimPC, true);
     const ClaimItems claims = items_in_order(c, B);
     FusedArgs* d_fargs = batch_filters(c, B, pp, 1u << 30, 0, false);
     const FusedArgs& fa = c.pinnedT<FusedArgs>(p + "b.hf", 1)[0];
@@ -880,16 +903,19 @@ void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
     FGSS_CK(cudaMemsetAsync(d_nc, 0, 32, c.stream));
     // ---- count pass
     upload_args(c, B, p + "b.ha2");
-    claim_launch<MODE_COUNT>(c, B.d_args, d_fargs, claims, ctr, sided);
-    tiny_launch<MODE_COUNT>(c, B.d_args, d_fargs, B.rec, sided);
-    HeavyScratch hs;
-    uint32_t hslots = 0;
     if (keyed) {
-        // probe prefixes above kClaimPC: the keyed table, or the global accumulator
         FGSS_CK(cudaMemsetAsync(a.ccnt, 0, n * 4, c.stream));
         FGSS_CK(cudaMemsetAsync(a.wcnt, 0, n * 4, c.stream));
         FGSS_CK(cudaMemsetAsync(a.heavy_count, 0, 4, c.stream));
-        probe_launch<MODE_COUNT, 256, 12>(c, B.d_args, n);
+    }
+    probe_beside<MODE_COUNT>(c, B.d_args, n, keyed, [&] {
+        claim_launch<MODE_COUNT>(c, B.d_args, d_fargs, claims, ctr, sided);
+        tiny_launch<MODE_COUNT>(c, B.d_args, d_fargs, B.rec, sided);
+    });
+    HeavyScratch hs;
+    uint32_t hslots = 0;
+    if (keyed) {
+        // probe prefixes beyond k_probe's shared memory: the global accumulator
         FGSS_CK(cudaMemcpyAsync(hcnt, a.heavy_count, 4, cudaMemcpyDeviceToHost, c.stream));
         c.sync();
         hslots = std::min<uint32_t>(hcnt[0], (uint32_t)c.num_sms);
@@ -916,9 +942,10 @@ void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
         ctr += 2;
         if (keyed) FGSS_CK(cudaMemsetAsync(a.heavy_count, 0, 4, c.stream));
         upload_args(c, B, p + "b.ha2");
-        claim_launch<MODE_FILL>(c, B.d_args, d_fargs, claims, ctr, sided);
-        tiny_launch<MODE_FILL>(c, B.d_args, d_fargs, B.rec, sided);
-        if (keyed) probe_launch<MODE_FILL, 256, 12>(c, B.d_args, n);
+        probe_beside<MODE_FILL>(c, B.d_args, n, keyed, [&] {
+            claim_launch<MODE_FILL>(c, B.d_args, d_fargs, claims, ctr, sided);
+            tiny_launch<MODE_FILL>(c, B.d_args, d_fargs, B.rec, sided);
+        });
         if (hslots) {
             k_probe_heavy<MODE_FILL, 512><<<hslots, 512, 0, c.stream>>>(B.d_args, 0, 1, hs.zero, hs.zero_words, hs.aux,
                                                                         hs.aux_words, ctr + 1);

@@ -149,13 +149,13 @@ static __global__ void k_join_totals(const JoinArgs* __restrict__ joins, const u
 // heavy-tailed records gain, 2.1 -> 1.5 ms).
 static __global__ void __launch_bounds__(256, 8) k_windows_mj(const JoinArgs* __restrict__ joins, TileMap m, const uint32_t* __restrict__ poff,
                                     uint2* __restrict__ win, uint32_t* __restrict__ wpre, uint32_t* __restrict__ wtot,
-                                    uint4* __restrict__ meta, bool classes) {
+                                    uint4* __restrict__ meta, uint32_t pc) {
     const uint32_t wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (uint32_t b = blockIdx.x; b < m.ntiles; b += gridDim.x) {
         const TileRange t = tile_range(m, b);
         const uint64_t g0 = __ldg(m.roff + t.j);
         for (uint32_t q = t.r0 + wid; q < t.r1; q += nw)
-            windows_query(joins[t.j], q, poff + g0, win, wpre, wtot + g0, meta + g0, classes);
+            windows_query(joins[t.j], q, poff + g0, win, wpre, wtot + g0, meta + g0, pc);
     }
 }
 

@@ -88,19 +88,19 @@ constexpr uint32_t kTinyMax = 128;   // window entries of a k_tiny query
 // Class of a query with W window entries and qp probe tokens.  Up to kTinyMax
 // entries fit four registers per lane of one warp; 500,000 reads (22 entries
 // each on average) take 1.1 ms with a warp each, 2.8 ms with the keyed table.
-// kClaimPC windows fit k_claim's shared memory at three CTAs per SM.
-__device__ __forceinline__ uint32_t query_class(uint32_t qp, uint32_t W) {
-    return W == 0 ? QC_NONE : W <= kTinyMax ? QC_TINY : qp <= kClaimPC ? QC_CLAIM : QC_KEYED;
+// kClaimPC windows fit k_claim's shared memory at three CTAs per SM; pc is at most that.
+__device__ __forceinline__ uint32_t query_class(uint32_t qp, uint32_t W, uint32_t pc) {
+    return W == 0 ? QC_NONE : W <= kTinyMax ? QC_TINY : qp <= pc ? QC_CLAIM : QC_KEYED;
 }
 
 // Windows of one query's probe tokens (warp-collective): win[poff[q] + j] =
 // (lo, hi), wpre[poff[q] + j] = entries in the query's windows before window j,
 // wtot[q] = sum of the window sizes (also meta[q].w).  The block table bounds
-// the searches to the blocks that hold q + 1 and send - 1.  classes: give the
-// query its class (else every query is QC_KEYED).
+// the searches to the blocks that hold q + 1 and send - 1.  pc: the probe
+// tokens up to which a query is k_claim's (0: every query is QC_KEYED).
 __device__ __forceinline__ void windows_query(const JoinArgs& a, uint32_t q, const uint32_t* __restrict__ poff,
                                               uint2* __restrict__ win, uint32_t* __restrict__ wpre,
-                                              uint32_t* __restrict__ wtot, uint4* __restrict__ meta, bool classes) {
+                                              uint32_t* __restrict__ wtot, uint4* __restrict__ meta, uint32_t pc) {
     const uint32_t lane = lane_id();
     const bool unsorted = (*a.status & ST_UNSORTED) != 0;
     const uint32_t lq = a.len[q];
@@ -139,7 +139,7 @@ __device__ __forceinline__ void windows_query(const JoinArgs& a, uint32_t q, con
     }
     if (lane == 0) {
         wtot[q] = tot;
-        const uint32_t cls = classes ? query_class(qp, tot) : (uint32_t)QC_KEYED;
+        const uint32_t cls = pc ? query_class(qp, tot, pc) : (uint32_t)QC_KEYED;
         meta[q] = make_uint4(a.pos[q], lq, (lq <= 65535u ? a.index[lq] : 0u) | (cls << 16), tot);
     }
 }
