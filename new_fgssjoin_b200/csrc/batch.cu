@@ -469,10 +469,7 @@ void batch_prep(Ctx& c, Batch& B, const std::vector<JoinState*>& js, const fgss_
         JoinState& J = *js[j];
         J.status = B.status + 8 * j;
         J.stats = B.stats + SS_N * j;
-        J.maxlen = J.status + 1;
         J.d_e = B.d_e + 2 * j;
-        J.icnt = B.icnt + B.roff[j];
-        J.pcnt = B.pcnt + B.roff[j];
         JoinArgs& a = J.args;
         a.status = J.status;
         a.stats = J.stats;
@@ -484,7 +481,7 @@ void batch_prep(Ctx& c, Batch& B, const std::vector<JoinState*>& js, const fgss_
     B.rec = upload_tiles(c, p + "b.rec", B.roff, kRecTile);
     upload_args(c, B, p + "b.ha0");
     if (B.R) {
-        const TileMap t = tiles_for(B.rec, (uint64_t)32 * c.num_sms, 8);
+        const TileMap t = warp_tiles(c, B.rec);
         k_prep_mj<<<tile_grid(c, t, 8), 256, 0, c.stream>>>(B.d_args, t, B.icnt, B.pcnt);
         FGSS_LAUNCH_CK();
         k_send_mj<<<grid_for((uint64_t)nj << 16, 256, c.num_sms * 32), 256, 0, c.stream>>>(B.d_args, (uint32_t)nj,

@@ -49,9 +49,6 @@ struct JoinState {
     uint32_t* status = nullptr;
     unsigned long long* stats = nullptr;
     uint64_t* d_e = nullptr;   // index entries (u64 copy of the scan total)
-    uint32_t* icnt = nullptr;
-    uint32_t* pcnt = nullptr;
-    uint32_t* maxlen = nullptr;
     // outputs (device)
     uint64_t* d_nres = nullptr;
     uint32_t *oq = nullptr, *os = nullptr, *oidq = nullptr, *oids = nullptr, *oo = nullptr;

@@ -354,10 +354,10 @@ int bits_for32(uint64_t v) {
 
 constexpr uint32_t kTextTile = 4096;       // text bytes per CTA of the line passes, 16 per thread
 constexpr uint32_t kMaxLineGrams = 8192;   // grams of a line of tokenize_lines
+constexpr uint64_t kPartTokens = 1 << 20;  // tokens from which a result is copied in parts
 // Classes of lines by grams (a warp each; tables of 512 and 2048 slots at eight and
 // four warps per CTA, beyond that of twice the longest line at one warp per CTA) and
 // of records by tokens (a warp, 256 and 1024 threads each).
-constexpr uint64_t kPartTokens = 1 << 20;  // tokens from which a result is copied in parts
 constexpr uint32_t kSmallLine = 256, kMidLine = 1024;
 
 // Counters of one call, read back together.
@@ -457,12 +457,6 @@ __global__ void k_line_classes(const uint32_t* __restrict__ lstart, const uint32
     mx = __reduce_max_sync(kFull, mx);
     if (lane_id() == 0 && mx) atomicMax(&cnt->max_grams, mx);
 }
-
-// How a gram becomes a key: code of every byte (dense, cb bits), q of them.
-struct GramCode {
-    const uint8_t* lut;
-    int cb;
-};
 
 // Grams of line l in rows of 32 positions, a warp per line: f(position, key,
 // valid) for every row (all lanes).  q-grams: the dense codes of q bytes.
