@@ -969,9 +969,13 @@ void plain_filter_verify(Ctx& c, Batch& B, bool want_cand) {
     // 4 % by them, of 500 and more gain up to 40 %.  Where a warp has fewer than 32 records the bound's
     // loads do not matter and every record is a group: 1,500 records of 1,500 to 4,000 tokens at
     // t = 0.8 1.65 ms in groups of 4, 1.52 of 1
-    const uint32_t group = B.len_max <= 256 ? per : per == 32 ? 4u : 1u;
-    k_verify<<<grid_for((C + per - 1) / per * 32, 256, c.num_sms * 32), 256, 0, c.stream>>>(a, cand, d_nc, per, group,
-                                                                                            ov, fa.bmap, fa.bmw);
+    // Beyond 64 rounds of all warps a warp's share of the runs evens out and only the loads are left:
+    // 200,000 heavy-tailed records at t = 0.8 (17 rounds) 5.09 ms without groups, 3.97 with, at 0.7 (54)
+    // 11.52 and 11.37; 500,000 at 0.8 (97) 13.6 and 14.0, 1,000,000 at 0.7 (1,190) 177 and 185.
+    const unsigned blocks = grid_for((C + per - 1) / per * 32, 256, c.num_sms * 32);
+    const bool spread = B.len_max > 256 && C / 64 <= (uint64_t)blocks * 256;
+    const uint32_t group = !spread ? per : per == 32 ? 4u : 1u;
+    k_verify<<<blocks, 256, 0, c.stream>>>(a, cand, d_nc, per, group, ov, fa.bmap, fa.bmw);
     FGSS_LAUNCH_CK();
     // ---- compaction of the verified pairs: count -> scan -> fill
     uint32_t* flag = c.devT<uint32_t>(J.pfx("flag"), C + 1);
