@@ -157,11 +157,11 @@ class Clocks:
 
 
 def profiled_traffic(workload):
-    """DRAM bytes (read + write) of one launch of the keyed kernel (k_fused, every query
-    on it) from the committed ncu summary of this workload
-    (profiles/k_fused_<workload>.md), or None."""
+    """DRAM bytes (read + write) of a step's filter kernels (k_claim, k_tiny, k_fused)
+    from the committed ncu summary of this workload (profiles/filter_<workload>.md),
+    or None."""
     import re
-    path = os.path.join(ROOT, "profiles", "k_fused_%s.md" % workload)
+    path = os.path.join(ROOT, "profiles", "filter_%s.md" % workload)
     if not os.path.exists(path):
         return None
     scale = {"byte": 1.0, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9}
@@ -703,8 +703,8 @@ def main():
                          "path": "text in host memory -> GPU tokenizer -> batched join -> pairs in host memory"},
             "roofline": {"bound": "hbm", "kernel": "k_claim + k_tiny + k_fused", "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": profiled_traffic(args.workload), "traffic_source": "profiles/k_fused_%s.md"
-                         " (the keyed kernel alone)" % args.workload, "alg_bytes": alg_bytes,
+                         "traffic": profiled_traffic(args.workload), "traffic_source": "profiles/filter_%s.md" % args.workload,
+                         "alg_bytes": alg_bytes,
                          "alg_bytes_formula": "12 probe_tokens + 8 window_entries + 4 merged_tokens + 12 results"
                                               " + 4 query_tokens", "kernel_ms": kern_ms, "heavy_kernel_ms": heavy_ms},
             "gpu_launches": launches * args.steps,

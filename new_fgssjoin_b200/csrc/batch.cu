@@ -135,8 +135,9 @@ namespace {
 
 // k_claim's shapes: 256 consumer threads, 8192 claim slots, 6 entries a thread or 8
 // (wide), 3 CTAs per SM (53 and 59 KB of shared memory each: at 66 KB and more the L1
-// that is left costs 10 %).  The wide shape has fewer steps, the other no spills and
-// less to lay out for a short step.  6 / 8 entries, kernel time: 1,000,000
+// that is left costs 10 %).  The wide shape has fewer steps, the other
+// less to lay out for a short one and fewer spills (80 bytes stored and 88 loaded a thread, the
+// wide one 116 and 96; 92 and 108, 128 and 116 with sides).  6 / 8 entries, kernel time: 1,000,000
 // heavy-tailed records at t = 0.7 (5,350 window entries a query) 99.9 / 94.9 ms;
 // 100,000 titles at t = 0.5 (3,356) 4.14 / 4.24; R-S of 2 x 60,000 titles at t = 0.6
 // 3.44 / 3.47; 150,000 heavy-tailed records at t = 0.85 (86) 0.54 / 0.58; 100,000 titles
@@ -145,7 +146,10 @@ namespace {
 using Claim = ClaimShape<256, 6, 13>;
 using ClaimWide = ClaimShape<256, 8, 13>;
 constexpr int kClaimCtas = 3;
-constexpr uint64_t kClaimWideCost = 4096;  // average cost (k_cost_mj) of k_claim's queries from which it is wide
+// Average cost (k_cost_mj) of k_claim's queries from which it is wide: between the averages
+// 3,356 and 5,350 above, nothing nearer was timed.  Without costs (a light call, the plain
+// method) it is narrow.
+constexpr uint64_t kClaimWideCost = 4096;
 
 template <class Shape, int MODE, bool SIDED>
 void claim_launch_as(Ctx& c, const JoinArgs* d_args, const FusedArgs* d_fargs, const ClaimItems& items,

@@ -13,8 +13,8 @@
 // every query, instead of a binary search per query, probe token and
 // range.  Measured (filter kernels of a call, chunk splits included): 1,000,000
 // heavy-tailed records at t = 0.7 177 -> 95 ms, 100,000 titles at t = 0.5
-// 12.1 -> 4.2 ms, 2 x 60,000 titles R-S at t = 0.6 6.3 -> 3.5 ms, 500,000
-// reads at t = 0.8 2.8 -> 0.95 ms, 100,000 titles at t = 0.7 with the plain method's
+// 12.1 -> 4.2 ms, 2 x 60,000 titles R-S at t = 0.6 6.3 -> 3.4 ms, 500,000
+// reads at t = 0.8 2.8 -> 0.99 ms, 100,000 titles at t = 0.7 with the plain method's
 // two passes 8.4 -> 1.6 ms.
 #pragma once
 
@@ -626,8 +626,9 @@ constexpr uint32_t kTinyWarps = 8;
 // 8 to 32 consecutive records of a join.  Bound by the latency of a query's chain of
 // loads (windows, entries, bounds, bitmaps, merges; 0.8 instructions a cycle):
 // 64 registers for 4 CTAs an SM, the queries' bounds and offsets and four chunks
-// of a merge's tokens fetched at once (500,000 reads at t = 0.8 1.05 -> 0.77 ms,
-// 48 joins of titles 0.57 -> 0.47; at 3 CTAs 0.94 and 0.55, at 5 0.81 and 0.61).
+// of a merge's tokens fetched at once (this kernel on 500,000 reads at t = 0.8
+// 1.05 -> 0.77 ms, on 48 joins of titles 0.57 -> 0.47; at 3 CTAs 0.94 and 0.55, at 5 0.81 and
+// 0.61), though MODE_FUSED then spills 40 bytes and loads 68 a thread.
 struct TinyShared {
     uint32_t at[kTinyMax];    // entry of number f
     uint32_t src[kTinyMax];

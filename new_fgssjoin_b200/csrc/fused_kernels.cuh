@@ -87,7 +87,7 @@ constexpr uint32_t kTinyMax = 128;   // window entries of a k_tiny query
 
 // Class of a query with W window entries and qp probe tokens.  Up to kTinyMax
 // entries fit four registers per lane of one warp; 500,000 reads (22 entries
-// each on average) take 1.1 ms with a warp each, 2.8 ms with the keyed table.
+// each on average) take 0.99 ms, nearly all with a warp each, 2.8 ms with the keyed table.
 // kClaimPC windows fit k_claim's shared memory at three CTAs per SM; pc is at most that.
 __device__ __forceinline__ uint32_t query_class(uint32_t qp, uint32_t W, uint32_t pc) {
     return W == 0 ? QC_NONE : W <= kTinyMax ? QC_TINY : qp <= pc ? QC_CLAIM : QC_KEYED;

@@ -30,10 +30,10 @@
 // positions out (8 bytes a token over the link); on the device, the table and the
 // sort of each line in shared memory and the one global sort.  The global-sort form
 // moves 16-byte records through 9 to 11 radix passes and 8-byte keys through 16 to
-// 20 more.  Call times, global sorts and lines (the sort passes the same):
-// 200,000 titles 7.2 and 4.4 ms (1.9 ms of it copies out, 1.2 ms in), 60,000
-// heavy-tailed records with occurrences 4.6 and 3.8 ms, 200,000 reads 23.6 and
-// 11.1 ms (3.8 and 2.6 ms copies).
+// 20 more.  Call times, global sorts and lines (the sort passes the same, results
+// copied whole), lines with the results in parts, and the copies out and in by
+// themselves: 200,000 titles 7.2, 4.4, 4.1 (1.9 + 0.7) ms, 60,000 heavy-tailed records
+// with occurrences 4.6, 3.8, 3.5 (1.2 + 0.5), 200,000 reads 23.6, 11.1, 10.2 (3.8 + 1.6).
 #include <string.h>
 
 #include <vector>
